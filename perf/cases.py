@@ -3,7 +3,7 @@
 A case is one call that a program searching protein sequences makes through
 ``cudahmmsearch_gb300.api``, by ``kind``:
 
-  dropin   p7_MSVFilter's drop-in on one sequence (what an unmodified caller loops over)
+  dropin   p7_MSVFilter's drop-in, called for one sequence after another as an unmodified program does
   search   one profile against a resident database, results left on the GPU
   batch    many profiles against one resident database (a captured batch, replayed)
   bias     the bias filter on a list of survivors of a resident database
@@ -40,7 +40,7 @@ MOST_CELLS = 400 * 2_000_000 * MEAN_LEN  # the largest listed case
 def listed():
     return [
         # the drop-in inside an unmodified program's loop: one call per sequence, launch and copies count
-        {"name": "dropin_m200", "kind": "dropin", "M": 200, "L": 350},
+        {"name": "dropin_m200", "kind": "dropin", "M": 200, "n": 16, "lmax": 5000},
         # a domain model against a handful of bacterial proteomes
         {"name": "search_m200_20k", "kind": "search", "M": 200, "n": 20_000, "lmax": 5000, "long_frac": 0.0},
         # a short domain model (most of Pfam) against a Swiss-Prot sized database
@@ -73,7 +73,7 @@ def _log(rng, lo, hi):
 def draw(rng):
     kind = rng.choice(["dropin", "search", "search", "search", "batch", "bias", "vit", "host", "filters"])
     if kind == "dropin":
-        return {"kind": kind, "M": _log(rng, 20, 2400), "L": _log(rng, 20, 5000)}
+        return {"kind": kind, "M": _log(rng, 20, 2400), "n": rng.randint(6, 32), "lmax": rng.choice([1000, 5000])}
     if kind in ("search", "host"):
         M = _log(rng, 20, 2400)
         long_frac = rng.choice([0.0, 0.0, 0.02])
@@ -186,10 +186,9 @@ def prepare(case, seed):
     ctx = _ctx()
     if kind == "dropin":
         p = api.sample_profile(case["M"], 1 + seed % 1000)
-        s = _sequences(seed, 4, lmax=20000, emit=F.emission_probs(p), hom_frac=0.5)
-        body = np.resize(s.codes, case["L"])
-        dsq = np.concatenate([[255], body, [255]]).astype(np.uint8)
-        return {"case": case, "ctx": ctx, "p": p, "dsq": dsq, "tjb": api.tjb_b(p.scale_b, case["L"])}
+        s = _sequences(seed, case["n"], lmax=case["lmax"], emit=F.emission_probs(p), hom_frac=0.1)
+        dsq = [np.concatenate([[255], s.seq(i), [255]]).astype(np.uint8) for i in range(s.n)]
+        return {"case": case, "ctx": ctx, "p": p, "dsq": dsq, "tjb": [api.tjb_b(p.scale_b, len(d) - 2) for d in dsq]}
     if kind in ("search", "host"):
         p = api.sample_profile(case["M"], 1 + seed % 1000, ctx)
         s = _sequences(seed, case["n"], lmax=case["lmax"], long_frac=case["long_frac"], emit=F.emission_probs(p),
@@ -226,8 +225,8 @@ def run(state):
     case = state["case"]
     kind, ctx = case["kind"], state["ctx"]
     if kind == "dropin":
-        status, sc = ctx.MSVFilter(state["dsq"], case["L"], state["p"], state["tjb"])
-        return {"status": int(status), "sc": float(sc)}
+        got = [ctx.MSVFilter(d, len(d) - 2, state["p"], t) for d, t in zip(state["dsq"], state["tjb"])]
+        return {"status": np.array([g[0] for g in got], np.int32), "sc": np.array([g[1] for g in got], np.float32)}
     if kind == "search":
         out = state["out"]
         api.search_device(ctx, state["prof"], state["db"], out[0].data_ptr(), out[1].data_ptr())
@@ -264,8 +263,8 @@ def work(case):
     and the emission for the ViterbiFilter; per residue of the bias filter 4
     multiplies by transitions, 2 by emissions, 2 adds, 2 divisions and a log."""
     kind = case["kind"]
-    n = 1 if kind == "dropin" else case["nlist"] if kind in ("bias", "vit") else case["n"]
-    res = case["L"] if kind == "dropin" else n * (MEAN_LEN + 20000.0 * case.get("long_frac", 0.0))
+    n = case["nlist"] if kind in ("bias", "vit") else case["n"]
+    res = n * (MEAN_LEN + 20000.0 * case.get("long_frac", 0.0))
     if kind in ("dropin", "search", "host"):
         return {"bytes": res + 2 * n + 29 * case["M"], "flops": 3.0 * case["M"] * res}
     if kind == "batch":
@@ -391,7 +390,7 @@ def exact(case, seed):
     kind = case["kind"]
     if kind == "dropin":
         st = prepare(case, seed)
-        return {"status": None, "sc": _exact_msv(st["p"], st["dsq"][1:-1], st["tjb"])}
+        return {"status": None, "sc": np.array([_exact_msv(st["p"], d[1:-1], t) for d, t in zip(st["dsq"], st["tjb"])])}
     if kind == "bias":
         return {"sc": _exact_bias(prepare(case, seed))}
     if kind == "vit" and case["nlist"] * VITERBI[case["model"]] <= 12_000_000:
