@@ -30,9 +30,16 @@
 
 #include "../../include/msvgb.h"
 #include "msv_internal.h"
+#include "msv_vit_fast.cuh"
 
 using namespace msvgb;
 using msvgb_detail::fail;
+
+namespace msvgb {
+template <int W>
+cudaError_t launch_vit_fast(const VitFastDev &V, const DbDev &db, const int64_t *ids, const int64_t *order, int64_t n,
+                            int *xc, uint8_t *st, unsigned long long *ticket, int sms, cudaStream_t stream);
+}
 
 namespace {
 
@@ -548,6 +555,116 @@ cudaError_t dispatch_vit(int CV, const VitDev &V, const DbDev &db, const int64_t
   return cudaErrorInvalidValue;
 }
 
+// Words per lane compiled for the packed kernel (msv_vit_fast.cuh).
+constexpr int kVitFastW[] = {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 16, 20, 24, 28, 32, 36, 40};
+
+cudaError_t dispatch_vit_fast(int W, const VitFastDev &V, const DbDev &db, const int64_t *ids, const int64_t *order,
+                              int64_t n, int *xc, uint8_t *st, unsigned long long *ticket, int sms,
+                              cudaStream_t stream) {
+  switch (W) {
+#define FCASE(c) case c: return launch_vit_fast<c>(V, db, ids, order, n, xc, st, ticket, sms, stream);
+    FCASE(1) FCASE(2) FCASE(3) FCASE(4) FCASE(5) FCASE(6) FCASE(7) FCASE(8) FCASE(9) FCASE(10) FCASE(11) FCASE(12)
+    FCASE(13) FCASE(14) FCASE(16) FCASE(20) FCASE(24) FCASE(28) FCASE(32) FCASE(36) FCASE(40)
+#undef FCASE
+  }
+  return cudaErrorInvalidValue;
+}
+
+// The packed kernel's tables for a profile, when its costs allow it, and the
+// lowest N/J/C move cost (that is, the longest target) up to which they do.
+// With F = base + move + min BM (every state value is kept at or above F, and
+// match cells at or above F + min e):
+//  * no sum of a stored value and a cost of a real node is below -32768;
+//  * padding nodes stay at or below the best real match cell of every row:
+//    a cost t_pad into them (from the entry, the last real node, I and D)
+//    keeps their candidates at or below xB + max BM, since xB is within
+//    E loop + move of the largest score so far, and their emissions are no
+//    larger than any real node's;
+//  * the D->D bound covers every D->D->M step, so that closing D->D more often
+//    than the bound asks changes no match cell;
+//  * N and J loop at no cost, and the striped padding scores -32768.
+struct VitFastPlan {
+  int W = 0;                                        // words per lane; 0: the profile needs the general kernels
+  int move_min = 0;
+  VitFastDev V{};                                   // scalars
+  std::vector<uint32_t> tab;                        // transitions [kFT][W * 32], then emissions [NRES][W * 32]
+
+  void build(const msvgb_vom *v, int Q8) {
+    constexpr int kLowEmission = -12000;            // below: the residue's rows saturate
+    const int M = v->M, Np = 8 * Q8;
+    int w = 0;
+    for (int c : kVitFastW) if (64 * c >= M) { w = c; break; }
+    if (!w || v->xw[1][1] != 0 || v->xw[2][1] != 0 || v->xw[0][1] > 0) return;
+    auto t_of = [&](int t, int k) -> int {          // t < 7: costs of node k; 7: D(k-1) -> D(k)
+      if (t == 7) return v->twv[(7 * Q8 + (k - 2) % Q8) * 8 + (k - 2) / Q8];
+      return v->twv[((k - 1) % Q8 * 7 + t) * 8 + (k - 1) / Q8];
+    };
+    auto e_of = [&](int x, int k) -> int { return v->rwv[(x * Q8 + (k - 1) % Q8) * 8 + (k - 1) / Q8]; };
+    for (int k = M + 1; k <= Np; ++k) {
+      for (int t = 0; t < 4; ++t) if (t_of(t, k) != -32768) return;
+      for (int x = 0; x < 29; ++x) if (e_of(x, k) != -32768) return;
+    }
+    int bm_min = 0, bm_max = -32768, t_m = 0, t_id = 0, emax = 0, emin = 0;
+    for (int k = 1; k <= M; ++k) {
+      bm_min = std::min(bm_min, t_of(0, k));
+      bm_max = std::max(bm_max, t_of(0, k));
+      if (k > 1) {
+        t_m = std::min(t_m, t_of(1, k));
+        t_id = std::min({t_id, t_of(2, k), t_of(3, k), t_of(7, k)});
+      }
+      if (k < M) {
+        t_m = std::min({t_m, t_of(4, k), t_of(5, k)});
+        t_id = std::min(t_id, t_of(6, k));
+      }
+    }
+    int e_low[NRES];
+    uint32_t low_res = 1u << 29;                    // 29, 30: never scored
+    for (int x = 0; x < 29; ++x) {
+      e_low[x] = 0;
+      for (int k = 1; k <= M; ++k) {
+        e_low[x] = std::min(e_low[x], e_of(x, k));
+        emax = std::max(emax, e_of(x, k));
+      }
+      if (e_low[x] < kLowEmission) low_res |= 1u << x;
+      else emin = std::min(emin, e_low[x]);
+    }
+    e_low[29] = -32768;
+    for (int k = 2; k <= M - 2; ++k)
+      if (t_of(7, k + 1) + t_of(3, k + 2) - t_of(0, k + 2) > v->ddbound_w) return;
+    const int base = v->base_w, eloop = v->xw[0][1];
+    // t_pad <= eloop + move + bm_max and t_pad >= -32768 - (F + emin): the lowest move where both hold
+    const int m0 = (int) std::ceil((-32768 - base - bm_min - emin - eloop - bm_max) / 2.0);
+    const int t_pad = std::min(0, eloop + m0 + bm_max);
+    if (t_pad < -32768 || bm_min < -32768 + 1) return;
+    move_min = std::max({m0, -32768 - base - bm_min - emin - t_pad, -32768 - base - t_pad - emin,
+                         -32768 - base - bm_min - emin - t_m, -32768 - base - bm_min - t_id, -32768 - base});
+    if (move_min > -1000) return;                   // not even short targets
+    V.base_w = base; V.ddbound_w = v->ddbound_w;
+    V.xwE_move = v->xw[0][0]; V.xwE_loop = eloop; V.xwC_loop = v->xw[3][1];
+    V.bm_min = bm_min; V.hot = 32767 - 2 * emax; V.low_res = low_res;
+    tab.assign((size_t) (kFT + NRES) * w * 32, 0);
+    for (int lane = 0; lane < 32; ++lane)
+      for (int i = 0; i < w; ++i)
+        for (int h = 0; h < 2; ++h) {
+          const int k = lane * 2 * w + h * w + i + 1;
+          auto put = [&](int row, int val) {
+            tab[(size_t) row * w * 32 + vitf_at(w, lane, i)] |= (uint32_t) (uint16_t) val << (16 * h);
+          };
+          for (int t = 0; t < kFT; ++t) {
+            const bool in = t < 4 || t == 7;        // into node k, else out of it
+            int c;
+            if (k > M) c = t == 1 ? (k == M + 1 ? t_pad : 0) : in ? t_pad : 0;
+            else if (k == 1 && in && t > 0) c = 0;  // from node 0, which holds the floor
+            else if (k == M && !in) c = t_pad;
+            else c = t_of(t, k);
+            put(t, c);
+          }
+          for (int x = 0; x < NRES; ++x) put(kFT + x, k > M || x == 29 ? e_low[x] : e_of(x, k));
+        }
+    W = w;
+  }
+};
+
 // wordify(): src/impl_sse/p7_oprofile.c:527-534
 int16_t wordify(float scale_w, float sc) {
   sc = roundf(scale_w * sc);
@@ -589,6 +706,9 @@ struct msvgb_vprofile {
   void *d_trans = nullptr;
   uint4 *d_emit = nullptr;
   int16_t *d_move = nullptr;
+  int fast_W = 0, fast_move_min = 0;         // the packed kernel's width (0: not used) and lowest move cost
+  VitFastDev fast{};
+  uint32_t *d_fast = nullptr;
   int move_cap = 0;
   std::vector<int16_t> h_move;
   std::mutex move_mu;                        // the move table grows under concurrent calls
@@ -681,7 +801,16 @@ extern "C" int msvgb_vprofile_create(msvgb_ctx *ctx, const msvgb_vom *v, msvgb_v
   p->ctx = ctx; p->device = ctx->device; p->M = v->M; p->Q8 = Q8; p->CV = CV;
   p->scale_w = v->scale_w; p->nj = v->nj; p->base_w = v->base_w; p->ddbound_w = v->ddbound_w;
   memcpy(p->xw, v->xw, sizeof p->xw);
+  VitFastPlan plan;
+  plan.build(v, Q8);
   cudaError_t e = cudaSetDevice(ctx->device);
+  if (e == cudaSuccess && plan.W) {
+    e = cudaMalloc(&p->d_fast, plan.tab.size() * 4);
+    if (e == cudaSuccess) e = cudaMemcpy(p->d_fast, plan.tab.data(), plan.tab.size() * 4, cudaMemcpyHostToDevice);
+    p->fast_W = plan.W; p->fast_move_min = plan.move_min;
+    p->fast = plan.V;
+    p->fast.trans = p->d_fast; p->fast.emit = p->d_fast + (size_t) kFT * plan.W * 32;
+  }
   if (e == cudaSuccess) e = cudaMalloc(&p->d_trans, tbytes);
   if (e == cudaSuccess) e = cudaMalloc(&p->d_emit, ebytes);
   if (e == cudaSuccess) e = cudaMemcpy(p->d_trans, tsrc, tbytes, cudaMemcpyHostToDevice);
@@ -697,7 +826,7 @@ extern "C" int msvgb_vprofile_create(msvgb_ctx *ctx, const msvgb_vom *v, msvgb_v
 extern "C" int msvgb_vprofile_destroy(msvgb_vprofile *p) {
   if (!p) return MSVGB_eslOK;
   cudaSetDevice(p->device);
-  cudaFree(p->d_trans); cudaFree(p->d_emit); cudaFree(p->d_move);
+  cudaFree(p->d_trans); cudaFree(p->d_emit); cudaFree(p->d_move); cudaFree(p->d_fast);
   for (int16_t *t : p->retired) cudaFree(t);
   delete p;
   return MSVGB_eslOK;
@@ -751,8 +880,13 @@ extern "C" int msvgb_vitfilter(msvgb_ctx *c, msvgb_vprofile *p, const msvgb_db *
   V.xwN_loop = p->xw[1][1]; V.xwJ_loop = p->xw[2][1]; V.xwC_loop = p->xw[3][1];
   V.trans = p->d_trans; V.emit = p->d_emit; V.move = d_move;
   DbDev dbv{db->d_codes, db->d_start, db->d_len, db->d_orig, db->n};
+  // the packed kernel wherever its tables hold for the database's longest target
+  const bool fast = p->fast_W && msvgb_vit_move_cost(p->scale_w, p->nj, db->Lmax) >= p->fast_move_min;
+  VitFastDev VF = p->fast;
+  VF.move = d_move;
   if (e == cudaSuccess)
-    e = dispatch_vit(p->CV, V, dbv, d_ids, d_order, nids, d_xc, d_st, c->d_ticket, c->num_sms, c->stream);
+    e = fast ? dispatch_vit_fast(p->fast_W, VF, dbv, d_ids, d_order, nids, d_xc, d_st, c->d_ticket, c->num_sms, c->stream)
+             : dispatch_vit(p->CV, V, dbv, d_ids, d_order, nids, d_xc, d_st, c->d_ticket, c->num_sms, c->stream);
   if (e == cudaSuccess) msvgb_detail::count_launch();
   if (e == cudaSuccess) e = cudaMemcpyAsync(out_xc, d_xc, nids * 4, cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(out_status, d_st, nids, cudaMemcpyDeviceToHost, c->stream);
