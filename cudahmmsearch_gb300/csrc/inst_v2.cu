@@ -1,3 +1,4 @@
-// Kernel instantiations: packed ViterbiFilter, 1793 to 2560 nodes (transitions in shared memory).
+// Kernel instantiations: packed ViterbiFilter, eight warps per sequence (up to 8192 nodes).
 #include "msv_vit_fast.cuh"
-MSVGB_INSTANTIATE_VITF(32) MSVGB_INSTANTIATE_VITF(36) MSVGB_INSTANTIATE_VITF(40)
+MSVGB_INSTANTIATE_VITF(9, 8) MSVGB_INSTANTIATE_VITF(10, 8) MSVGB_INSTANTIATE_VITF(12, 8) MSVGB_INSTANTIATE_VITF(14, 8)
+MSVGB_INSTANTIATE_VITF(16, 8)

@@ -36,7 +36,7 @@ using namespace msvgb;
 using msvgb_detail::fail;
 
 namespace msvgb {
-template <int W>
+template <int W, int NW>
 cudaError_t launch_vit_fast(const VitFastDev &V, const DbDev &db, const int64_t *ids, const int64_t *order, int64_t n,
                             int *xc, uint8_t *st, unsigned long long *ticket, int sms, cudaStream_t stream);
 }
@@ -555,18 +555,24 @@ cudaError_t dispatch_vit(int CV, const VitDev &V, const DbDev &db, const int64_t
   return cudaErrorInvalidValue;
 }
 
-// Words per lane compiled for the packed kernel (msv_vit_fast.cuh).
-constexpr int kVitFastW[] = {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 16, 20, 24, 28, 32, 36, 40};
+// The packed kernel's compiled forms (msv_vit_fast.cuh): words per lane by warps per sequence.
+struct VitForm { int W, NW; };
+constexpr VitForm kVitForms[] = {{1, 1}, {2, 1}, {3, 1}, {4, 1}, {5, 1}, {6, 1}, {7, 1}, {8, 1}, {9, 1}, {10, 1},
+                                 {11, 1}, {12, 1}, {13, 1}, {14, 1}, {16, 1},                        // up to 1024 nodes
+                                 {5, 4}, {6, 4}, {7, 4}, {8, 4}, {9, 4}, {10, 4}, {12, 4}, {14, 4}, {16, 4},   // 4096
+                                 {9, 8}, {10, 8}, {12, 8}, {14, 8}, {16, 8}};                        // 8192
 
-cudaError_t dispatch_vit_fast(int W, const VitFastDev &V, const DbDev &db, const int64_t *ids, const int64_t *order,
-                              int64_t n, int *xc, uint8_t *st, unsigned long long *ticket, int sms,
-                              cudaStream_t stream) {
-  switch (W) {
-#define FCASE(c) case c: return launch_vit_fast<c>(V, db, ids, order, n, xc, st, ticket, sms, stream);
-    FCASE(1) FCASE(2) FCASE(3) FCASE(4) FCASE(5) FCASE(6) FCASE(7) FCASE(8) FCASE(9) FCASE(10) FCASE(11) FCASE(12)
-    FCASE(13) FCASE(14) FCASE(16) FCASE(20) FCASE(24) FCASE(28) FCASE(32) FCASE(36) FCASE(40)
-#undef FCASE
+cudaError_t dispatch_vit_fast(VitForm f, const VitFastDev &V, const DbDev &db, const int64_t *ids,
+                              const int64_t *order, int64_t n, int *xc, uint8_t *st, unsigned long long *ticket,
+                              int sms, cudaStream_t stream) {
+#define FCASE(c, g) case g * 100 + c: return launch_vit_fast<c, g>(V, db, ids, order, n, xc, st, ticket, sms, stream);
+  switch (f.NW * 100 + f.W) {
+    FCASE(1, 1) FCASE(2, 1) FCASE(3, 1) FCASE(4, 1) FCASE(5, 1) FCASE(6, 1) FCASE(7, 1) FCASE(8, 1) FCASE(9, 1)
+    FCASE(10, 1) FCASE(11, 1) FCASE(12, 1) FCASE(13, 1) FCASE(14, 1) FCASE(16, 1)
+    FCASE(5, 4) FCASE(6, 4) FCASE(7, 4) FCASE(8, 4) FCASE(9, 4) FCASE(10, 4) FCASE(12, 4) FCASE(14, 4) FCASE(16, 4)
+    FCASE(9, 8) FCASE(10, 8) FCASE(12, 8) FCASE(14, 8) FCASE(16, 8)
   }
+#undef FCASE
   return cudaErrorInvalidValue;
 }
 
@@ -584,16 +590,17 @@ cudaError_t dispatch_vit_fast(int W, const VitFastDev &V, const DbDev &db, const
 //    than the bound asks changes no match cell;
 //  * N and J loop at no cost, and the striped padding scores -32768.
 struct VitFastPlan {
-  int W = 0;                                        // words per lane; 0: the profile needs the general kernels
+  VitForm form{0, 0};                               // W = 0: the profile needs the general kernels
   int move_min = 0;
   VitFastDev V{};                                   // scalars
-  std::vector<uint32_t> tab;                        // transitions [kFT][W * 32], then emissions [NRES][W * 32]
+  std::vector<uint32_t> tab;                        // transitions [kFT][W * N], then emissions [NRES][W * N]; N = 32 NW
 
   void build(const msvgb_vom *v, int Q8) {
     constexpr int kLowEmission = -12000;            // below: the residue's rows saturate
     const int M = v->M, Np = 8 * Q8;
-    int w = 0;
-    for (int c : kVitFastW) if (64 * c >= M) { w = c; break; }
+    VitForm f{0, 0};
+    for (VitForm c : kVitForms) if (64 * c.W * c.NW >= M) { f = c; break; }
+    const int w = f.W, N = 32 * f.NW;
     if (!w || v->xw[1][1] != 0 || v->xw[2][1] != 0 || v->xw[0][1] > 0) return;
     auto t_of = [&](int t, int k) -> int {          // t < 7: costs of node k; 7: D(k-1) -> D(k)
       if (t == 7) return v->twv[(7 * Q8 + (k - 2) % Q8) * 8 + (k - 2) / Q8];
@@ -642,13 +649,13 @@ struct VitFastPlan {
     V.base_w = base; V.ddbound_w = v->ddbound_w;
     V.xwE_move = v->xw[0][0]; V.xwE_loop = eloop; V.xwC_loop = v->xw[3][1];
     V.bm_min = bm_min; V.hot = 32767 - 2 * emax; V.low_res = low_res;
-    tab.assign((size_t) (kFT + NRES) * w * 32, 0);
-    for (int lane = 0; lane < 32; ++lane)
+    tab.assign((size_t) (kFT + NRES) * w * N, 0);
+    for (int lane = 0; lane < N; ++lane)
       for (int i = 0; i < w; ++i)
         for (int h = 0; h < 2; ++h) {
           const int k = lane * 2 * w + h * w + i + 1;
           auto put = [&](int row, int val) {
-            tab[(size_t) row * w * 32 + vitf_at(w, lane, i)] |= (uint32_t) (uint16_t) val << (16 * h);
+            tab[(size_t) row * w * N + vitf_at(w, N, lane, i)] |= (uint32_t) (uint16_t) val << (16 * h);
           };
           for (int t = 0; t < kFT; ++t) {
             const bool in = t < 4 || t == 7;        // into node k, else out of it
@@ -661,7 +668,7 @@ struct VitFastPlan {
           }
           for (int x = 0; x < NRES; ++x) put(kFT + x, k > M || x == 29 ? e_low[x] : e_of(x, k));
         }
-    W = w;
+    form = f;
   }
 };
 
@@ -706,7 +713,8 @@ struct msvgb_vprofile {
   void *d_trans = nullptr;
   uint4 *d_emit = nullptr;
   int16_t *d_move = nullptr;
-  int fast_W = 0, fast_move_min = 0;         // the packed kernel's width (0: not used) and lowest move cost
+  VitForm fast_form{0, 0};                   // the packed kernel's form (W = 0: not used)
+  int fast_move_min = 0;                     // and lowest move cost
   VitFastDev fast{};
   uint32_t *d_fast = nullptr;
   int move_cap = 0;
@@ -804,12 +812,12 @@ extern "C" int msvgb_vprofile_create(msvgb_ctx *ctx, const msvgb_vom *v, msvgb_v
   VitFastPlan plan;
   plan.build(v, Q8);
   cudaError_t e = cudaSetDevice(ctx->device);
-  if (e == cudaSuccess && plan.W) {
+  if (e == cudaSuccess && plan.form.W) {
     e = cudaMalloc(&p->d_fast, plan.tab.size() * 4);
     if (e == cudaSuccess) e = cudaMemcpy(p->d_fast, plan.tab.data(), plan.tab.size() * 4, cudaMemcpyHostToDevice);
-    p->fast_W = plan.W; p->fast_move_min = plan.move_min;
+    p->fast_form = plan.form; p->fast_move_min = plan.move_min;
     p->fast = plan.V;
-    p->fast.trans = p->d_fast; p->fast.emit = p->d_fast + (size_t) kFT * plan.W * 32;
+    p->fast.trans = p->d_fast; p->fast.emit = p->d_fast + (size_t) kFT * plan.form.W * 32 * plan.form.NW;
   }
   if (e == cudaSuccess) e = cudaMalloc(&p->d_trans, tbytes);
   if (e == cudaSuccess) e = cudaMalloc(&p->d_emit, ebytes);
@@ -881,11 +889,11 @@ extern "C" int msvgb_vitfilter(msvgb_ctx *c, msvgb_vprofile *p, const msvgb_db *
   V.trans = p->d_trans; V.emit = p->d_emit; V.move = d_move;
   DbDev dbv{db->d_codes, db->d_start, db->d_len, db->d_orig, db->n};
   // the packed kernel wherever its tables hold for the database's longest target
-  const bool fast = p->fast_W && msvgb_vit_move_cost(p->scale_w, p->nj, db->Lmax) >= p->fast_move_min;
+  const bool fast = p->fast_form.W && msvgb_vit_move_cost(p->scale_w, p->nj, db->Lmax) >= p->fast_move_min;
   VitFastDev VF = p->fast;
   VF.move = d_move;
   if (e == cudaSuccess)
-    e = fast ? dispatch_vit_fast(p->fast_W, VF, dbv, d_ids, d_order, nids, d_xc, d_st, c->d_ticket, c->num_sms, c->stream)
+    e = fast ? dispatch_vit_fast(p->fast_form, VF, dbv, d_ids, d_order, nids, d_xc, d_st, c->d_ticket, c->num_sms, c->stream)
              : dispatch_vit(p->CV, V, dbv, d_ids, d_order, nids, d_xc, d_st, c->d_ticket, c->num_sms, c->stream);
   if (e == cudaSuccess) msvgb_detail::count_launch();
   if (e == cudaSuccess) e = cudaMemcpyAsync(out_xc, d_xc, nids * 4, cudaMemcpyDeviceToHost, c->stream);

@@ -27,8 +27,11 @@
 //
 // Bound: the fused add-maximum runs at half rate (64 lanes per clock and SM);
 // six per word of two nodes. The transition costs stay in registers across
-// rows (up to 16 words per lane; wider models read them from shared memory),
-// a row reads only its residue's emissions.
+// rows (up to 16 words per lane); a row reads only its residue's emissions.
+// One warp scores a sequence up to 1024 nodes; above, the 4 or 8 warps of a
+// block share it: one warp with its row in registers and the transitions in
+// shared memory took 5.46 ms for a call on 3,000 listed sequences at M = 2400
+// (4.1 without its host work), four warps take 2.27.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -38,8 +41,6 @@ namespace msvgb {
 
 // Transition tables: BM MM IM DM (into the node), MD MI II (out of it), DD (into it).
 constexpr int kFT = 8;
-// Words per lane with the transitions in registers; above, in shared memory.
-constexpr int kVitFastRegW = 16;
 
 struct VitFastDev {
   int base_w, ddbound_w, xwE_move, xwE_loop, xwC_loop;
@@ -51,198 +52,173 @@ struct VitFastDev {
   const int16_t *move;      // [Lmax + 1]
 };
 
-// One row of W words per lane, lane-contiguous in 16-byte quads [q][32][4],
-// then a pair [32][2] and a single [32] for the remainder: W * 32 words.
-// Word w of lane l holds nodes l * 2W + w + 1 (low half) and l * 2W + W + w + 1.
-__host__ __device__ constexpr int vitf_at(int W, int lane, int w) {
-  return w < W / 4 * 4 ? (w / 4 * 32 + lane) * 4 + w % 4
-       : (W % 4 >= 2 && w < W / 4 * 4 + 2) ? W / 4 * 128 + lane * 2 + (w - W / 4 * 4)
-                                           : W / 4 * 128 + (W % 4 >= 2 ? 64 : 0) + lane;
+// N lanes (32 per warp) score one sequence. One row of W words per lane,
+// lane-contiguous in 16-byte quads [q][N][4], then a pair [N][2] and a single
+// [N] for the remainder: W * N words. Word w of lane l holds nodes
+// l * 2W + w + 1 (low half) and l * 2W + W + w + 1.
+__host__ __device__ constexpr int vitf_at(int W, int N, int lane, int w) {
+  return w < W / 4 * 4 ? (w / 4 * N + lane) * 4 + w % 4
+       : (W % 4 >= 2 && w < W / 4 * 4 + 2) ? W / 4 * 4 * N + lane * 2 + (w - W / 4 * 4)
+                                           : W / 4 * 4 * N + (W % 4 >= 2 ? 2 * N : 0) + lane;
 }
 
 // Words 4q .. 4q+3 of a row (the last call of a row takes the remainder).
-template <int W>
+template <int W, int N>
 __device__ __forceinline__ void vitf_load(uint32_t (&e)[W], const uint32_t *__restrict__ row, int lane, int q) {
   if (q < W / 4) {
-    const uint4 v = *reinterpret_cast<const uint4 *>(row + (q * 32 + lane) * 4);
+    const uint4 v = *reinterpret_cast<const uint4 *>(row + (q * N + lane) * 4);
     e[4 * q] = v.x; e[4 * q + 1] = v.y; e[4 * q + 2] = v.z; e[4 * q + 3] = v.w;
   } else {
     if constexpr (W % 4 >= 2) {
-      const uint2 v = *reinterpret_cast<const uint2 *>(row + W / 4 * 128 + lane * 2);
+      const uint2 v = *reinterpret_cast<const uint2 *>(row + W / 4 * 4 * N + lane * 2);
       e[W / 4 * 4] = v.x; e[W / 4 * 4 + 1] = v.y;
     }
-    if constexpr (W % 2) e[W - 1] = row[W / 4 * 128 + (W % 4 >= 2 ? 64 : 0) + lane];
+    if constexpr (W % 2) e[W - 1] = row[W / 4 * 4 * N + (W % 4 >= 2 ? 2 * N : 0) + lane];
   }
 }
 
 __device__ __forceinline__ uint32_t splat16(int v) { return (uint32_t) (v & 0xffff) * 0x10001u; }
 __device__ __forceinline__ int half_max(uint32_t v) { return max((int) (int16_t) (v & 0xffffu), (int) v >> 16); }
 
-// Four words of one transition table: from registers, or from the shared copy.
-template <int W, bool REG>
-struct VitTrans {
-  uint32_t r[REG ? kFT : 1][REG ? W : 1];
-  const uint32_t *s;        // shared copy (REG false)
-  __device__ __forceinline__ void group(int t, int q, int lane, uint32_t (&o)[4]) const {
-    if constexpr (REG) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) if (4 * q + e < W) o[e] = r[t][4 * q + e];
-    } else {
-      const uint4 v = *reinterpret_cast<const uint4 *>(s + t * W * 32 + (q * 32 + lane) * 4);
-      o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
-    }
-  }
-};
-
-// Match, insert and delete cells of one row; e[] is this row's emissions and
-// is refilled from next_row behind its last use.
-template <int W, bool REG, bool SAT>
+// Match, insert and delete cells of one row from the predecessors of this
+// lane's word 0 (pM, pI, pD); em[] is this row's emissions and is refilled from
+// next_row behind its last use. Dv[0] is left to the caller; dc_out is the
+// M->D of the last word. xe and dmax: this lane's maxima.
+template <int W, int N, bool SAT>
 __device__ __forceinline__ void vitf_row(uint32_t (&Mv)[W], uint32_t (&Iv)[W], uint32_t (&Dv)[W], uint32_t (&em)[W],
-                                         const VitTrans<W, REG> &T, const uint32_t *__restrict__ next_row, int lane,
-                                         int xB, uint32_t F2, int &xe_out, int &dm_out) {
-  constexpr int NQ = (W + 3) / 4;
+                                         const uint32_t (&T)[kFT][W], const uint32_t *__restrict__ next_row, int lane,
+                                         int xB, uint32_t F2, uint32_t pM, uint32_t pI, uint32_t pD, uint32_t &dc_out,
+                                         int &xe_out, int &dm_out) {
   const uint32_t xBp = splat16(xB);
-  uint32_t sM = __shfl_up_sync(FULL, Mv[W - 1], 1), sI = __shfl_up_sync(FULL, Iv[W - 1], 1),
-           sD = __shfl_up_sync(FULL, Dv[W - 1], 1);
-  if (lane == 0) sM = sI = sD = F2;
-  // predecessors of word 0: the previous lane's last node, this lane's word W-1 low half
-  uint32_t pM = __byte_perm(sM, Mv[W - 1], 0x5432), pI = __byte_perm(sI, Iv[W - 1], 0x5432),
-           pD = __byte_perm(sD, Dv[W - 1], 0x5432);
   uint32_t xe = 0x80008000u, dmax = F2, dc = F2, sv1 = 0, dc1 = 0;
 #pragma unroll
-  for (int q = 0; q < NQ; ++q) {
-    uint32_t t[7][4];
-#pragma unroll
-    for (int j = 0; j < 7; ++j) T.group(j, q, lane, t[j]);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int w = 4 * q + e;
-      if (w >= W) break;
-      const uint32_t cM = Mv[w], cI = Iv[w], cD = Dv[w];
-      // the row's late values (D after its closure, xB) come last
-      uint32_t sv = add_s16x2(pM, t[1][e]);
-      sv = __viaddmax_s16x2(pI, t[2][e], sv);
-      sv = __viaddmax_s16x2(pD, t[3][e], sv);
-      sv = __viaddmax_s16x2(xBp, t[0][e], sv);
-      if constexpr (SAT) {
-        const uint32_t ev = em[w], en = min_s16x2(ev, 0u), ep = max_s16x2(ev, 0u);
-        sv = add_s16x2(min_s16x2(max_s16x2(sv, ~add_s16x2(en, 0x7fff7fffu)), ep ^ 0x7fff7fffu), ev);
-      } else {
-        sv = add_s16x2(sv, em[w]);
-      }
-      // running maxima, one three-input maximum per two words
-      if (w & 1) xe = __vimax3_s16x2(xe, sv1, sv);
-      else if (w == W - 1) xe = max_s16x2(xe, sv);
-      else sv1 = sv;
-      Iv[w] = __viaddmax_s16x2(cI, t[6][e], __viaddmax_s16x2(cM, t[5][e], F2));
-      const uint32_t mv = SAT ? max_s16x2(sv, F2) : sv;
-      Mv[w] = mv;
-      Dv[w] = dc;                                     // M->D from word w-1
-      dc = __viaddmax_s16x2(mv, t[4][e], F2);
-      if (w & 1) dmax = __vimax3_s16x2(dmax, dc1, dc);
-      else if (w == W - 1) dmax = max_s16x2(dmax, dc);
-      else dc1 = dc;
-      pM = cM; pI = cI; pD = cD;
+  for (int w = 0; w < W; ++w) {
+    const uint32_t cM = Mv[w], cI = Iv[w], cD = Dv[w];
+    // the row's late values (D after its closure, xB) come last
+    uint32_t sv = add_s16x2(pM, T[1][w]);
+    sv = __viaddmax_s16x2(pI, T[2][w], sv);
+    sv = __viaddmax_s16x2(pD, T[3][w], sv);
+    sv = __viaddmax_s16x2(xBp, T[0][w], sv);
+    if constexpr (SAT) {
+      const uint32_t ev = em[w], en = min_s16x2(ev, 0u), ep = max_s16x2(ev, 0u);
+      sv = add_s16x2(min_s16x2(max_s16x2(sv, ~add_s16x2(en, 0x7fff7fffu)), ep ^ 0x7fff7fffu), ev);
+    } else {
+      sv = add_s16x2(sv, em[w]);
     }
-    vitf_load<W>(em, next_row, lane, q);
+    // running maxima, one three-input maximum per two words
+    if (w & 1) xe = __vimax3_s16x2(xe, sv1, sv);
+    else if (w == W - 1) xe = max_s16x2(xe, sv);
+    else sv1 = sv;
+    Iv[w] = __viaddmax_s16x2(cI, T[6][w], __viaddmax_s16x2(cM, T[5][w], F2));
+    const uint32_t mv = SAT ? max_s16x2(sv, F2) : sv;
+    Mv[w] = mv;
+    Dv[w] = dc;                                       // M->D from word w-1
+    dc = __viaddmax_s16x2(mv, T[4][w], F2);
+    if (w & 1) dmax = __vimax3_s16x2(dmax, dc1, dc);
+    else if (w == W - 1) dmax = max_s16x2(dmax, dc);
+    else dc1 = dc;
+    pM = cM; pI = cI; pD = cD;
+    if (w % 4 == 3 || w == W - 1) vitf_load<W, N>(em, next_row, lane, w / 4);
   }
-  uint32_t sdc = __shfl_up_sync(FULL, dc, 1);
-  if (lane == 0) sdc = F2;
-  Dv[0] = __byte_perm(sdc, dc, 0x5432);
-  xe_out = __reduce_max_sync(FULL, half_max(xe));
-  dm_out = __reduce_max_sync(FULL, half_max(dmax));
+  dc_out = dc;
+  xe_out = half_max(xe);
+  dm_out = half_max(dmax);
 }
 
-// D->D closure: both halves of a lane as two chains of W nodes, then a warp
-// scan over the lanes' ends (bd[s]: the chain cost of the last 2^s lanes). A
-// value loses at least -bmax[s] over any 2^s lanes, so the scan stops where
-// even the row's largest D, dm, would end at the floor: usually before its
-// first step.
-template <int W, bool REG>
-__device__ __forceinline__ void vitf_close(uint32_t (&Dv)[W], const VitTrans<W, REG> &T, int lane, int bl, int bh,
-                                           const int (&bd)[5], const int (&bmax)[5], int F, int dm) {
-  constexpr int NQ = (W + 3) / 4;
-  uint32_t c = Dv[0];
+// Chain costs of the D->D closure: the low and the high half of a lane, sums
+// over the warp's last 1, 2, 4, 8, 16 lanes (bd) with their largest over the
+// lanes (bmax), and over the warp's lanes before this one (pre).
+struct VitChains {
+  int bl, bh, bd[5], bmax[5], pre;
+};
+template <int W>
+__device__ __forceinline__ void vitf_chains(const uint32_t (&dd)[W], int lane, VitChains &c) {
+  c.bl = c.bh = 0;
 #pragma unroll
-  for (int q = 0; q < NQ; ++q) {
-    uint32_t t[4];
-    T.group(7, q, lane, t);
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (4 * q + e > 0 && 4 * q + e < W) { c = __viaddmax_s16x2(c, t[e], Dv[4 * q + e]); Dv[4 * q + e] = c; }
-  }
-  const int clo = (int) (int16_t) (c & 0xffffu), chi = (int) c >> 16;
-  int end = max(chi, clo + bh);
+  for (int w = 0; w < W; ++w) { c.bl += (int) (int16_t) (dd[w] & 0xffffu); c.bh += (int) dd[w] >> 16; }
+  int bs = c.bl + c.bh;
+  const int own = bs;
 #pragma unroll
   for (int s = 0; s < 5; ++s) {
-    if (dm + bmax[s] <= F) break;
-    const int o = __shfl_up_sync(FULL, end, 1 << s);
-    if (lane >= (1 << s)) end = max(end, o + bd[s]);
-  }
-  int vin = __shfl_up_sync(FULL, end, 1);
-  if (lane == 0) vin = F;
-  const int vhi = max(clo, vin + bl);
-  uint32_t v = __byte_perm((uint32_t) max(vin, F), (uint32_t) max(vhi, F), 0x5410);
-  // the first word tells whether anything comes in from another chain
-  uint32_t t0[4];
-  T.group(7, 0, lane, t0);
-  const uint32_t first = __viaddmax_s16x2(v, t0[0], Dv[0]);
-  if (!__any_sync(FULL, first != Dv[0])) return;
-#pragma unroll
-  for (int q = 0; q < NQ; ++q) {
-    uint32_t t[4];
-    T.group(7, q, lane, t);
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (4 * q + e < W) { v = __viaddmax_s16x2(v, t[e], Dv[4 * q + e]); Dv[4 * q + e] = v; }
-  }
-}
-
-template <int W>
-constexpr int vitf_threads() { return W <= kVitFastRegW ? 64 : 128; }
-
-template <int W>
-__global__ void __launch_bounds__(vitf_threads<W>())
-vit_fast_kernel(VitFastDev V, DbDev db, const int64_t *__restrict__ slots, const int64_t *__restrict__ order,
-                int64_t nids, int *__restrict__ out_xc, uint8_t *__restrict__ out_st,
-                unsigned long long *__restrict__ ticket) {
-  constexpr bool REG = W <= kVitFastRegW;
-  extern __shared__ __align__(16) uint32_t s_trans[];
-  const int lane = threadIdx.x & 31;
-  VitTrans<W, REG> T;
-  T.s = s_trans;
-  if constexpr (REG) {
-#pragma unroll
-    for (int t = 0; t < kFT; ++t)
-#pragma unroll
-      for (int q = 0; q < (W + 3) / 4; ++q) vitf_load<W>(T.r[t], V.trans + t * W * 32, lane, q);
-  } else {
-    for (int i = threadIdx.x; i < kFT * W * 8; i += blockDim.x)
-      reinterpret_cast<uint4 *>(s_trans)[i] = __ldg(reinterpret_cast<const uint4 *>(V.trans) + i);
-    __syncthreads();
-  }
-  // chain costs of the closure: the low and the high half, then sums over 1, 2, 4, 8, 16 lanes
-  int bl = 0, bh = 0, bd[5], bmax[5];
-#pragma unroll
-  for (int q = 0; q < (W + 3) / 4; ++q) {
-    uint32_t t[4];
-    T.group(7, q, lane, t);
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (4 * q + e < W) { bl += (int) (int16_t) (t[e] & 0xffffu); bh += (int) t[e] >> 16; }
-  }
-  int bs = bl + bh;
-#pragma unroll
-  for (int s = 0; s < 5; ++s) {
-    bd[s] = bs;
-    bmax[s] = __reduce_max_sync(FULL, lane >= (1 << s) ? bs : -0x40000000);
+    c.bd[s] = bs;
+    c.bmax[s] = __reduce_max_sync(FULL, lane >= (1 << s) ? bs : -0x40000000);
     const int o = __shfl_up_sync(FULL, bs, 1 << s);
     if (lane >= (1 << s)) bs += o;
   }
+  c.pre = bs - own;
+}
+
+// The closure: both halves of a lane as two chains of W nodes (vitf_chain),
+// then a warp scan over the lanes' ends. A value loses at least -bmax[s] over
+// any 2^s lanes, so the scan stops where even the row's largest D, dm, would
+// end at the floor: usually before its first step. end: the value leaving
+// each lane, from within the warp.
+template <int W>
+__device__ __forceinline__ int vitf_chain(uint32_t (&Dv)[W], const uint32_t (&dd)[W], int lane, const VitChains &ch,
+                                          int F, int dm, int &clo) {
+  uint32_t c = Dv[0];
+#pragma unroll
+  for (int w = 1; w < W; ++w) { c = __viaddmax_s16x2(c, dd[w], Dv[w]); Dv[w] = c; }
+  clo = (int) (int16_t) (c & 0xffffu);
+  int end = max((int) c >> 16, clo + ch.bh);
+#pragma unroll
+  for (int s = 0; s < 5; ++s) {
+    if (dm + ch.bmax[s] <= F) break;
+    const int o = __shfl_up_sync(FULL, end, 1 << s);
+    if (lane >= (1 << s)) end = max(end, o + ch.bd[s]);
+  }
+  return end;
+}
+
+// Runs the value vin coming into the lane through both of its chains.
+template <int W>
+__device__ __forceinline__ void vitf_apply(uint32_t (&Dv)[W], const uint32_t (&dd)[W], const VitChains &ch, int F,
+                                           int vin, int clo) {
+  uint32_t v = __byte_perm((uint32_t) max(vin, F), (uint32_t) max(max(clo, vin + ch.bl), F), 0x5410);
+  // the first word tells whether anything comes in from another chain
+  const uint32_t first = __viaddmax_s16x2(v, dd[0], Dv[0]);
+  if (!__any_sync(FULL, first != Dv[0])) return;
+#pragma unroll
+  for (int w = 0; w < W; ++w) { v = __viaddmax_s16x2(v, dd[w], Dv[w]); Dv[w] = v; }
+}
+
+// One sequence of the list, NW warps: NW = 1, a warp on its own; else the
+// block's warps share it, exchanging their last lanes' cells and their maxima
+// through shared memory (two barriers a row, three with a closure).
+template <int NW>
+struct VitShared {
+  uint32_t M[2][NW], I[2][NW], D[NW], dc[NW];         // last lanes; M, I of the row's parity
+  int xe[NW], dm[NW], end[NW], sum[NW];               // maxima, closure ends, chain cost of the whole warp
+  unsigned long long t;
+};
+
+template <int W, int NW>
+__global__ void __launch_bounds__(NW == 1 ? 64 : NW * 32)
+vit_fast_kernel(VitFastDev V, DbDev db, const int64_t *__restrict__ slots, const int64_t *__restrict__ order,
+                int64_t nids, int *__restrict__ out_xc, uint8_t *__restrict__ out_st,
+                unsigned long long *__restrict__ ticket) {
+  constexpr int N = 32 * NW;
+  __shared__ VitShared<NW> sh;
+  const int lane = threadIdx.x & 31, warp = NW == 1 ? 0 : threadIdx.x >> 5, vlane = warp * 32 + lane;
+  uint32_t T[kFT][W];
+#pragma unroll
+  for (int t = 0; t < kFT; ++t)
+#pragma unroll
+    for (int q = 0; q < (W + 3) / 4; ++q) vitf_load<W, N>(T[t], V.trans + t * W * N, vlane, q);
+  VitChains ch;
+  vitf_chains<W>(T[7], lane, ch);
+  if (NW > 1 && lane == 31) sh.sum[warp] = ch.pre + ch.bl + ch.bh;
   for (;;) {
     unsigned long long t = 0;
-    if (lane == 0) t = atomicAdd(ticket, 1ull);
-    t = __shfl_sync(FULL, t, 0);
+    if constexpr (NW == 1) {
+      if (lane == 0) t = atomicAdd(ticket, 1ull);
+      t = __shfl_sync(FULL, t, 0);
+    } else {
+      __syncthreads();                                // the last sequence is done with sh
+      if (threadIdx.x == 0) sh.t = atomicAdd(ticket, 1ull);
+      __syncthreads();
+      t = sh.t;
+    }
     if (t >= (unsigned long long) nids) break;
     const int64_t j = order[t];                       // the longest sequences first
     const int64_t s = slots[j];
@@ -261,12 +237,12 @@ vit_fast_kernel(VitFastDev V, DbDev db, const int64_t *__restrict__ slots, const
       uint32_t cur = __ldg(sq), nxt = L > 4 ? __ldg(sq + 1) : 0u;
       int x = cur & 0xff;
 #pragma unroll
-      for (int q = 0; q < (W + 3) / 4; ++q) vitf_load<W>(em, V.emit + x * W * 32, lane, q);
+      for (int q = 0; q < (W + 3) / 4; ++q) vitf_load<W, N>(em, V.emit + x * W * N, vlane, q);
       for (int i = 0; i < L; ++i) {
-        // the next row's residue (padding after the last one)
         // (the largest score is taken from two rows back, whose reduction is long done)
         const bool sat = top1 > V.hot || (V.low_res >> x & 1u);
         top1 = top;
+        // the next row's residue
         if ((i & 3) == 3) {
           cur = nxt;
           if (i + 5 < L) nxt = __ldg(sq + (i >> 2) + 2);
@@ -274,49 +250,81 @@ vit_fast_kernel(VitFastDev V, DbDev db, const int64_t *__restrict__ slots, const
           cur >>= 8;
         }
         x = i + 1 < L ? (int) (cur & 0xff) : 0;
-        const uint32_t *next_row = V.emit + x * W * 32;
+        const uint32_t *next_row = V.emit + x * W * N;
+        // predecessors of word 0: the previous lane's last node, this lane's word W-1 low half
+        uint32_t sM = __shfl_up_sync(FULL, Mv[W - 1], 1), sI = __shfl_up_sync(FULL, Iv[W - 1], 1),
+                 sD = __shfl_up_sync(FULL, Dv[W - 1], 1);
+        if (lane == 0) {
+          sM = sI = sD = F2;
+          if (NW > 1 && warp > 0 && i > 0) { sM = sh.M[i & 1][warp - 1]; sI = sh.I[i & 1][warp - 1]; sD = sh.D[warp - 1]; }
+        }
+        const uint32_t pM = __byte_perm(sM, Mv[W - 1], 0x5432), pI = __byte_perm(sI, Iv[W - 1], 0x5432),
+                       pD = __byte_perm(sD, Dv[W - 1], 0x5432);
+        uint32_t dc;
         int xe, dm;
-        if (sat) vitf_row<W, REG, true>(Mv, Iv, Dv, em, T, next_row, lane, xB, F2, xe, dm);
-        else     vitf_row<W, REG, false>(Mv, Iv, Dv, em, T, next_row, lane, xB, F2, xe, dm);
+        if (sat) vitf_row<W, N, true>(Mv, Iv, Dv, em, T, next_row, vlane, xB, F2, pM, pI, pD, dc, xe, dm);
+        else     vitf_row<W, N, false>(Mv, Iv, Dv, em, T, next_row, vlane, xB, F2, pM, pI, pD, dc, xe, dm);
+        xe = __reduce_max_sync(FULL, xe);
+        dm = __reduce_max_sync(FULL, dm);
+        uint32_t sdc = __shfl_up_sync(FULL, dc, 1);
+        if (lane == 0) sdc = F2;
+        if constexpr (NW > 1) {
+          if (lane == 31) {
+            sh.M[~i & 1][warp] = Mv[W - 1]; sh.I[~i & 1][warp] = Iv[W - 1];
+            sh.dc[warp] = dc; sh.xe[warp] = xe; sh.dm[warp] = dm;
+          }
+          __syncthreads();
+          if (lane == 0 && warp > 0) sdc = sh.dc[warp - 1];
+#pragma unroll
+          for (int k = 0; k < NW; ++k) { xe = max(xe, sh.xe[k]); dm = max(dm, sh.dm[k]); }
+        }
+        Dv[0] = __byte_perm(sdc, dc, 0x5432);
         top = max(top, xe);
         xC = (int16_t) max(xC + V.xwC_loop, xe + V.xwE_move);
         xJ = max(xJ, xe + V.xwE_loop);
         xB = max(xJ, xN) + move;
         if (dm + V.ddbound_w > xB || xe >= 32767) {
           if (xe >= 32767) { xC = 32767; st = 1; break; }   // eslERANGE
-          vitf_close<W, REG>(Dv, T, lane, bl, bh, bd, bmax, F, dm);
+          int clo;
+          const int end = vitf_chain<W>(Dv, T[7], lane, ch, F, dm, clo);
+          int vin = __shfl_up_sync(FULL, end, 1), into = F;
+          if constexpr (NW > 1) {                     // the earlier warps' ends, carried through the warps between
+            if (lane == 31) sh.end[warp] = end;
+            __syncthreads();
+            for (int k = 0; k < warp; ++k) into = max(sh.end[k], into + sh.sum[k]);
+          }
+          vin = lane == 0 ? into : NW > 1 ? max(vin, into + ch.pre) : vin;
+          vitf_apply<W>(Dv, T[7], ch, F, vin, clo);
+        }
+        if constexpr (NW > 1) {
+          if (lane == 31) sh.D[warp] = Dv[W - 1];
+          __syncthreads();
         }
       }
     }
-    if (lane == 0) { out_xc[j] = xC; out_st[j] = (uint8_t) st; }
+    if (vlane == 0) { out_xc[j] = xC; out_st[j] = (uint8_t) st; }
   }
 }
 
-template <int W>
+template <int W, int NW>
 cudaError_t launch_vit_fast(const VitFastDev &V, const DbDev &db, const int64_t *ids, const int64_t *order, int64_t n,
                             int *xc, uint8_t *st, unsigned long long *ticket, int sms, cudaStream_t stream) {
-  constexpr int threads = vitf_threads<W>();
-  constexpr size_t smem = W <= kVitFastRegW ? 0 : (size_t) kFT * W * 32 * 4;
-  auto kern = vit_fast_kernel<W>;
-  static std::atomic<unsigned long long> configured{0};
-  if (smem) {
-    const cudaError_t e = ensure_smem_attr((const void *) kern, smem, configured);
-    if (e != cudaSuccess) return e;
-  }
+  constexpr int threads = NW == 1 ? 64 : NW * 32, per_block = threads / 32 / NW;
+  auto kern = vit_fast_kernel<W, NW>;
   int per_sm = 0;
-  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
+  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, 0);
   if (e != cudaSuccess) return e;
   long long grid = (long long) (per_sm < 1 ? 1 : per_sm) * sms;
-  const long long need = (n + threads / 32 - 1) / (threads / 32);
+  const long long need = (n + per_block - 1) / per_block;
   if (need < grid) grid = need < 1 ? 1 : need;
   (void) cudaGetLastError();
-  kern<<<(unsigned) grid, threads, smem, stream>>>(V, db, ids, order, n, xc, st, ticket);
+  kern<<<(unsigned) grid, threads, 0, stream>>>(V, db, ids, order, n, xc, st, ticket);
   return cudaGetLastError();
 }
 
 }  // namespace msvgb
 
-#define MSVGB_INSTANTIATE_VITF(W)                                                                          \
-  template cudaError_t msvgb::launch_vit_fast<W>(const msvgb::VitFastDev &, const msvgb::DbDev &,          \
+#define MSVGB_INSTANTIATE_VITF(W, NW)                                                                      \
+  template cudaError_t msvgb::launch_vit_fast<W, NW>(const msvgb::VitFastDev &, const msvgb::DbDev &,          \
                                                  const int64_t *, const int64_t *, int64_t, int *, uint8_t *, \
                                                  unsigned long long *, int, cudaStream_t);

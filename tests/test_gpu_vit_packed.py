@@ -67,10 +67,29 @@ def check(ctx, vp, s):
     return st
 
 
+def resized(vp, M):
+    """A profile of M nodes: cropped, or its inner nodes repeated."""
+    if M <= vp.M:
+        return crop_vprofile(vp, M)
+    k = np.arange(M)
+    src = np.where(k == 0, 0, 1 + (k - 1) % (vp.M - 2))
+    Q0, Q8 = vp.Q8, (M - 1) // 8 + 1
+    tw = np.full((8 * Q8, 8), -32768, np.int16)
+    rw = np.full((vp.Kp, Q8, 8), -32768, np.int16)
+    for t in range(7):
+        tw[k % Q8 * 7 + t, k // Q8] = vp.twv[src % Q0 * 7 + t, src // Q0]
+    tw[7 * Q8 + k % Q8, k // Q8] = vp.twv[7 * Q0 + src % Q0, src // Q0]
+    for t in (4, 5, 6):
+        tw[(M - 1) % Q8 * 7 + t, (M - 1) // Q8] = -32768
+    tw[7 * Q8 + (M - 1) % Q8, (M - 1) // Q8] = -32768
+    rw[:, k % Q8, k // Q8] = vp.rwv[:, src % Q0, src // Q0]
+    return F.VProfile(M, tw, rw, vp.xw, vp.scale_w, vp.nj, vp.base_w, vp.ddbound_w)
+
+
 @pytest.mark.parametrize("M", [1, 2, 5, 63, 64, 65, 127, 128, 129, 511, 512, 513, 896, 897, 1024, 1025, 1280, 1281,
-                               2303, 2304, 2399])
+                               2303, 2304, 2399, 3072, 3584, 3585, 4096, 4097, 5120, 6200, 8191, 8192])
 def test_row_widths(ctx, M):
-    vp = crop_vprofile(vprofile("m2400_s1"), M)
+    vp = resized(vprofile("m2400_s1"), M)
     check(ctx, vp, targets(vp, M))
 
 
