@@ -149,12 +149,7 @@ template <int C, int G, int CI> cudaError_t launch_ssv_group(const GroupArgs &a,
 // below 10 words (4 lost 2.5% at M = 120), 4 up to 17 words (+4 to +7%), 8
 // from 18 words (+7 to +10%; 12 and 16 were slower than 8 everywhere); at 16
 // lanes 4 up to 23 words (+3 to +9%), 8 from 24 (+8%).
-int msvgb_detail::hyb_default_words(int C, int G) {
-  if (G == 8) return C < 10 ? 0 : C < 18 ? 4 : 8;
-  if (G == 16) return C < 13 ? 0 : C < 24 ? 4 : 8;
-  if (G == 32) return C < 17 ? 0 : 8;     // the split 32-lane passes (M 1024-2047): always mixed width
-  return 0;
-}
+int msvgb_detail::hyb_default_words(int C, int G) { return msvgb::hyb_words(C, G); }
 
 bool msvgb_detail::hyb_compiled(int C, int G, int CI) {
 #define MSVGB_HYB_HAS(c, g, ci) if (C == c && G == g && CI == ci) return true;
@@ -190,21 +185,22 @@ namespace msvgb {
 template <int C, int G>
 cudaError_t launch_list_group(const ProfDev &P, const DbDev &db, uint8_t *out_xj, uint8_t *out_flags,
                               unsigned long long *ticket, const int64_t *list, const unsigned long long *list_count,
-                              int num_sms, cudaStream_t stream);
+                              const SegDev &segs, int num_sms, cudaStream_t stream);
 }
 
 cudaError_t msvgb_detail::dispatch_list_group(int C, int G, const ProfDev &P, const DbDev &db, uint8_t *out_xj,
                                               uint8_t *out_flags, unsigned long long *ticket, const int64_t *list,
-                                              const unsigned long long *list_count, int sms, cudaStream_t stream) {
-#define L32(c) case c: return launch_list_group<c, 32>(P, db, out_xj, out_flags, ticket, list, list_count, sms, stream);
+                                              const unsigned long long *list_count, const SegDev &segs, int sms,
+                                              cudaStream_t stream) {
+#define L32(c) case c: return launch_list_group<c, 32>(P, db, out_xj, out_flags, ticket, list, list_count, segs, sms, stream);
   if (G == 32) {
     switch (C) { L32(17) L32(18) L32(19) L32(20) L32(21) L32(22) L32(23) L32(24) L32(25) L32(26) L32(27)
                  L32(28) L32(29) L32(30) L32(31) L32(32) }
     return cudaErrorInvalidValue;
   }
 #undef L32
-#define L16(c) case c: return launch_list_group<c, 16>(P, db, out_xj, out_flags, ticket, list, list_count, sms, stream);
-#define L8(c)  case c: return launch_list_group<c, 8>(P, db, out_xj, out_flags, ticket, list, list_count, sms, stream);
+#define L16(c) case c: return launch_list_group<c, 16>(P, db, out_xj, out_flags, ticket, list, list_count, segs, sms, stream);
+#define L8(c)  case c: return launch_list_group<c, 8>(P, db, out_xj, out_flags, ticket, list, list_count, segs, sms, stream);
   if (G == 16) {
     switch (C) { L16(2) L16(3) L16(4) L16(5) L16(6) L16(7) L16(8) L16(9) L16(10) L16(11) L16(12) L16(13)
                  L16(14) L16(15) L16(16) L16(17) L16(18) L16(19) L16(20) L16(21) L16(22) L16(23) L16(24)
@@ -233,10 +229,8 @@ extern "C" int msvgb_ctx_create(int device, msvgb_ctx **ret_ctx) {
   c->device = device;
   cudaError_t e = cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMalloc(&c->d_ticket, sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMalloc(&c->d_out, 64);
+  if (e == cudaSuccess) e = cudaMalloc(&c->d_ticket, 4 * sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaMalloc(&c->d_bad, sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&c->d_aux, 4 * sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->upload, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->dma, cudaStreamNonBlocking);
@@ -263,8 +257,8 @@ extern "C" int msvgb_ctx_destroy(msvgb_ctx *c) {
   for (auto &e : c->dropin) msvgb_profile_destroy(e.p);
   c->dropin.clear();
   if (c->own) cudaStreamSynchronize(c->own);
-  cudaFree(c->d_ticket); cudaFree(c->d_out);
-  cudaFree(c->d_one); cudaFree(c->d_bad); cudaFree(c->d_aux); cudaFree(c->d_list);
+  cudaFree(c->d_ticket);
+  cudaFree(c->d_one); cudaFree(c->d_bad); cudaFree(c->d_list); cudaFree(c->d_seg);
   if (c->own) cudaStreamDestroy(c->own);
   if (c->side) { cudaStreamSynchronize(c->side); cudaStreamDestroy(c->side); }
   if (c->upload) { cudaStreamSynchronize(c->upload); cudaStreamDestroy(c->upload); }
@@ -1090,6 +1084,12 @@ extern "C" int64_t msvgb_db_residues(const msvgb_db *db) { return db ? db->resid
 // ------------------------------------------------------------------------------
 // search
 
+// Lanes or 8-bit words set by the caller keep their documented launches (long
+// targets at 32 lanes); other searches may cut their long targets.
+static bool may_cut(const msvgb_profile *p) {
+  return !p->d_stab_g || (p->lanes_auto && p->CI == msvgb_detail::hyb_default_words(p->Cg, p->G));
+}
+
 extern "C" int msvgb_search_device(msvgb_ctx *c, const msvgb_profile *pc, const msvgb_db *db, double F1,
                                    void *d_xj, void *d_flags) {
   if (!c || !pc || !db || (!d_xj && db->n) || (!d_flags && db->n)) return fail(MSVGB_eslEINVAL, "NULL argument");
@@ -1108,10 +1108,80 @@ extern "C" int msvgb_search_device(msvgb_ctx *c, const msvgb_profile *pc, const 
     c->list_cap = db->n;
   }
   SearchScratch sc;
+  sc.cut = may_cut(p);
+  if (sc.cut) sc.segs = plan_segments(p, db, c->num_sms);
+  const size_t need = seg_bytes(sc.segs);
+  if (c->seg_cap < need) {
+    CUDA_TRY(cudaStreamSynchronize(c->stream));            // as the list
+    cudaFree(c->d_seg); c->d_seg = nullptr; c->seg_cap = 0;
+    CUDA_TRY(cudaMalloc(&c->d_seg, need));
+    c->seg_cap = need;
+  }
+  sc.seg = c->d_seg;
   sc.stream = c->stream; sc.side = c->side; sc.ev_fork = c->ev_fork; sc.ev_join = c->ev_join;
-  sc.ticket = c->d_ticket; sc.aux = c->d_aux; sc.list = c->d_list;
+  sc.counters = c->d_ticket; sc.list = c->d_list;
   return enqueue_search(sc, p, db, t, (uint8_t *) d_xj, (uint8_t *) d_flags, c->num_sms);
 }
+
+// Whether the search of a profile that chose its lanes itself runs at 32
+// lanes in the fused kernel: where the database is too small to fill the lane
+// groups, by its residues. Lane groups / fused, us: M = 60, 19M residues
+// 295 / 304, 23M 322 / 379; 120, 23M 410 / 395; 160, 23M 460 / 535; 200, 23M
+// 480 / 487; 240, 25M 604 / 550; 400, 23M 749 / 697, 31M 906 / 1111; from 512
+// nodes later: 520, 38M 1457 / 1348; 800, 34M 1734 / 1654; 1200, 23M 1813 /
+// 1575, 34M 2448 / 2337; 2000, 23M 2663 / 2527.
+constexpr int64_t kFusedShort = 24000000, kFusedLong = 36000000;
+static bool search_fused(const msvgb_profile *p, const msvgb_db *db, bool others) {
+  return !p->d_stab_g || (p->lanes_auto && !others && db->residues < (p->M < 512 ? kFusedShort : kFusedLong));
+}
+
+// The segments of a search's long targets. A segment costs its run-in of M
+// rows, so none is shorter than 2 M, and only as many are cut as the chains
+// the launch holds can use: T is the rows each of them scores on average
+// (24 warps per SM in the lane-group pass, 32 in the fused kernel, 16 where
+// its tables leave one block per SM). 20,000 targets up to 35,000 rows, M =
+// 2400: 6.81 ms (half of that T 7.45, uncut 15.5). R, the rows of a block
+// that the full MSV may skip: 128 in the fused kernel (M = 200, 20,000
+// targets: 207 us; 256 212 to 238, 512 265, 1024 364), 256 in the lane-group
+// pass, whose list kernel reads them (M = 86, 500,000 targets: 1272 us; 128
+// 1325, 512 1430).
+SegDev msvgb_detail::plan_segments(const msvgb_profile *p, const msvgb_db *db, int num_sms, bool others) {
+  SegDev g;
+  const int M = p->M;
+  const bool fused = search_fused(p, db, others);
+  const double chains = (double) num_sms * (fused ? (p->C > 32 ? 16.0 : 32.0) : 24.0 * 32.0 / p->G);
+  const double avg = (double) db->residues / chains;
+  if (db->Lmax < avg / 2) return SegDev();                // no chain sets the search's length
+  const double T = std::max({avg, 2.0 * M, 768.0, (double) db->Lmax / kMaxSegs});
+  if (T > 1e8) return SegDev();
+  g.R = fused ? 128 : 256;
+  g.T = ((int) T + g.R - 1) / g.R * g.R;
+  g.warm = (M + 15) / 16 * 16;
+  const int cut = 2 * std::max(M, g.R);                   // shorter targets stay whole
+  if (db->Lmax < cut) return SegDev();
+  g.S = (db->Lmax + g.T - 1) / g.T;
+  g.NB = (db->Lmax + g.R - 1) / g.R;
+  if (g.S > kMaxSegs) return SegDev();
+  // sequences with more than k * T rows, longest first
+  int64_t longer[kMaxSegs] = {}, c = 0;
+  size_t i = db->distinct_len.size();
+  for (int k = g.S - 1; k >= 0; --k) {
+    const int64_t at = std::max<int64_t>(cut, (int64_t) k * g.T + 1);
+    while (i > 0 && db->distinct_len[i - 1] >= at) c += db->len_count[--i];
+    longer[k] = c;
+  }
+  g.nl = longer[0];
+  int64_t total = 0;
+  for (int k = 0; k < g.S; ++k) {
+    g.base[k] = (uint32_t) total;
+    total += longer[k];
+  }
+  if (total > (int64_t) 1 << 30 || g.nl * g.NB > (int64_t) 1 << 30) return SegDev();
+  for (int k = g.S; k <= kMaxSegs; ++k) g.base[k] = (uint32_t) total;
+  return g;
+}
+
+size_t msvgb_detail::seg_bytes(const SegDev &g) { return (size_t) g.nl * (4 + g.NB); }
 
 int msvgb_detail::enqueue_search(const SearchScratch &sc, const msvgb_profile *p, const msvgb_db *db,
                                  const LenTables *t, uint8_t *d_xj, uint8_t *d_flags, int num_sms) {
@@ -1119,41 +1189,43 @@ int msvgb_detail::enqueue_search(const SearchScratch &sc, const msvgb_profile *p
   ProfDev P32;
   P32.M = p->M; P32.C = p->C; P32.tbm = p->tbm; P32.tec = p->tec; P32.base = p->base; P32.bias = p->bias;
   P32.stab = p->d_stab; P32.mtab = p->d_mtab; P32.tjb = t->d_tjb; P32.xjmin = t->d_xjmin; P32.ssv_f16 = p->f16;
-  // Lane groups lengthen each sequence's latency (2-4x): below ~40 G cells the
-  // launch tail they add outweighs their throughput, unless lanes were set
-  // explicitly.
-  const bool small = p->lanes_auto && (double) p->M * (double) db->residues < 4e10;
-  if (!p->d_stab_g || small) {
+  SegDev segs;
+  if (sc.cut && sc.segs.S) {
+    segs = sc.segs;
+    segs.done = (uint32_t *) sc.seg;
+    segs.u = sc.seg + (size_t) segs.nl * 4;
+    CUDA_TRY(cudaMemsetAsync(segs.done, 0, (size_t) segs.nl * 4, sc.stream));
+  }
+  // counters: the main pass's ticket, the list's ticket, the list's count, the long targets' ticket
+  unsigned long long *ctr = sc.counters;
+  CUDA_TRY(cudaMemsetAsync(ctr, 0, 4 * sizeof(unsigned long long), sc.stream));
+  if (search_fused(p, db, sc.others)) {
     LaunchArgs a;
-    a.P = P32; a.db = dbv; a.out_xj = d_xj; a.out_flags = d_flags; a.ticket = sc.ticket;
-    a.stream = sc.stream; a.grid = 0; a.skip_empty = 1;
-    CUDA_TRY(cudaMemsetAsync(sc.ticket, 0, sizeof(unsigned long long), sc.stream));
+    a.P = P32; a.db = dbv; a.out_xj = d_xj; a.out_flags = d_flags; a.ticket = ctr;
+    a.stream = sc.stream; a.grid = 0; a.skip_empty = 1; a.segs = segs;
     CUDA_TRY(dispatch(p->C, p->f16 != 0, a, num_sms));
     count_launch();
     return MSVGB_eslOK;
   }
-  // Long targets (they sort first) on the 32-lane kernel, in the side stream
-  // when there is one; the rest: the G-lane SSV pass, then the full MSV on the
-  // sequences it left undecided. The side stream forks from and joins back
-  // into the search's. Targets too long for a lane group to finish within the
-  // pass go to 32 lanes: with the longest first, a group's latency only
-  // matters beyond about a third of the rows each group scores on average
-  // (SMs x 32 warps x 32/G groups), and never below kLongTarget residues.
+  // The G-lane SSV pass, then the full MSV on the sequences it left undecided.
+  // Where they are not cut, long targets (they sort first) run on the
+  // 32-lane kernel, in the side stream when there is one (forked from and
+  // joined back into the search's): those too long for a lane group to finish
+  // within the pass, beyond about a third of the rows each group scores on
+  // average (SMs x 32 warps x 32/G groups), and never below kLongTarget.
   const double groups = (double) num_sms * 32.0 * (32.0 / p->G);
   const int t_long = (int) std::min<double>(1e9, std::max<double>(kLongTarget, (double) db->residues / groups / 3.0));
-  const int64_t n_long = std::min(db->count_at_least(t_long), db->n);
+  const int64_t n_long = sc.cut ? 0 : std::min(db->count_at_least(t_long), db->n);
   ProfDev P;
   P.M = p->M; P.C = p->Cg; P.tbm = p->tbm; P.tec = p->tec; P.base = p->base; P.bias = p->bias;
   P.stab = p->d_stab_g; P.mtab = p->d_mtab; P.tjb = t->d_tjb; P.xjmin = t->d_xjmin; P.ssv_f16 = 1;
   GroupArgs g;
   g.P = P; g.db = dbv; g.out_xj = d_xj; g.out_flags = d_flags;
-  g.ticket = sc.ticket; g.undecided = sc.list; g.n_undecided = sc.aux + 1; g.stream = sc.stream;
-  g.s_begin = n_long;
-  CUDA_TRY(cudaMemsetAsync(sc.ticket, 0, sizeof(unsigned long long), sc.stream));
-  CUDA_TRY(cudaMemsetAsync(sc.aux, 0, 3 * sizeof(unsigned long long), sc.stream));
+  g.ticket = ctr; g.undecided = sc.list; g.n_undecided = ctr + 2; g.stream = sc.stream;
+  g.s_begin = n_long; g.segs = segs;
   if (n_long > 0) {
     LaunchArgs l;
-    l.P = P32; l.db = dbv; l.out_xj = d_xj; l.out_flags = d_flags; l.ticket = sc.aux + 2;
+    l.P = P32; l.db = dbv; l.out_xj = d_xj; l.out_flags = d_flags; l.ticket = ctr + 3;
     l.stream = sc.side ? sc.side : sc.stream; l.grid = 0; l.skip_empty = 1; l.range_end = n_long;
     if (sc.side) {
       CUDA_TRY(cudaEventRecord(sc.ev_fork, sc.stream));
@@ -1167,17 +1239,10 @@ int msvgb_detail::enqueue_search(const SearchScratch &sc, const msvgb_profile *p
     CUDA_TRY(dispatch_group(p->Cg, p->G, p->CI, g, num_sms));
     count_launch();
   }
-  if (p->d_mtab_g) {                                       // the full MSV on the same lane groups
-    ProfDev Pl = P;
-    Pl.mtab = p->d_mtab_g;
-    CUDA_TRY(dispatch_list_group(p->Cg, p->G, Pl, dbv, d_xj, d_flags, sc.aux, sc.list, sc.aux + 1, num_sms,
-                                 sc.stream));
-  } else {
-    LaunchArgs a;
-    a.P = P32; a.db = dbv; a.out_xj = d_xj; a.out_flags = d_flags; a.ticket = sc.aux;
-    a.stream = sc.stream; a.grid = 0; a.skip_empty = 1; a.list = sc.list; a.list_count = sc.aux + 1;
-    CUDA_TRY(dispatch(p->C, p->f16 != 0, a, num_sms));
-  }
+  ProfDev Pl = P;                                          // the full MSV on the same lane groups
+  Pl.mtab = p->d_mtab_g;
+  CUDA_TRY(dispatch_list_group(p->Cg, p->G, Pl, dbv, d_xj, d_flags, ctr + 1, sc.list, ctr + 2, segs, num_sms,
+                               sc.stream));
   count_launch();
   if (n_long > 0 && sc.side) CUDA_TRY(cudaStreamWaitEvent(sc.stream, sc.ev_join, 0));
   return MSVGB_eslOK;
@@ -1189,7 +1254,9 @@ extern "C" int msvgb_search(msvgb_ctx *c, const msvgb_profile *p, const msvgb_db
   if (db->n == 0) return MSVGB_eslOK;
   CUDA_TRY(cudaSetDevice(c->device));
   uint8_t *d = nullptr;
-  CUDA_TRY(cudaMallocAsync((void **) &d, 2 * (size_t) db->n, c->stream));
+  cudaMemPool_t pool = msvgb_detail::scratch_pool(c->device);   // stays mapped between calls
+  if (!pool) return fail(MSVGB_eslESYS, "search: no memory pool");
+  CUDA_TRY(cudaMallocFromPoolAsync((void **) &d, 2 * (size_t) db->n, pool, c->stream));
   int st = msvgb_search_device(c, p, db, F1, d, d + db->n);
   if (st == MSVGB_eslOK) {
     cudaError_t e = cudaMemcpyAsync(out_xj, d, db->n, cudaMemcpyDeviceToHost, c->stream);
@@ -1217,13 +1284,29 @@ static int search_chunked(msvgb_ctx *c, const msvgb_profile *p, msvgb_db *db, co
   using namespace msvgb_detail;
   const int sms = c->num_sms;
   cudaStream_t S[2] = {c->stream, c->upload};
+  const int K = (int) db->chunk_slot.size() - 1;
+  if (K == 1) {                                             // a resident search behind the packing
+    int st = pack_chunk_on(c, db, 0, S[0]);
+    if (st != MSVGB_eslOK) return st;
+    release_chunks_on(db, S[0]);
+    gt.mark("packed", S[0]);
+    SearchScratch sc;
+    sc.stream = S[0]; sc.side = c->side; sc.ev_fork = c->ev_fork; sc.ev_join = c->ev_join;
+    sc.counters = ctr; sc.list = list;
+    sc.cut = may_cut(p);
+    if (sc.cut) sc.segs = plan_segments(p, db, sms);
+    const size_t need = seg_bytes(sc.segs);
+    if (need) CUDA_TRY(cudaMallocFromPoolAsync((void **) &sc.seg, need, scratch_pool(c->device), S[0]));
+    st = enqueue_search(sc, p, db, t, d_xj, d_flags, sms);
+    if (need) cudaFreeAsync(sc.seg, S[0]);
+    gt.mark("passed", S[0]);
+    return st;
+  }
   const DbDev full{db->d_codes, db->d_start, db->d_len, db->d_orig, db->n};
   ProfDev P32;
   P32.M = p->M; P32.C = p->C; P32.tbm = p->tbm; P32.tec = p->tec; P32.base = p->base; P32.bias = p->bias;
   P32.stab = p->d_stab; P32.mtab = p->d_mtab; P32.tjb = t->d_tjb; P32.xjmin = t->d_xjmin; P32.ssv_f16 = p->f16;
-  // as in enqueue_search: lane groups only where the whole search is large
-  const bool small = p->lanes_auto && (double) p->M * (double) db->residues < 4e10;
-  const bool groups = p->d_stab_g && !small;
+  const bool groups = !search_fused(p, db, false);          // as in enqueue_search, by the whole search
   ProfDev P = P32;
   int t_long = INT32_MAX;
   if (groups) {
@@ -1231,7 +1314,6 @@ static int search_chunked(msvgb_ctx *c, const msvgb_profile *p, msvgb_db *db, co
     const double ngroups = (double) sms * 32.0 * (32.0 / p->G);
     t_long = (int) std::min<double>(1e9, std::max<double>(kLongTarget, (double) db->residues / ngroups / 3.0));
   }
-  const int K = (int) db->chunk_slot.size() - 1;
   for (int k = 0; k < K; ++k) {
     cudaStream_t s = S[k & 1];
     unsigned long long *tk_long = ctr + (k & 1), *tk = ctr + 2 + (k & 1);
@@ -1264,16 +1346,9 @@ static int search_chunked(msvgb_ctx *c, const msvgb_profile *p, msvgb_db *db, co
   CUDA_TRY(cudaStreamWaitEvent(S[0], c->ev_join, 0));
   release_chunks_on(db, S[0]);
   if (groups) {                                             // the full MSV of the undecided sequences
-    if (p->d_mtab_g) {
-      ProfDev Pl = P;
-      Pl.mtab = p->d_mtab_g;
-      CUDA_TRY(dispatch_list_group(p->Cg, p->G, Pl, full, d_xj, d_flags, ctr + 5, list, ctr + 4, sms, S[0]));
-    } else {
-      LaunchArgs a;
-      a.P = P32; a.db = full; a.out_xj = d_xj; a.out_flags = d_flags; a.ticket = ctr + 5;
-      a.stream = S[0]; a.grid = 0; a.skip_empty = 1; a.list = list; a.list_count = ctr + 4;
-      CUDA_TRY(dispatch(p->C, p->f16 != 0, a, sms));
-    }
+    ProfDev Pl = P;
+    Pl.mtab = p->d_mtab_g;
+    CUDA_TRY(dispatch_list_group(p->Cg, p->G, Pl, full, d_xj, d_flags, ctr + 5, list, ctr + 4, SegDev(), sms, S[0]));
     count_launch();
     gt.mark("list passed", S[0]);
   }
@@ -1323,10 +1398,12 @@ int msvgb_detail::host_search(msvgb_ctx *c, const msvgb_profile *pc, const uint8
   const size_t o_bad = (2 * (size_t) n + 15) / 16 * 16, o_ctr = o_bad + 16;
   uint8_t *d = nullptr;
   int64_t *d_list = nullptr;
-  CUDA_TRY(cudaMallocAsync((void **) &d, o_ctr + 6 * sizeof(unsigned long long), c->stream));
+  cudaMemPool_t pool = scratch_pool(c->device);             // stays mapped between calls
+  if (!pool) return fail(MSVGB_eslESYS, "search: no memory pool");
+  CUDA_TRY(cudaMallocFromPoolAsync((void **) &d, o_ctr + 6 * sizeof(unsigned long long), pool, c->stream));
   int *d_bad = (int *) (d + o_bad);
   unsigned long long *ctr = (unsigned long long *) (d + o_ctr);
-  cudaError_t e = cudaMallocAsync((void **) &d_list, sizeof(int64_t) * (size_t) n, c->stream);
+  cudaError_t e = cudaMallocFromPoolAsync((void **) &d_list, sizeof(int64_t) * (size_t) n, pool, c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d + o_bad, 0, 16 + 6 * sizeof(unsigned long long), c->stream);
   if (e == cudaSuccess) e = cudaEventRecord(c->ev_fork, c->stream);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(c->upload, c->ev_fork, 0);   // scratch ready before any pack
@@ -1476,49 +1553,59 @@ extern "C" int msvgb_MSVFilter(msvgb_ctx *c, const uint8_t *dsq, int L, const ms
   int st = dropin_profile(c, om, &p);
   if (st != MSVGB_eslOK) return st;
   // One block, staged in pinned memory and uploaded in one copy:
-  // [0, 64) ticket (zero) and the one-sequence database arrays (start = 0,
-  // orig = 0, len); [64, 64 + T) the tjb table (the caller's om->tjb_b at
-  // index L, the reference reads om->tjb_b as set) then the xjmin table (255:
-  // the pass flag is unused here); then the residues padded to 16 bytes with
-  // the pad code.
+  // [0, 64) ticket (zero), the one-sequence database arrays (start = 0,
+  // orig = 0, len) and a zero count of finished segments; [64, 128) segment
+  // maxima; [128, 128 + T) the tjb table (the caller's om->tjb_b at index L,
+  // the reference reads om->tjb_b as set) then the xjmin table (255: the pass
+  // flag is unused here); then the residues padded to 16 bytes with the pad
+  // code. The kernel writes its two result bytes into pinned memory after it.
   const size_t T = ((2 * ((size_t) L + 1)) + 15) / 16 * 16;
   const size_t padded = ((size_t) L + 15) / 16 * 16 + 64;
-  const size_t bytes = 64 + T + padded;
+  const size_t bytes = 128 + T + padded;
   if (c->h_one_cap < bytes || c->d_one_cap < bytes) {
     CUDA_TRY(cudaStreamSynchronize(c->stream));               // nothing still reads the old blocks
     const size_t cap = std::max<size_t>(bytes, 16384);
     if (c->h_one) cudaFreeHost(c->h_one);
     cudaFree(c->d_one);
     c->h_one = nullptr; c->d_one = nullptr; c->h_one_cap = c->d_one_cap = 0;
-    CUDA_TRY(cudaMallocHost((void **) &c->h_one, cap));
+    CUDA_TRY(cudaMallocHost((void **) &c->h_one, cap + 64));
     c->h_one_cap = cap;
     CUDA_TRY(cudaMalloc((void **) &c->d_one, cap));
     c->d_one_cap = cap;
   }
   uint8_t *h = c->h_one;
-  memset(h, 0, 64);
+  memset(h, 0, 128);
   const int32_t len32 = L;
   memcpy(h + 32, &len32, 4);                                  // [8,16) start = 0, [16,24) orig = 0, [32,36) len
-  memset(h + 64, 0, T);
-  h[64 + L] = om->tjb_b;
-  h[64 + (L + 1) + L] = 255;
-  uint8_t *hs = h + 64 + T;
+  memset(h + 128, 0, T);
+  h[128 + L] = om->tjb_b;
+  h[128 + (L + 1) + L] = 255;
+  uint8_t *hs = h + 128 + T;
   if (L) memcpy(hs, dsq + 1, (size_t) L);
   memset(hs + L, PAD_CODE, padded - (size_t) L);
   uint8_t *d = c->d_one;
   CUDA_TRY(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, c->stream));
-  const DbDev dbv{d + 64 + T, (const int64_t *) (d + 8), (const int32_t *) (d + 32), (const int64_t *) (d + 16), 1};
+  const DbDev dbv{d + 128 + T, (const int64_t *) (d + 8), (const int32_t *) (d + 32), (const int64_t *) (d + 16), 1};
   ProfDev P;
   P.M = p->M; P.C = p->C; P.tbm = p->tbm; P.tec = p->tec; P.base = p->base; P.bias = p->bias;
-  P.stab = p->d_stab; P.mtab = p->d_mtab; P.tjb = d + 64; P.xjmin = d + 64 + L + 1; P.ssv_f16 = p->f16;
+  P.stab = p->d_stab; P.mtab = p->d_mtab; P.tjb = d + 128; P.xjmin = d + 128 + L + 1; P.ssv_f16 = p->f16;
+  volatile uint8_t *res = h + c->h_one_cap;                   // pinned: the kernel's two result bytes
   LaunchArgs a;
-  a.P = P; a.db = dbv; a.out_xj = c->d_out; a.out_flags = c->d_out + 1;
+  a.P = P; a.db = dbv; a.out_xj = (uint8_t *) res; a.out_flags = (uint8_t *) res + 1;
+  // the block's 8 warps share a sequence whose segments, run-in included, are
+  // well below its length
+  const int warm = (om->M + 15) / 16 * 16, rows = ((L + 7) / 8 + 15) / 16 * 16;
+  if (rows + warm < L - L / 4) {
+    SegDev &g = a.segs;
+    g.nl = 1; g.T = g.R = rows; g.warm = warm;
+    g.S = g.NB = (L + rows - 1) / rows;
+    for (int k = 0; k <= kMaxSegs; ++k) g.base[k] = (uint32_t) std::min(k, g.S);
+    g.u = d + 64; g.done = (uint32_t *) (d + 40);
+  }
   a.ticket = (unsigned long long *) d;
   a.stream = c->stream; a.grid = 1; a.skip_empty = 0;
   CUDA_TRY(dispatch(p->C, p->f16 != 0, a, c->num_sms));
   g_launches.fetch_add(1);
-  uint8_t *res = h;                                           // the results come back into the staged block
-  CUDA_TRY(cudaMemcpyAsync(res, c->d_out, 2, cudaMemcpyDeviceToHost, c->stream));
   CUDA_TRY(cudaStreamSynchronize(c->stream));
   if (res[1] & MSVGB_FLAG_ERANGE) { *ret_sc = INFINITY; return MSVGB_eslERANGE; }
   *ret_sc = score_from_xj(res[0], om->tjb_b, om->base_b, om->scale_b);

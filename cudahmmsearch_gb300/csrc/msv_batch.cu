@@ -104,6 +104,7 @@ struct msvgb_batch {
   // per branch of those searches: its scratch (ticket, 3 counters, list) and capture stream
   unsigned long long *d_solo_counters[kSoloBranches] = {};
   int64_t *d_solo_list[kSoloBranches] = {};
+  uint8_t *d_solo_seg[kSoloBranches] = {};               // segments of the long targets
   cudaStream_t branch[kSoloBranches] = {};
   cudaEvent_t ev[kSoloBranches + 1] = {};                // per branch: joined; last: forked
 };
@@ -117,7 +118,7 @@ extern "C" int msvgb_batch_destroy(msvgb_batch *b) {
   for (auto *t : b->gtabs) cudaFree(t);
   for (auto *p : b->own) msvgb_profile_destroy(p);
   for (int k = 0; k < kSoloBranches; ++k) {
-    cudaFree(b->d_solo_counters[k]); cudaFree(b->d_solo_list[k]);
+    cudaFree(b->d_solo_counters[k]); cudaFree(b->d_solo_list[k]); cudaFree(b->d_solo_seg[k]);
     if (b->branch[k]) cudaStreamDestroy(b->branch[k]);
   }
   for (auto ev : b->ev) if (ev) cudaEventDestroy(ev);
@@ -271,7 +272,15 @@ int msvgb_detail::batch_create(msvgb_ctx *ctx, const msvgb_om *const *oms, int n
   e = cudaMalloc(&b->d_vars, sizeof(ProfDev) * std::max(1, b->nvars));
   if (e == cudaSuccess) e = cudaMalloc(&b->d_items, sizeof(BatchItem) * std::max<int64_t>(1, b->nitems));
   if (e == cudaSuccess) e = cudaMalloc(&b->d_ticket, sizeof(unsigned long long));
+  size_t seg_need = 16;
+  std::vector<SegDev> large_segs;
+  for (auto &lp : large) {
+    large_segs.push_back(msvgb_detail::plan_segments(lp.second, db, ctx->num_sms, true));
+    seg_need = std::max(seg_need, msvgb_detail::seg_bytes(large_segs.back()));
+  }
   for (int k = 0; k < kSoloBranches && e == cudaSuccess && !large.empty(); ++k) {
+    e = cudaMalloc(&b->d_solo_seg[k], seg_need);
+    if (e != cudaSuccess) break;
     e = cudaMalloc(&b->d_solo_counters[k], 4 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_solo_list[k], sizeof(int64_t) * std::max<int64_t>(1, db->n));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->branch[k], cudaStreamNonBlocking);
@@ -304,7 +313,8 @@ int msvgb_detail::batch_create(msvgb_ctx *ctx, const msvgb_om *const *oms, int n
       const int k = (int) (jj % kSoloBranches);
       msvgb_detail::SearchScratch sc;
       sc.stream = b->branch[k]; sc.side = nullptr;
-      sc.ticket = b->d_solo_counters[k]; sc.aux = b->d_solo_counters[k] + 1; sc.list = b->d_solo_list[k];
+      sc.counters = b->d_solo_counters[k]; sc.list = b->d_solo_list[k];
+      sc.others = sc.cut = true; sc.segs = large_segs[j]; sc.seg = b->d_solo_seg[k];
       const int st = msvgb_detail::enqueue_search(sc, large[j].second, db, large_tables[j],
                                                   (uint8_t *) d_xj + (int64_t) large[j].first * db->n,
                                                   (uint8_t *) d_flags + (int64_t) large[j].first * db->n,

@@ -58,6 +58,73 @@ struct DbDev {
   int64_t         n;
 };
 
+// ---- segments of long targets ---------------------------------------------------
+// A target's rows are a serial chain, and the longest targets' chains set the
+// length of a search that is not much longer than they are. The SSV recurrence
+// is local: a diagonal crosses the model within M rows, so a run started M rows
+// early from empty cells has every cell right from its first own row on (its
+// earlier cells are only too low, which no maximum notices). The longest nl
+// sorted sequences of a pass are therefore cut into segments of T rows, scored
+// as work items of their own after warm >= M rows of run-in. Each leaves the
+// largest cell of every block of R of its rows in u[], and the segment that
+// finishes last decides the sequence.
+//
+// The full MSV of such a sequence reads u[] too: relative to the begin score
+// its cells follow the same recurrence (equal to the SSV cells while the begin
+// score has not changed, at most equal afterwards), so a block whose largest
+// cell cannot raise xJ above the base or above its record, and cannot
+// overflow, is skipped, and the recurrence resumes warm rows before the next
+// one that can.
+//
+// Items are ordered by segment index: sequences [0, base[k+1] - base[k]) have
+// a k-th segment (they are sorted longest first), item base[k] + slot.
+constexpr int kMaxSegs = 64;
+struct SegDev {
+  int64_t nl = 0;                // sequences cut into segments (the first of the pass)
+  int T = 0, warm = 0, S = 0;    // rows per segment, run-in rows, segments of the longest (0: none are cut)
+  int R = 0, NB = 0;             // rows per block (T is a multiple), blocks of the longest
+  uint32_t base[kMaxSegs + 1] = {};
+  uint8_t *u = nullptr;          // [nl][NB] largest cell of each block, at most 255
+  uint32_t *done = nullptr;      // [nl] finished segments (zeroed before the search)
+};
+
+__device__ __forceinline__ int seg_of(const SegDev &g, uint32_t item) {
+  int k = 0;
+  while (item >= g.base[k + 1]) ++k;
+  return k;
+}
+
+// A segment's blocks are all in u[]: the sequence's largest cell when it was
+// the last of its segments to finish, else -1. One thread (the one that wrote
+// the blocks).
+__device__ __forceinline__ int seg_finish(const SegDev &g, int64_t slot, int L) {
+  __threadfence();
+  if (atomicAdd(&g.done[slot], 1u) != (uint32_t) ((L + g.T - 1) / g.T - 1)) return -1;
+  __threadfence();
+  const int nb = (L + g.R - 1) / g.R;
+  const uint8_t *u = g.u + slot * g.NB;
+  int m = 0;
+  for (int b = 0; b < nb; ++b) m = max(m, (int) __ldcg(u + b));
+  return m;
+}
+
+// The first block from b on whose rows the full MSV has to run at the current
+// xJ and begin score xB (as clamped for the row): its cells may leave the
+// range the SSV cells are exact in, overflow, or raise xJ above both its
+// record and the base. Below the base xJ does not feed back: there the skipped
+// blocks' scores, xB + u, are taken into it directly. nb when none is left.
+__device__ __forceinline__ int seg_next_hot(const SegDev &g, int64_t slot, int nb, int b, int xB, int tec, int base,
+                                            int bias, int &xJ) {
+  const uint8_t *us = g.u + slot * g.NB;
+  for (; b < nb; ++b) {
+    const int u = __ldcg(us + b);
+    const int xE = xB + u;
+    if (u >= 127 - bias || xE + bias >= 255 || xE - tec > max(xJ, base) || (u == 0 && xJ < xE - tec)) break;
+    if (u > 0) xJ = max(xJ, xE - tec);
+  }
+  return b;
+}
+
 // ---- packed 16-bit integer helpers (native on sm_90+) ------------------------
 __device__ __forceinline__ uint32_t add_s16x2(uint32_t a, uint32_t b) {
   uint32_t d; asm("add.s16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d;
@@ -225,31 +292,39 @@ __device__ __forceinline__ int ssv_decide(int umax, int tjb, int tbm, int tec, i
   return -1;                                     // the J state could have been used
 }
 
-template <int C, bool F16>
-__device__ __forceinline__ int msv_one(const ProfDev &P, const uint32_t *__restrict__ stab,
-                                       const uint32_t *__restrict__ mtab,
-                                       const uint32_t *__restrict__ sq, int L, int lane,
-                                       int &xj_out, int &full_out, bool skip_ssv = false) {
-  const int tjb  = P.tjb[L];
-  const int tbm  = P.tbm, tec = P.tec, base = P.base, bias = P.bias;
-  full_out = 0;
-
-  // ---------- Phase A: SSV (ssvfilter.c:1364-1413) ----------
-  if (!skip_ssv && tjb + tbm + tec + bias < 127) {
-    uint32_t dp[C];
+// Phase A (ssvfilter.c:1364-1413): the largest SSV cell of rows [i0, end) run
+// from empty cells. i0 is a multiple of 4 RW, the rows of a step; sq holds the whole sequence. With
+// segs the rows are a segment of sorted slot slot, whose own rows start at r0,
+// and the largest cell of every block goes to segs->u (0 is returned).
+template <int C, bool F16, int RW = 1>
+__device__ __forceinline__ int ssv_range(const uint32_t *__restrict__ stab, const uint32_t *__restrict__ sq, int i0,
+                                         int end, int lane, const SegDev *segs = nullptr, int64_t slot = 0,
+                                         int r0 = 0) {
+  uint32_t dp[C];
 #pragma unroll
-    for (int w = 0; w < C; ++w) dp[w] = 0u;
-    uint32_t acc0 = 0u, acc1 = 0u;
-    const int src_lane = (lane + 31) & 31;
-    uint32_t nextw = (L > 0) ? __ldg(sq) : 0u;
-    for (int i0 = 0; i0 < L; i0 += 4) {
-      const uint32_t w4 = nextw;
-      if (i0 + 4 < L) nextw = __ldg(sq + (i0 >> 2) + 1);
-      // Rows past L hold PAD_CODE, whose costs keep every cell at the floor:
-      // processing them cannot raise the running maximum.
+  for (int w = 0; w < C; ++w) dp[w] = 0u;
+  uint32_t acc0 = 0u, acc1 = 0u;
+  const int src_lane = (lane + 31) & 31;
+  int stop = segs ? min(end, r0 + segs->R) : end;
+  auto fetch = [&](int i, uint32_t (&w)[2]) {
+    if constexpr (RW == 2) {
+      const uint2 v = __ldg(reinterpret_cast<const uint2 *>(sq) + (i >> 3));
+      w[0] = v.x; w[1] = v.y;
+    } else {
+      w[0] = __ldg(sq + (i >> 2));
+    }
+  };
+  uint32_t nextw[2] = {0u, 0u};
+  if (end > i0) fetch(i0, nextw);
+  for (;;) {
+    for (; i0 < stop; i0 += 4 * RW) {
+      const uint32_t w8[2] = {nextw[0], nextw[1]};
+      if (i0 + 4 * RW < end) fetch(i0 + 4 * RW, nextw);
+      // Rows past the sequence's end hold PAD_CODE, whose costs keep every cell
+      // at the floor: processing them cannot raise the running maximum.
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int x = (w4 >> (8 * j)) & 0xFF;
+      for (int j = 0; j < 4 * RW; ++j) {
+        const int x = (w8[j >> 2] >> (8 * (j & 3))) & 0xFF;
         if constexpr (F16) ssv_row_f16<C>(dp, acc0, acc1, stab, x, lane, src_lane);
         else               ssv_row_i8<C>(dp, acc0, acc1, stab + lane + x * ((C / 2) * 32), src_lane);
       }
@@ -267,23 +342,46 @@ __device__ __forceinline__ int msv_one(const ProfDev &P, const uint32_t *__restr
       umax = max(max(lo, hi), 0);
     }
     umax = (int) __reduce_max_sync(FULL, (unsigned) umax);
-
-    const int st = ssv_decide(umax, tjb, tbm, tec, base, bias, xj_out);
-    if (st >= 0) return st;
+    if (!segs) return umax;
+    if (lane == 0) segs->u[slot * segs->NB + (stop - 1) / segs->R] = (uint8_t) min(umax, 255);
+    if (stop >= end) return 0;
+    stop = min(end, stop + segs->R);
+    acc0 = acc1 = 0u;
   }
+}
 
-  // ---------- Phase B: full MSV (msvfilter.c:112-212) ----------
-  full_out = 1;
+// Phase B (msvfilter.c:112-212): the full MSV of one sequence. segs: the
+// sequence is cut into segments (sorted slot slot), and the largest cells of
+// its blocks say which rows need not be run.
+template <int C>
+__device__ __forceinline__ int msv_full(const ProfDev &P, const uint32_t *__restrict__ mtab,
+                                        const uint32_t *__restrict__ sq, int L, int tjb, int lane, int &xj_out,
+                                        const SegDev *segs = nullptr, int64_t slot = 0) {
+  const int tec = P.tec, base = P.base, bias = P.bias;
   uint32_t dp[C];
 #pragma unroll
   for (int w = 0; w < C; ++w) dp[w] = 0u;
-  const int tjbm = (tjb + tbm) & 0xFF;                 // (int8_t) tjb + (int8_t) tbm, splatted as bytes
+  const int tjbm = (tjb + P.tbm) & 0xFF;               // (int8_t) tjb + (int8_t) tbm, splatted as bytes
   int xJ = 0, xB = max(base - tjbm, 0);
   const uint32_t kneg = ((uint32_t) (bias - 255) & 0xFFFFu) * 0x00010001u;
   const uint32_t *tl = mtab + lane;
   const int src_lane = (lane + 31) & 31;
   uint32_t nextw = (L > 0) ? __ldg(sq) : 0u;
+  int next_blk = segs ? 0 : -1;                        // block to look at when its first row comes up
   for (int i0 = 0; i0 < L; i0 += 4) {
+    if (next_blk >= 0 && i0 == next_blk * segs->R) {
+      const int nb = (L + segs->R - 1) / segs->R;
+      const int k = seg_next_hot(*segs, slot, nb, next_blk, min(xB, 255 - bias), tec, base, bias, xJ);
+      if (k >= nb) break;
+      const int r = k * segs->R - segs->warm;
+      if (r > i0) {
+        i0 = r;
+        nextw = __ldg(sq + (i0 >> 2));
+#pragma unroll
+        for (int w = 0; w < C; ++w) dp[w] = 0u;
+      }
+      next_blk = k + 1;
+    }
     const uint32_t w4 = nextw;
     if (i0 + 4 < L) nextw = __ldg(sq + (i0 >> 2) + 1);
 #pragma unroll
@@ -301,6 +399,22 @@ __device__ __forceinline__ int msv_one(const ProfDev &P, const uint32_t *__restr
   }
   xj_out = xJ;
   return ST_OK;
+}
+
+template <int C, bool F16>
+__device__ __forceinline__ int msv_one(const ProfDev &P, const uint32_t *__restrict__ stab,
+                                       const uint32_t *__restrict__ mtab,
+                                       const uint32_t *__restrict__ sq, int L, int lane,
+                                       int &xj_out, int &full_out, bool skip_ssv = false) {
+  const int tjb = P.tjb[L];
+  full_out = 0;
+  if (!skip_ssv && tjb + P.tbm + P.tec + P.bias < 127) {
+    const int umax = ssv_range<C, F16>(stab, sq, 0, L, lane);
+    const int st = ssv_decide(umax, tjb, P.tbm, P.tec, P.base, P.bias, xj_out);
+    if (st >= 0) return st;
+  }
+  full_out = 1;
+  return msv_full<C>(P, mtab, sq, L, tjb, lane, xj_out);
 }
 
 // The dynamic shared memory opt-in of a kernel, once per device (the

@@ -180,27 +180,30 @@ struct GroupArgs {
   int64_t *undecided;              // sorted indices left for the full MSV pass
   unsigned long long *n_undecided;
   int64_t s_begin = 0;             // first sorted sequence of the pass (the rest of the database follows)
+  SegDev segs{};                   // segments of the longest sequences (s_begin 0)
   cudaStream_t stream;
 };
 
+constexpr int64_t kSegItem = (int64_t) 1 << 62;
 constexpr uint32_t kPadWord = 0x1D1D1D1Du;   // four PAD_CODE residues
 
 // The lockstep SSV loop of one warp. fetch() (called by lane 0 of a group)
 // returns the next sorted sequence index, or a negative value when there is
 // none; undecided(s) (lane 0 of a group) records a sequence that needs the full
 // MSV. Decided sequences (and empty ones) are written to out_xj / out_flags.
-// CI > 0: the mixed-width table (HybLayout<C, CI, G>, units of 2^-24).
-template <int C, int G, int CI = 0, class Fetch, class Undecided>
+// CI > 0: the mixed-width table (HybLayout<C, CI, G>, units of 2^-24). SEG:
+// fetch() returns a work item, the segments of segs first.
+template <int C, int G, int CI = 0, bool SEG = false, class Fetch, class Undecided>
 __device__ __forceinline__ void ssv_group_loop(const ProfDev &P, const uint32_t *__restrict__ tab, const DbDev &db,
                                                uint8_t *__restrict__ out_xj, uint8_t *__restrict__ out_flags,
-                                               Fetch fetch, Undecided undecided) {
+                                               Fetch fetch, Undecided undecided, const SegDev &segs = SegDev()) {
   const int lane = threadIdx.x & 31, glane = lane % G, gbase = lane - glane, gidx = lane / G;
   const int src_lane = gbase + (glane + G - 1) % G;
   const unsigned gmask = (G == 32) ? FULL : (((1u << G) - 1u) << gbase);
   const int tbm = P.tbm, tec = P.tec, base = P.base, bias = P.bias;
 
-  int64_t s = 0;
-  int L = 0, i = 0, tjb = 0;
+  int64_t s = 0;                                      // SEG: kSegItem | work item while the group scores a segment
+  int L = 0, i = 0;                                   // L: where the item's rows (SEG: the block's) end
   const uint32_t *sq = nullptr;
   uint32_t nextw = kPadWord;
   bool need = true, done = false;
@@ -218,9 +221,25 @@ __device__ __forceinline__ void ssv_group_loop(const ProfDev &P, const uint32_t 
         done = true;
       } else {
         s = (int64_t) t;
+        int k = -1;                                   // segment index
+        if constexpr (SEG) {
+          const long long nseg = segs.base[segs.S];
+          if (t < nseg) { k = seg_of(segs, (uint32_t) t); s = t - segs.base[k]; }
+          else s = t - nseg + segs.nl;
+        }
         L = db.len[s];
-        tjb = P.tjb[L];
-        if (L == 0) {                                 // skipped, as p7_Pipeline does
+        const int tjb = P.tjb[L];
+        if (SEG && k >= 0) {
+          sq = reinterpret_cast<const uint32_t *>(db.codes + db.start[s]);
+          i = max(0, k * segs.T - segs.warm);
+          L = min(L, k * segs.T + segs.R);
+          s = kSegItem | t;
+          nextw = __ldg(sq + (i >> 2));
+          need = false;
+#pragma unroll
+          for (int w = 0; w < C; ++w) dp[w] = 0u;
+          acc0 = acc1 = 0u;
+        } else if (L == 0) {                                 // skipped, as p7_Pipeline does
           if (glane == 0) { const int64_t oi = db.orig[s]; out_xj[oi] = 0; out_flags[oi] = 0x08; }
         } else if (tjb + tbm + tec + bias >= 127) {   // SSV disabled for this length: full MSV
           if (glane == 0) undecided(s);
@@ -238,7 +257,7 @@ __device__ __forceinline__ void ssv_group_loop(const ProfDev &P, const uint32_t 
     if (__all_sync(FULL, done)) break;
     const bool active = !need && !done;
     const uint32_t w4 = active ? nextw : kPadWord;
-    if (active && i + 4 < L) nextw = __ldg(sq + (i >> 2) + 1);
+    if (active && (SEG || i + 4 < L)) nextw = __ldg(sq + (i >> 2) + 1);   // SEG: may run into the buffer's padding
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       if constexpr (CI > 0) ssv_row_hyb<C, CI, G>(dp, acc0, acc1, tab, (w4 >> (8 * j)) & 0xFF, glane, gidx, src_lane);
@@ -258,9 +277,27 @@ __device__ __forceinline__ void ssv_group_loop(const ProfDev &P, const uint32_t 
 #pragma unroll
       for (int off = G / 2; off >= 1; off >>= 1) f = fmaxf(f, __shfl_xor_sync(FULL, f, off));
       if (fin) {
-        int xj = 0;
-        const int st = ssv_decide((int) f, tjb, tbm, tec, base, bias, xj);
-        if (glane == 0) {
+        int xj = 0, umax = (int) f;
+        need = true;
+        if (SEG && (s & kSegItem)) {                  // a segment's block
+          const uint32_t item = (uint32_t) (s & ~kSegItem);
+          const int k = seg_of(segs, item);
+          const int64_t slot = item - segs.base[k];
+          const int len = db.len[slot], end = min(len, (k + 1) * segs.T);
+          if (glane == 0) segs.u[slot * segs.NB + (L - 1) / segs.R] = (uint8_t) min(umax, 255);
+          if (L < end) {
+            L = min(end, L + segs.R);
+            acc0 = acc1 = 0u;
+            need = false;
+          } else if (glane == 0) {                    // the sequence's last segment to finish decides it
+            s = slot;
+            L = len;
+            umax = seg_finish(segs, slot, len);
+          }
+        }
+        if (need && glane == 0 && umax >= 0) {
+          const int tjb = P.tjb[L];
+          const int st = tjb + tbm + tec + bias < 127 ? ssv_decide(umax, tjb, tbm, tec, base, bias, xj) : -1;
           if (st < 0) {
             undecided(s);
           } else {
@@ -272,7 +309,6 @@ __device__ __forceinline__ void ssv_group_loop(const ProfDev &P, const uint32_t 
             out_flags[oi] = (uint8_t) flags;
           }
         }
-        need = true;
       }
     }
   }
@@ -294,11 +330,12 @@ __host__ __device__ constexpr int group_table_words() {
   else return GroupLayout<C, G>::WORDS;
 }
 
-template <int C, int G, int CI = 0>
+template <int C, int G, int CI, bool SEG>
 __global__ void __launch_bounds__(256)
 msv_ssv_group_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t *__restrict__ out_flags,
                      unsigned long long *__restrict__ ticket, int64_t *__restrict__ undecided,
-                     unsigned long long *__restrict__ n_undecided, int64_t s_begin) {
+                     unsigned long long *__restrict__ n_undecided, int64_t s_begin,
+                     const __grid_constant__ SegDev segs) {
   extern __shared__ __align__(16) uint32_t smem[];
   {
     const uint4 *gs = reinterpret_cast<const uint4 *>(P.stab);
@@ -306,14 +343,14 @@ msv_ssv_group_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t 
     for (int i = threadIdx.x; i < group_table_words<C, G, CI>() / 4; i += blockDim.x) ss[i] = __ldg(gs + i);
   }
   __syncthreads();
-  const unsigned long long n = (unsigned long long) db.n;
-  ssv_group_loop<C, G, CI>(
+  const unsigned long long n = SEG ? (unsigned long long) (db.n - segs.nl) + segs.base[segs.S] : (unsigned long long) db.n;
+  ssv_group_loop<C, G, CI, SEG>(
       P, smem, db, out_xj, out_flags,
       [&]() -> long long {
         const unsigned long long t = atomicAdd(ticket, 1ull) + (unsigned long long) s_begin;
         return t < n ? (long long) t : -1ll;
       },
-      [&](int64_t s) { undecided[atomicAdd(n_undecided, 1ull)] = s; });
+      [&](int64_t s) { undecided[atomicAdd(n_undecided, 1ull)] = s; }, segs);
 }
 
 // SSV pass of one CTA over the sorted sequences [s0, s0 + nseq) (a work item
@@ -333,25 +370,41 @@ __device__ __forceinline__ void ssv_group_chunk(const ProfDev &P, const uint32_t
       [&](int64_t s) { und[atomicAdd(n_und, 1u)] = (uint16_t) (s - s0); });
 }
 
+constexpr int hyb_words(int C, int G) {
+  if (G == 8) return C < 10 ? 0 : C < 18 ? 4 : 8;
+  if (G == 16) return C < 13 ? 0 : C < 24 ? 4 : 8;
+  if (G == 32) return C < 17 ? 0 : 8;     // the split 32-lane passes (M 1024-2047): always mixed width
+  return 0;
+}
+
 template <int C, int G, int CI = 0>
 cudaError_t launch_ssv_group(const GroupArgs &a, int num_sms) {
-  auto kern = msv_ssv_group_kernel<C, G, CI>;
+  // wide rows without segments keep their own kernel: the segments' state
+  // takes registers (64 -> 78 at 26 words per lane: 3 blocks per SM for 4);
+  // tables set by hand run without segments
+  constexpr bool cuts = CI == hyb_words(C, G), whole = !cuts || C >= 20;
+  if (!cuts && a.segs.S) return cudaErrorInvalidValue;
+  auto kern = msv_ssv_group_kernel<C, G, CI, !whole>;
+  if constexpr (cuts && whole) {
+    if (a.segs.S) kern = msv_ssv_group_kernel<C, G, CI, true>;
+  }
   static_assert(group_words(C, G, CI) == group_table_words<C, G, CI>(), "host and device table sizes agree");
   constexpr size_t smem = (size_t) group_table_words<C, G, CI>() * 4;
-  static std::atomic<unsigned long long> configured{0};
+  static std::atomic<unsigned long long> configured[2];
   {
-    cudaError_t e = ensure_smem_attr((const void *) kern, smem, configured);
+    cudaError_t e = ensure_smem_attr((const void *) kern, smem, configured[a.segs.S != 0]);
     if (e != cudaSuccess) return e;
   }
   int per_sm = 0;
   cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem);
   if (e != cudaSuccess) return e;
   int grid = std::max(1, per_sm) * num_sms;
-  const long long need = ((a.db.n - a.s_begin) * G + 255) / 256;   // 256 threads hold 256/G sequences
+  const long long items = a.db.n - a.s_begin - a.segs.nl + (a.segs.S ? a.segs.base[a.segs.S] : 0);
+  const long long need = (items * G + 255) / 256;                  // 256 threads hold 256/G sequences
   if (need < grid) grid = (int) std::max(1LL, need);
   (void) cudaGetLastError();
   kern<<<grid, 256, smem, a.stream>>>(a.P, a.db, a.out_xj, a.out_flags, a.ticket, a.undecided, a.n_undecided,
-                                      a.s_begin);
+                                      a.s_begin, a.segs);
   return cudaGetLastError();
 }
 
@@ -414,7 +467,7 @@ template <int C, int G>
 __global__ void __launch_bounds__(256)
 msv_list_group_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t *__restrict__ out_flags,
                       unsigned long long *__restrict__ ticket, const int64_t *__restrict__ list,
-                      const unsigned long long *__restrict__ list_count) {
+                      const unsigned long long *__restrict__ list_count, const __grid_constant__ SegDev segs) {
   extern __shared__ __align__(16) uint32_t smem[];
   {
     const uint4 *gs = reinterpret_cast<const uint4 *>(P.mtab);
@@ -433,6 +486,7 @@ msv_list_group_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t
   const uint32_t *sq = nullptr;
   uint32_t nextw = kPadWord;
   bool need = true, done = false, er = false;
+  int next_blk = -1;                                  // block to look at when its first row comes up
   uint32_t dp[C];
 #pragma unroll
   for (int w = 0; w < C; ++w) dp[w] = 0u;
@@ -454,6 +508,7 @@ msv_list_group_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t
         xJ = 0;
         xB = max(base - tjbm, 0);
         er = false;
+        next_blk = s < segs.nl ? 0 : -1;
         sq = reinterpret_cast<const uint32_t *>(db.codes + db.start[s]);
         nextw = __ldg(sq);
         i = 0;
@@ -464,6 +519,20 @@ msv_list_group_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t
     }
     if (__all_sync(FULL, done)) break;
     const bool active = !need && !done;
+    if (active && next_blk >= 0 && i == next_blk * segs.R) {   // rows no score depends on are skipped
+      const int nb = (L + segs.R - 1) / segs.R;
+      const int k = seg_next_hot(segs, s, nb, next_blk, min(xB, 255 - bias), tec, base, bias, xJ);
+      const int r = k * segs.R - segs.warm;
+      if (k >= nb) {
+        i = L;                                        // no rows left: the sequence ends with this step
+      } else if (r > i) {
+        i = r;
+        nextw = __ldg(sq + (i >> 2));
+#pragma unroll
+        for (int w = 0; w < C; ++w) dp[w] = 0u;
+      }
+      next_blk = k + 1;
+    }
     const uint32_t w4 = active ? nextw : kPadWord;
     if (active && i + 4 < L) nextw = __ldg(sq + (i >> 2) + 1);
 #pragma unroll
@@ -500,7 +569,7 @@ msv_list_group_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t
 template <int C, int G>
 cudaError_t launch_list_group(const ProfDev &P, const DbDev &db, uint8_t *out_xj, uint8_t *out_flags,
                               unsigned long long *ticket, const int64_t *list, const unsigned long long *list_count,
-                              int num_sms, cudaStream_t stream) {
+                              const SegDev &segs, int num_sms, cudaStream_t stream) {
   auto kern = msv_list_group_kernel<C, G>;
   constexpr size_t smem = (size_t) GroupLayout<C, G>::WORDS * 4;
   static std::atomic<unsigned long long> configured{0};
@@ -511,8 +580,14 @@ cudaError_t launch_list_group(const ProfDev &P, const DbDev &db, uint8_t *out_xj
   int per_sm = 0;
   cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem);
   if (e != cudaSuccess) return e;
+  // a block per SM holds a small search's list (about a 16th of the sequences
+  // at most, as a rule) and leaves the rest of the SM to searches on other
+  // streams; larger lists fill the SMs
+  constexpr int groups = 256 / G;
+  const long long want = (db.n / 16 + groups - 1) / groups;
+  const long long grid = std::max<long long>(num_sms, std::min<long long>((long long) std::max(1, per_sm) * num_sms, want));
   (void) cudaGetLastError();
-  kern<<<std::max(1, per_sm) * num_sms, 256, smem, stream>>>(P, db, out_xj, out_flags, ticket, list, list_count);
+  kern<<<(unsigned) grid, 256, smem, stream>>>(P, db, out_xj, out_flags, ticket, list, list_count, segs);
   return cudaGetLastError();
 }
 
@@ -521,4 +596,5 @@ cudaError_t launch_list_group(const ProfDev &P, const DbDev &db, uint8_t *out_xj
 #define MSVGB_INSTANTIATE_LIST(C, G)                                                                       \
   template cudaError_t msvgb::launch_list_group<C, G>(const msvgb::ProfDev &, const msvgb::DbDev &, uint8_t *, \
                                                       uint8_t *, unsigned long long *, const int64_t *,      \
-                                                      const unsigned long long *, int, cudaStream_t);
+                                                      const unsigned long long *, const msvgb::SegDev &, int, \
+                                                      cudaStream_t);

@@ -44,10 +44,9 @@ struct msvgb_ctx {
   // staged in pinned host memory and uploaded in one copy
   uint8_t *d_one = nullptr; size_t d_one_cap = 0;
   uint8_t *h_one = nullptr; size_t h_one_cap = 0;
-  uint8_t *d_out = nullptr;
   int *d_bad = nullptr;                                 // database packing: invalid-code flag
   int64_t *d_list = nullptr; size_t list_cap = 0;       // G-lane search: sequences left for the full MSV
-  unsigned long long *d_aux = nullptr;                  // [0] second ticket, [1] list count, [2] third ticket
+  uint8_t *d_seg = nullptr; size_t seg_cap = 0;         // segment maxima and counts of the long targets
   cudaStream_t side = nullptr;                          // long targets of the lane-group search
   cudaStream_t upload = nullptr;                        // chunk uploads of msvgb_search_host
   cudaStream_t dma = nullptr;                           // raw residue copies of database creation
@@ -217,7 +216,8 @@ std::vector<uint32_t> build_group_msv_table(const msvgb_om *om, int C, int G);
 // Launches the full-MSV pass of a list on lane groups (msv_list_group_kernel).
 cudaError_t dispatch_list_group(int C, int G, const msvgb::ProfDev &P, const msvgb::DbDev &db, uint8_t *out_xj,
                                 uint8_t *out_flags, unsigned long long *ticket, const int64_t *list,
-                                const unsigned long long *list_count, int sms, cudaStream_t stream);
+                                const unsigned long long *list_count, const msvgb::SegDev &segs, int sms,
+                                cudaStream_t stream);
 // Target-length bins of the lane choice: [0,150) [150,600) [600,2400) [2400,inf).
 constexpr int kNLBins = 4;
 int lbin_of(int L);
@@ -237,10 +237,16 @@ struct SearchScratch {
   cudaStream_t stream = nullptr;     // the search's stream
   cudaStream_t side = nullptr;       // long targets run here, concurrently (null: on stream, first)
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;   // needed with side
-  unsigned long long *ticket = nullptr;               // 1 counter
-  unsigned long long *aux = nullptr;                  // 3 counters
+  unsigned long long *counters = nullptr;             // 4 counters
   int64_t *list = nullptr;                            // room for every sequence of the database
+  bool others = false;                                // other searches share the GPU: throughput before latency
+  bool cut = false;                                   // long targets are cut as segs says (else they run at 32 lanes)
+  msvgb::SegDev segs{};                               // plan_segments
+  uint8_t *seg = nullptr;                             // seg_bytes(segs) bytes
 };
+// How a search of db by p cuts its long targets (pointers unset).
+msvgb::SegDev plan_segments(const msvgb_profile *p, const msvgb_db *db, int num_sms, bool others = false);
+size_t seg_bytes(const msvgb::SegDev &g);
 // Enqueues the single-profile search of db (per-length tables t) with the
 // lane-group pass when the profile has one (and the search is not small),
 // else the 32-lane kernel. The database must be in place on sc.stream.

@@ -15,12 +15,10 @@ struct LaunchArgs {
   cudaStream_t        stream;
   int                 grid;       // 0: fill the GPU
   int                 skip_empty; // 1: L == 0 is skipped as p7_Pipeline does; 0: scored like p7_MSVFilter
-  // List mode: score only the sorted sequences list[0 .. *list_count) with the
-  // full MSV recurrence (they are the ones the G-lane SSV pass left undecided).
-  const int64_t            *list = nullptr;
-  const unsigned long long *list_count = nullptr;
   // Range mode (range_end > 0): only the sorted sequences [0, range_end).
   int64_t                   range_end = 0;
+  // Segments of the longest sequences (not in range mode).
+  SegDev                    segs{};
 };
 
 constexpr int WARPS_PER_CTA = 8;
@@ -43,6 +41,14 @@ constexpr size_t smem_bytes() {   // SSV table + MSV table
 template <int C, bool F16>
 constexpr int cta_threads() { return 2 * smem_bytes<C, F16>() > 227 * 1024 ? MAX_WARPS_PER_CTA * 32 : WARPS_PER_CTA * 32; }
 
+// Words of four residues per step of the SSV loop. Narrow rows go eight a step,
+// so that the next rows' costs are loaded under a row's shuffle (M = 200, 20,000
+// targets: 217 us, 251 at four; M = 400, 40,000: 552 and 611; one call of the
+// drop-in at M = 200: 29 us and 34); from 9 words four rows keep as much in flight
+// (M = 700: 716 and 744, 900: 689 and 672).
+template <int C, bool F16>
+__host__ __device__ constexpr int row_words() { return F16 && C <= 8 ? 2 : 1; }
+
 // Persistent kernel: every CTA stages the profile's cost tables into shared
 // memory once, then its warps pull sequences (longest first) from a global
 // ticket until the database is exhausted.
@@ -50,8 +56,7 @@ template <int C, bool F16>
 __global__ void __launch_bounds__(cta_threads<C, F16>())
 msv_search_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t *__restrict__ out_flags,
                   unsigned long long *__restrict__ ticket, int skip_empty,
-                  const int64_t *__restrict__ list, const unsigned long long *__restrict__ list_count,
-                  int64_t range_end) {
+                  int64_t range_end, const __grid_constant__ SegDev segs) {
   extern __shared__ __align__(16) uint32_t smem[];
   constexpr int SW = F16 ? NRES * C * 32 : NRES * (C / 2) * 32;   // words of the SSV table
   constexpr int MW = NRES * ((C + 1) / 2) * 32;                    // words of the MSV table
@@ -69,13 +74,17 @@ msv_search_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t *__
   }
 
   const int lane = threadIdx.x & 31;
-  const unsigned long long nitems = list ? *list_count : (unsigned long long) (range_end > 0 ? range_end : db.n);
+  const unsigned long long nseg = segs.S ? segs.base[segs.S] : 0ull;
+  const unsigned long long nitems = (unsigned long long) (range_end > 0 ? range_end : db.n - segs.nl) + nseg;
   for (;;) {
     unsigned long long s = 0;
     if (lane == 0) s = atomicAdd(ticket, 1ull);
     s = __shfl_sync(FULL, s, 0);
     if (s >= nitems) break;
-    if (list) s = (unsigned long long) list[s];
+    const unsigned long long item = s;
+    int k = -1;                                       // segment index
+    if (item < nseg) { k = seg_of(segs, (uint32_t) item); s = item - segs.base[k]; }
+    else s = item - nseg + (unsigned long long) segs.nl;
     const int L = db.len[s];
     const int64_t oi = db.orig[s];
     if (L == 0 && skip_empty) {
@@ -83,8 +92,24 @@ msv_search_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t *__
       continue;
     }
     const uint32_t *sq = reinterpret_cast<const uint32_t *>(db.codes + db.start[s]);
-    int xj, full;
-    const int st = msv_one<C, F16>(P, stab, mtab, sq, L, lane, xj, full, list != nullptr);
+    const int tjb = P.tjb[L];
+    const bool ssv_off = tjb + P.tbm + P.tec + P.bias >= 127;   // SSV disabled for this length
+    int xj, full = 0, st = -1;
+    if (k >= 0 || !ssv_off) {
+      const int r0 = k >= 0 ? k * segs.T : 0, end = k >= 0 ? min(L, r0 + segs.T) : L;
+      int umax = ssv_range<C, F16, row_words<C, F16>()>(stab, sq, max(0, r0 - segs.warm), end, lane, k >= 0 ? &segs : nullptr,
+                                   (int64_t) s, r0);
+      if (k >= 0) {                                   // the sequence's last segment to finish decides it
+        if (lane == 0) umax = seg_finish(segs, (int64_t) s, L);
+        umax = __shfl_sync(FULL, umax, 0);
+        if (umax < 0) continue;
+      }
+      if (!ssv_off) st = ssv_decide(umax, tjb, P.tbm, P.tec, P.base, P.bias, xj);
+    }
+    if (st < 0) {
+      full = 1;
+      st = msv_full<C>(P, mtab, sq, L, tjb, lane, xj, k >= 0 ? &segs : nullptr, (int64_t) s);
+    }
     if (lane == 0) {
       int flags = full ? 0x04 : 0;
       if (st == ST_ERANGE) flags |= 0x01 | 0x02;                 // +inf always passes F1
@@ -111,14 +136,21 @@ cudaError_t launch_search(const LaunchArgs &a, int num_sms) {
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
+    // Where long targets are cut the chains set the time, and they run faster
+    // with fewer warps beside them (8 / 4 / 3 / 2 blocks per SM, us: M = 130, 40,000
+    // targets 369 / 370 / 381 / 431; M = 200, 20,000 247 / 239 / 241 / 243; M = 400, 5,000 261 /
+    // 260 / 248 / 232, 40,000 552 / 553 / 484 / 483; M = 550, 10,000 334 / 329 / 310 / 286,
+    // 60,000 872 / 876 / 834 / 844; M = 800, 10,000 393 / 392 / 398 / 344).
+    if (F16 && a.segs.S) per_sm = std::min(per_sm, C <= 3 ? 4 : C == 4 ? 3 : 2);
     grid = per_sm * num_sms;
     const int warps = threads / 32;
-    const long long need = ((a.range_end > 0 ? a.range_end : a.db.n) + warps - 1) / warps;
-    if (!a.list && need < grid) grid = (int) (need > 0 ? need : 1);
+    const long long items = a.range_end > 0 ? a.range_end : a.db.n - a.segs.nl + (a.segs.S ? a.segs.base[a.segs.S] : 0);
+    const long long need = (items + warps - 1) / warps;
+    if (need < grid) grid = (int) (need > 0 ? need : 1);
   }
   (void) cudaGetLastError();   // clear a stale error left by an unrelated call
   kern<<<grid, threads, smem, a.stream>>>(a.P, a.db, a.out_xj, a.out_flags, a.ticket, a.skip_empty,
-                                               a.list, a.list_count, a.range_end);
+                                               a.range_end, a.segs);
   return cudaGetLastError();
 }
 

@@ -368,7 +368,7 @@ static int submit_solo(msvgb_server *s, const msvgb_om *om, const msvgb_detail::
   s->next_solo ^= 1;
   msvgb_detail::SearchScratch sc;
   sc.stream = s->solo_stream[k];
-  sc.ticket = s->d_solo_counters[k]; sc.aux = s->d_solo_counters[k] + 1; sc.list = s->d_solo_list[k];
+  sc.counters = s->d_solo_counters[k]; sc.list = s->d_solo_list[k];
   int st = msvgb_detail::enqueue_search(sc, &p, s->db, &lt, base + s->off_xj, base + s->off_fl, s->ctx->num_sms);
   cudaFreeAsync(tabs, sc.stream);                      // after the search, in stream order
   if (st != MSVGB_eslOK) return st;
