@@ -144,11 +144,6 @@ template <int C, int G, int CI> cudaError_t launch_ssv_group(const GroupArgs &a,
 // Mixed-width instantiations (inst_hyb*.cu): (C, G, CI) triples.
 #include "msv_hyb_list.h"
 
-// Default 8-bit words per lane of the G-lane SSV pass at DP width C, from a
-// sweep on GB300 (1,000,000 sequences; M from 120 to 1008): at 8 lanes none
-// below 10 words (4 lost 2.5% at M = 120), 4 up to 17 words (+4 to +7%), 8
-// from 18 words (+7 to +10%; 12 and 16 were slower than 8 everywhere); at 16
-// lanes 4 up to 23 words (+3 to +9%), 8 from 24 (+8%).
 int msvgb_detail::hyb_default_words(int C, int G) { return msvgb::hyb_words(C, G); }
 
 bool msvgb_detail::hyb_compiled(int C, int G, int CI) {
@@ -167,10 +162,13 @@ cudaError_t msvgb_detail::dispatch_group(int C, int G, int CI, const GroupArgs &
   }
 #define G16(c) case c: return launch_ssv_group<c, 16, 0>(a, sms);
 #define G8(c)  case c: return launch_ssv_group<c, 8, 0>(a, sms);
+#define G4(c)  case c: return launch_ssv_group<c, 4, 0>(a, sms);
   if (G == 16) {
     switch (C) { G16(2) G16(3) G16(4) G16(5) G16(6) G16(7) G16(8) G16(9) G16(10) G16(11) G16(12) G16(13)
                  G16(14) G16(15) G16(16) G16(17) G16(18) G16(19) G16(20) G16(21) G16(22) G16(23) G16(24)
                  G16(25) G16(26) G16(27) G16(28) G16(29) G16(30) G16(31) G16(32) }
+  } else if (G == 4) {
+    switch (C) { G4(2) G4(3) G4(4) G4(5) G4(6) G4(7) G4(8) G4(9) }
   } else if (G == 8) {
     switch (C) { G8(2) G8(3) G8(4) G8(5) G8(6) G8(7) G8(8) G8(9) G8(10) G8(11) G8(12) G8(13)
                  G8(14) G8(15) G8(16) G8(17) G8(18) G8(19) G8(20) G8(21) G8(22) G8(23) G8(24)
@@ -179,6 +177,7 @@ cudaError_t msvgb_detail::dispatch_group(int C, int G, int CI, const GroupArgs &
   return cudaErrorInvalidValue;
 #undef G16
 #undef G8
+#undef G4
 }
 
 namespace msvgb {
@@ -200,11 +199,16 @@ cudaError_t msvgb_detail::dispatch_list_group(int C, int G, const ProfDev &P, co
   }
 #undef L32
 #define L16(c) case c: return launch_list_group<c, 16>(P, db, out_xj, out_flags, ticket, list, list_count, segs, sms, stream);
+#define L4(c)  case c: return launch_list_group<c, 4>(P, db, out_xj, out_flags, ticket, list, list_count, segs, sms, stream);
 #define L8(c)  case c: return launch_list_group<c, 8>(P, db, out_xj, out_flags, ticket, list, list_count, segs, sms, stream);
   if (G == 16) {
     switch (C) { L16(2) L16(3) L16(4) L16(5) L16(6) L16(7) L16(8) L16(9) L16(10) L16(11) L16(12) L16(13)
                  L16(14) L16(15) L16(16) L16(17) L16(18) L16(19) L16(20) L16(21) L16(22) L16(23) L16(24)
                  L16(25) L16(26) L16(27) L16(28) L16(29) L16(30) L16(31) L16(32) }
+  } else if (G == 4) {
+    switch (C) { L4(2) L4(3) L4(4) L4(5) L4(6) L4(7) L4(8) L4(9) L4(10) L4(11) L4(12) L4(13)
+                 L4(14) L4(15) L4(16) L4(17) L4(18) L4(19) L4(20) L4(21) L4(22) L4(23) L4(24)
+                 L4(25) L4(26) L4(27) L4(28) L4(29) L4(30) L4(31) L4(32) }
   } else if (G == 8) {
     switch (C) { L8(2) L8(3) L8(4) L8(5) L8(6) L8(7) L8(8) L8(9) L8(10) L8(11) L8(12) L8(13)
                  L8(14) L8(15) L8(16) L8(17) L8(18) L8(19) L8(20) L8(21) L8(22) L8(23) L8(24)
@@ -213,6 +217,7 @@ cudaError_t msvgb_detail::dispatch_list_group(int C, int G, const ProfDev &P, co
   return cudaErrorInvalidValue;
 #undef L16
 #undef L8
+#undef L4
 }
 
 // ------------------------------------------------------------------------------
@@ -368,7 +373,6 @@ static int width_for(const msvgb_om *om, int want_f16, int force_C, int *ret_C, 
 // DP words per lane and 8-bit words per lane of the G-lane tables (G = 16 or
 // 8, or 32 for the split passes of models of 1024-2047 nodes).
 static int group_width(int M, int G, int *ret_C, int *ret_CI) {
-  if (G != 16 && G != 8 && G != 32) return fail(MSVGB_eslEINVAL, "lanes per sequence must be 32, 16 or 8");
   const int C = M / (2 * G) + 1;                          // 2*C*G > M: the last node is padding
   if (C > 32) return fail(MSVGB_eslEINVAL, "model too long for this many lanes per sequence");
   if (C < 2) return fail(MSVGB_eslEINVAL, "model too short for this many lanes per sequence");
@@ -440,7 +444,7 @@ extern "C" int msvgb_profile_create(msvgb_ctx *ctx, const msvgb_om *om, msvgb_pr
     st = msvgb_profile_set_lanes(*ret, om, G);
     if (st != MSVGB_eslOK) { msvgb_profile_destroy(*ret); *ret = nullptr; }
   }
-  if (st == MSVGB_eslOK) (*ret)->lanes_auto = true;
+  if (st == MSVGB_eslOK) st = msvgb_detail::profile_auto_lanes(*ret, om);
   return st;
 }
 
@@ -477,8 +481,8 @@ static std::vector<uint32_t> group_table_from(int C, int G, Cost cost) {
     uint16_t b; memcpy(&b, &h, 2); return b;
   };
   const int Q4 = C / 4, R = C % 4;
-  const int pair = G < 16 ? 16 / G : 1, single = 32 / G;      // region copies (GroupCopies)
-  const size_t a_words = (size_t) NRES * Q4 * G * 4, b_words = (R >= 2) ? (size_t) NRES * pair * G * 2 : 0;
+  const int quad = G < 8 ? 8 / G : 1, pair = G < 16 ? 16 / G : 1, single = 32 / G;   // region copies (GroupCopies)
+  const size_t a_words = (size_t) NRES * Q4 * quad * G * 4, b_words = (R >= 2) ? (size_t) NRES * pair * G * 2 : 0;
   std::vector<uint32_t> st((size_t) group_words(C, G, 0));
   for (int x = 0; x < NRES; ++x)
     for (int g = 0; g < G; ++g)
@@ -486,7 +490,7 @@ static std::vector<uint32_t> group_table_from(int C, int G, Cost cost) {
         const int k0 = g * 2 * C + w + 1, k1 = g * 2 * C + C + w + 1;
         const uint32_t v = f16bits(cost(x, k0)) | (f16bits(cost(x, k1)) << 16);
         if (w < 4 * Q4) {
-          st[(((size_t) x * Q4 + w / 4) * G + g) * 4 + (w % 4)] = v;
+          for (int cp = 0; cp < quad; ++cp) st[((((size_t) x * Q4 + w / 4) * quad + cp) * G + g) * 4 + (w % 4)] = v;
         } else if (R >= 2 && w < 4 * Q4 + 2) {
           for (int cp = 0; cp < pair; ++cp) st[a_words + (((size_t) x * pair + cp) * G + g) * 2 + (w - 4 * Q4)] = v;
         } else {
@@ -515,9 +519,12 @@ std::vector<uint32_t> msvgb_detail::build_group_msv_table(const msvgb_om *om, in
   });
 }
 
+static int set_group_tables(msvgb_profile *p, const msvgb_om *om, int G);
+
 extern "C" int msvgb_profile_set_lanes(msvgb_profile *p, const msvgb_om *om, int G) {
   if (!p || !om) return fail(MSVGB_eslEINVAL, "NULL argument");
   if (om->M != p->M) return fail(MSVGB_eslEINVAL, "om does not match the profile");
+  if (G != 16 && G != 8 && G != 32) return fail(MSVGB_eslEINVAL, "lanes per sequence must be 32, 16 or 8");
   p->lanes_auto = false;                                  // set by the caller: applies at any size
   // 32 lanes: the fused kernel, and for models of 1024 to 2047 nodes also
   // the split passes (32-lane groups, mixed-width SSV table), which large
@@ -526,9 +533,22 @@ extern "C" int msvgb_profile_set_lanes(msvgb_profile *p, const msvgb_om *om, int
   if (G == 32 && !wide) {
     cudaFree(p->d_stab_g); cudaFree(p->d_mtab_g);
     p->d_stab_g = p->d_mtab_g = nullptr;
-    p->G = 32; p->CI = 0;
+    p->G = p->Gk = 32; p->CI = 0;
     return MSVGB_eslOK;
   }
+  const int st = set_group_tables(p, om, G);
+  if (st == MSVGB_eslOK) p->G = G;
+  return st;
+}
+
+int msvgb_detail::profile_auto_lanes(msvgb_profile *p, const msvgb_om *om) {
+  p->lanes_auto = true;
+  return p->d_stab_g && p->G == 8 && p->M < kNarrowMaxM ? set_group_tables(p, om, 4) : MSVGB_eslOK;
+}
+
+// The lane-group tables at G lanes per sequence.
+static int set_group_tables(msvgb_profile *p, const msvgb_om *om, int G) {
+  using namespace msvgb_detail;
   int C = 0, CI = 0;
   const int gs = group_width(p->M, G, &C, &CI);
   if (gs != MSVGB_eslOK) return gs;
@@ -545,7 +565,7 @@ extern "C" int msvgb_profile_set_lanes(msvgb_profile *p, const msvgb_om *om, int
   if (e != cudaSuccess) { cudaFree(d); cudaFree(dm); return fail(MSVGB_eslESYS, cudaGetErrorString(e)); }
   cudaFree(p->d_stab_g);
   cudaFree(p->d_mtab_g);
-  p->d_stab_g = d; p->d_mtab_g = dm; p->Cg = C; p->G = G; p->CI = CI;
+  p->d_stab_g = d; p->d_mtab_g = dm; p->Cg = C; p->Gk = G; p->CI = CI;
   return MSVGB_eslOK;
 }
 
@@ -573,7 +593,7 @@ int msvgb_detail::build_profile_tables(msvgb_ctx *ctx, const msvgb_om *om, Profi
 
 // Mixed-width lane-group table: the first C - CI words of every lane as f16
 // bits of s units of 2^-24 (sign-magnitude: s < 0 -> 0x8000 | -s), the last
-// CI words (a multiple of 4) as bytes t = s + 128 (layout HybLayout<C, CI, G>,
+// CI words (a multiple of 4) as bytes, t = s + 128 or signed s (layout HybLayout<C, CI, G>,
 // msv_group.cuh).
 std::vector<uint32_t> msvgb_detail::build_hyb_table(const msvgb_om *om, int C, int G, int CI) {
   const int M = om->M, Q = std::max(2, (M - 1) / 16 + 1), bias = om->bias_b;
@@ -582,10 +602,10 @@ std::vector<uint32_t> msvgb_detail::build_hyb_table(const msvgb_om *om, int C, i
     return std::min(127, std::max(-128, bias - rbv_at(om, Q, x, k)));
   };
   auto sm16 = [](int v) -> uint32_t { return v < 0 ? 0x8000u | (uint32_t) (-v) : (uint32_t) v; };
-  const int CF = C - CI, Q4 = CF / 4, R = CF % 4, NO = CI / 8, HALF = (CI % 8) / 4;
-  const int pair = G < 16 ? 16 / G : 1, single = 32 / G;      // region copies (GroupCopies)
-  const size_t a_words = (size_t) NRES * Q4 * G * 4, b_words = (R >= 2) ? (size_t) NRES * pair * G * 2 : 0;
-  const size_t c_words = (R & 1) ? (size_t) NRES * single * G : 0, d_words = (size_t) NRES * NO * G * 4;
+  const int CF = C - CI, CB = CF + hyb_biased(C, CI), Q4 = CF / 4, R = CF % 4, NO = CI / 8, HALF = (CI % 8) / 4;
+  const int quad = G < 8 ? 8 / G : 1, pair = G < 16 ? 16 / G : 1, single = 32 / G;   // region copies (GroupCopies)
+  const size_t a_words = (size_t) NRES * Q4 * quad * G * 4, b_words = (R >= 2) ? (size_t) NRES * pair * G * 2 : 0;
+  const size_t c_words = (R & 1) ? (size_t) NRES * single * G : 0, d_words = (size_t) NRES * NO * quad * G * 4;
   std::vector<uint32_t> st((size_t) group_words(C, G, CI));
   for (int x = 0; x < NRES; ++x)
     for (int g = 0; g < G; ++g) {
@@ -593,18 +613,19 @@ std::vector<uint32_t> msvgb_detail::build_hyb_table(const msvgb_om *om, int C, i
       for (int w = 0; w < CF; ++w) {
         const uint32_t v = sm16(s_of(x, k_of(w, 0))) | (sm16(s_of(x, k_of(w, 1))) << 16);
         if (w < 4 * Q4) {
-          st[(((size_t) x * Q4 + w / 4) * G + g) * 4 + (w % 4)] = v;
+          for (int cp = 0; cp < quad; ++cp) st[((((size_t) x * Q4 + w / 4) * quad + cp) * G + g) * 4 + (w % 4)] = v;
         } else if (R >= 2 && w < 4 * Q4 + 2) {
           for (int cp = 0; cp < pair; ++cp) st[a_words + (((size_t) x * pair + cp) * G + g) * 2 + (w - 4 * Q4)] = v;
         } else {
           for (int cp = 0; cp < single; ++cp) st[a_words + b_words + ((size_t) x * single + cp) * G + g] = v;
         }
       }
-      auto t = [&](int ww, int h) { return (uint32_t) (s_of(x, k_of(ww, h)) + 128); };
+      auto t = [&](int ww, int h) { return (uint32_t) (uint8_t) (s_of(x, k_of(ww, h)) + (ww < CB ? 128 : 0)); };
       auto tword = [&](int w) { return t(w, 0) | (t(w + 1, 0) << 8) | (t(w, 1) << 16) | (t(w + 1, 1) << 24); };
       for (int o = 0; o < NO; ++o)
         for (int k = 0; k < 4; ++k)
-          st[a_words + b_words + c_words + (((size_t) x * NO + o) * G + g) * 4 + k] = tword(CF + 8 * o + 2 * k);
+          for (int cp = 0; cp < quad; ++cp)
+            st[a_words + b_words + c_words + ((((size_t) x * NO + o) * quad + cp) * G + g) * 4 + k] = tword(CF + 8 * o + 2 * k);
       for (int k = 0; k < 2 * HALF; ++k)
         for (int cp = 0; cp < pair; ++cp)
           st[a_words + b_words + c_words + d_words + (((size_t) x * pair + cp) * G + g) * 2 + k] =
@@ -618,6 +639,10 @@ extern "C" int msvgb_profile_set_ssv_int8_words(msvgb_profile *p, const msvgb_om
   if (om->M != p->M) return fail(MSVGB_eslEINVAL, "om does not match the profile");
   if (p->G == 32 || !p->d_stab_g)
     return fail(MSVGB_eslEINVAL, "8-bit SSV words are set for 16 or 8 lanes per sequence (32 lanes: fixed)");
+  if (p->Gk != p->G) {                                    // 4 lanes: the words are those of the lane count asked for
+    const int st = set_group_tables(p, om, p->G);
+    if (st != MSVGB_eslOK) return st;
+  }
   if (words == p->CI) return MSVGB_eslOK;
   if (words != 0 && !hyb_compiled(p->Cg, p->G, words))
     return fail(MSVGB_eslEINVAL, "no mixed-width SSV kernel for this model length, lane count and word count");
@@ -633,7 +658,12 @@ extern "C" int msvgb_profile_set_ssv_int8_words(msvgb_profile *p, const msvgb_om
   return MSVGB_eslOK;
 }
 
-extern "C" int msvgb_profile_ssv_int8_words(const msvgb_profile *p) { return p ? p->CI : -1; }
+extern "C" int msvgb_profile_ssv_int8_words(const msvgb_profile *p) {
+  if (!p) return -1;
+  int C = 0, CI = p->CI;
+  if (p->Gk != p->G && group_width(p->M, p->G, &C, &CI) != MSVGB_eslOK) return -1;
+  return CI;
+}
 
 // ------------------------------------------------------------------------------
 // per-length tables: tjb_b(L) and the smallest xJ that passes F1 at length L
@@ -1087,7 +1117,7 @@ extern "C" int64_t msvgb_db_residues(const msvgb_db *db) { return db ? db->resid
 // Lanes or 8-bit words set by the caller keep their documented launches (long
 // targets at 32 lanes); other searches may cut their long targets.
 static bool may_cut(const msvgb_profile *p) {
-  return !p->d_stab_g || (p->lanes_auto && p->CI == msvgb_detail::hyb_default_words(p->Cg, p->G));
+  return !p->d_stab_g || (p->lanes_auto && p->CI == msvgb_detail::hyb_default_words(p->Cg, p->Gk));
 }
 
 extern "C" int msvgb_search_device(msvgb_ctx *c, const msvgb_profile *pc, const msvgb_db *db, double F1,
@@ -1149,7 +1179,7 @@ SegDev msvgb_detail::plan_segments(const msvgb_profile *p, const msvgb_db *db, i
   SegDev g;
   const int M = p->M;
   const bool fused = search_fused(p, db, others);
-  const double chains = (double) num_sms * (fused ? (p->C > 32 ? 16.0 : 32.0) : 24.0 * 32.0 / p->G);
+  const double chains = (double) num_sms * (fused ? (p->C > 32 ? 16.0 : 32.0) : 24.0 * 32.0 / p->Gk);
   const double avg = (double) db->residues / chains;
   if (db->Lmax < avg / 2) return SegDev();                // no chain sets the search's length
   const double T = std::max({avg, 2.0 * M, 768.0, (double) db->Lmax / kMaxSegs});
@@ -1213,7 +1243,7 @@ int msvgb_detail::enqueue_search(const SearchScratch &sc, const msvgb_profile *p
   // joined back into the search's): those too long for a lane group to finish
   // within the pass, beyond about a third of the rows each group scores on
   // average (SMs x 32 warps x 32/G groups), and never below kLongTarget.
-  const double groups = (double) num_sms * 32.0 * (32.0 / p->G);
+  const double groups = (double) num_sms * 32.0 * (32.0 / p->Gk);
   const int t_long = (int) std::min<double>(1e9, std::max<double>(kLongTarget, (double) db->residues / groups / 3.0));
   const int64_t n_long = sc.cut ? 0 : std::min(db->count_at_least(t_long), db->n);
   ProfDev P;
@@ -1236,12 +1266,12 @@ int msvgb_detail::enqueue_search(const SearchScratch &sc, const msvgb_profile *p
     if (sc.side) CUDA_TRY(cudaEventRecord(sc.ev_join, sc.side));
   }
   if (n_long < db->n) {
-    CUDA_TRY(dispatch_group(p->Cg, p->G, p->CI, g, num_sms));
+    CUDA_TRY(dispatch_group(p->Cg, p->Gk, p->CI, g, num_sms));
     count_launch();
   }
   ProfDev Pl = P;                                          // the full MSV on the same lane groups
   Pl.mtab = p->d_mtab_g;
-  CUDA_TRY(dispatch_list_group(p->Cg, p->G, Pl, dbv, d_xj, d_flags, ctr + 1, sc.list, ctr + 2, segs, num_sms,
+  CUDA_TRY(dispatch_list_group(p->Cg, p->Gk, Pl, dbv, d_xj, d_flags, ctr + 1, sc.list, ctr + 2, segs, num_sms,
                                sc.stream));
   count_launch();
   if (n_long > 0 && sc.side) CUDA_TRY(cudaStreamWaitEvent(sc.stream, sc.ev_join, 0));
@@ -1311,7 +1341,7 @@ static int search_chunked(msvgb_ctx *c, const msvgb_profile *p, msvgb_db *db, co
   int t_long = INT32_MAX;
   if (groups) {
     P.C = p->Cg; P.stab = p->d_stab_g; P.ssv_f16 = 1;
-    const double ngroups = (double) sms * 32.0 * (32.0 / p->G);
+    const double ngroups = (double) sms * 32.0 * (32.0 / p->Gk);
     t_long = (int) std::min<double>(1e9, std::max<double>(kLongTarget, (double) db->residues / ngroups / 3.0));
   }
   for (int k = 0; k < K; ++k) {
@@ -1337,7 +1367,7 @@ static int search_chunked(msvgb_ctx *c, const msvgb_profile *p, msvgb_db *db, co
       g.P = P; g.db = full; g.db.n = s1; g.out_xj = d_xj; g.out_flags = d_flags;
       g.ticket = tk; g.undecided = list; g.n_undecided = ctr + 4; g.stream = s; g.s_begin = s0 + n_long;
       CUDA_TRY(cudaMemsetAsync(tk, 0, sizeof(unsigned long long), s));
-      CUDA_TRY(dispatch_group(p->Cg, p->G, p->CI, g, sms));
+      CUDA_TRY(dispatch_group(p->Cg, p->Gk, p->CI, g, sms));
       count_launch();
     }
     gt.mark("chunk " + std::to_string(k) + " passed", s);
@@ -1348,7 +1378,7 @@ static int search_chunked(msvgb_ctx *c, const msvgb_profile *p, msvgb_db *db, co
   if (groups) {                                             // the full MSV of the undecided sequences
     ProfDev Pl = P;
     Pl.mtab = p->d_mtab_g;
-    CUDA_TRY(dispatch_list_group(p->Cg, p->G, Pl, full, d_xj, d_flags, ctr + 5, list, ctr + 4, SegDev(), sms, S[0]));
+    CUDA_TRY(dispatch_list_group(p->Cg, p->Gk, Pl, full, d_xj, d_flags, ctr + 5, list, ctr + 4, SegDev(), sms, S[0]));
     count_launch();
     gt.mark("list passed", S[0]);
   }

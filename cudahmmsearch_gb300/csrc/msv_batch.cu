@@ -183,7 +183,8 @@ int msvgb_detail::batch_create(msvgb_ctx *ctx, const msvgb_om *const *oms, int n
       if (st == MSVGB_eslOK && p->f16) st = msvgb_profile_set_lanes(p, oms[i], G);   // 32: split passes for M 1024-2047
       if (p) b->own.push_back(p);
       if (st != MSVGB_eslOK) { msvgb_batch_destroy(b); return st; }
-      p->lanes_auto = true;
+      if (st == MSVGB_eslOK) st = msvgb_detail::profile_auto_lanes(p, oms[i]);
+      if (st != MSVGB_eslOK) { msvgb_batch_destroy(b); return st; }
       large.emplace_back(i, p);
       continue;
     }

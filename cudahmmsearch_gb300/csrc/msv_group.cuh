@@ -16,14 +16,15 @@
 
 namespace msvgb {
 
-// Copies of the 8-byte and 4-byte table regions. A shared-memory access is
-// served in phases of 128 bytes (8 lanes for 16-byte loads, 16 for 8-byte,
-// 32 for 4-byte loads); with 8-byte loads at 8 lanes per group, or 4-byte
-// loads at 8 or 16, one phase holds several groups, each reading its own
-// residue's row, and two rows whose offsets meet on the same banks conflict.
+// Copies of the table regions. A shared-memory access is served in phases of
+// 128 bytes (8 lanes for 16-byte loads, 16 for 8-byte, 32 for 4-byte loads);
+// where one phase holds several groups (16-byte loads at 4 lanes per group,
+// 8-byte loads at 8 or fewer, 4-byte loads at 16 or fewer), each reading its
+// own residue's row, two rows whose offsets meet on the same banks conflict.
 // Those regions are therefore stored once per group of a phase, each copy on
 // its own banks: group j of the phase reads copy j.
 template <int G> struct GroupCopies {
+  static constexpr int QUAD = G < 8 ? 8 / G : 1;          // 16-byte loads: groups per 8 lanes
   static constexpr int PAIR = G < 16 ? 16 / G : 1;       // 8-byte loads: groups per 16 lanes
   static constexpr int SINGLE = 32 / G;                   // 4-byte loads: groups per warp
 };
@@ -31,7 +32,7 @@ template <int G> struct GroupCopies {
 template <int C, int G>
 struct GroupLayout {
   static constexpr int Q4 = C / 4, R = C % 4;
-  static constexpr int A_WORDS = NRES * Q4 * G * 4;                                    // quads [x][q][g][4]
+  static constexpr int A_WORDS = NRES * Q4 * GroupCopies<G>::QUAD * G * 4;             // quads [x][q][copy][g][4]
   static constexpr int B_WORDS = (R >= 2) ? NRES * GroupCopies<G>::PAIR * G * 2 : 0;   // pair  [x][copy][g][2]
   static constexpr int C_WORDS = (R & 1) ? NRES * GroupCopies<G>::SINGLE * G : 0;      // single [x][copy][g]
   static constexpr int WORDS = A_WORDS + B_WORDS + C_WORDS;
@@ -47,7 +48,7 @@ __device__ __forceinline__ void ssv_row_group(uint32_t (&dp)[C], uint32_t &acc0,
   uint32_t s[C];
 #pragma unroll
   for (int q = 0; q < Lay::Q4; ++q) {
-    const uint4 v = *reinterpret_cast<const uint4 *>(tab + ((x * Lay::Q4 + q) * G + glane) * 4);
+    const uint4 v = *reinterpret_cast<const uint4 *>(tab + (((x * Lay::Q4 + q) * Cp::QUAD + gidx % Cp::QUAD) * G + glane) * 4);
     s[4 * q] = v.x; s[4 * q + 1] = v.y; s[4 * q + 2] = v.z; s[4 * q + 3] = v.w;
   }
   if constexpr (Lay::R >= 2) {
@@ -73,38 +74,63 @@ __device__ __forceinline__ void ssv_row_group(uint32_t (&dp)[C], uint32_t &acc0,
 // lane keep their costs as bytes (1 byte per cell) and widen them in
 // registers, trading shared-memory bytes for instructions on the idle pipes.
 //
-// Units: cells and costs are integers times 2^-24, i.e. f16 subnormals (and
-// the smallest normals): an integer n with |n| < 2048 is exact, its bits are
-// sign-magnitude (n < 0: 0x8000 | -n). A byte t is widened to a cost with one
-// PRMT (t as the low byte of a zero high byte: t * 2^-24) and one f16 add of
-// -128 units, so the table stores t = s + 128. Cell updates stay one
-// fma.relu per word as in the f16 row, and they are exact for the same
-// reason (integers below 2048 units; the relu clamps at 0). Non-negative f16
-// bits order like signed 16-bit integers, so the running maximum is taken on
-// the bits with integer instructions (ALU pipe) instead of f16 maxima (FMA
-// pipe).
+// Units: cells and f16 costs are integers times 2^-24, i.e. f16 subnormals
+// (and the smallest normals): an integer n with |n| < 2048 is exact, and the
+// bits of a cell (n >= 0) are the 16-bit integer n itself (a cost n < 0 is
+// 0x8000 | -n). So a cell is an f16 and an integer at once, and each word
+// takes whichever update suits the pipes: f16 words one fma.relu (FMA pipe);
+// 8-bit words either one PRMT that sign-extends the byte and one integer
+// add-and-maximum max(u + s, 0) (both on the ALU pipe), or, where the ALU pipe
+// with the running maximum on it is the fuller one, one PRMT to the f16 t =
+// s + 128, one f16 add of -128 and the fma.relu (hyb_biased of the words; their
+// bytes hold t). All are exact for the same reason. Bits order like signed
+// 16-bit integers, so the running maximum is taken on the bits too.
 //
 // Layout for residue x (CF = C - CI f16 words, CI a multiple of 4): the f16
 // regions of GroupLayout<CF, G> (quads, pair, single), then 16-byte octets
-// [x][o][g][4 words], then, when CI % 8 == 4, one 8-byte half octet
+// [x][o][copy][g][4 words], then, when CI % 8 == 4, one 8-byte half octet
 // [x][copy][g][2 words] (copies as GroupCopies): word k of octet o of lane g holds the bytes
-// [t(w, h0), t(w+1, h0), t(w, h1), t(w+1, h1)] of DP words w = CF + 8o + 2k
+// [s(w, h0), s(w+1, h0), s(w, h1), s(w+1, h1)] of DP words w = CF + 8o + 2k
 // and w + 1 (the half octet: w = CF + 8 * NO + 2k).
+__device__ __forceinline__ uint32_t add_f16x2(uint32_t a, uint32_t b) {
+  uint32_t d; asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d;
+}
+// Default 8-bit words per lane of the G-lane SSV pass at DP width C, and how
+// many of them take the FMA pipe, from a sweep on GB300 (TCUPS with 0 / 4 / 8 /
+// 12 words; 800,000 sequences at 8 lanes, 400,000 at 16, 250,000 at 32; a: 4 of
+// the words on the FMA pipe): C = 10: 13.4 / 14.3a; 12: 14.0 / 15.6 / 14.1a;
+// 16: 15.2 / 16.7 / 16.7a; 18: 15.6 / 16.9 / 17.3a; 22: 15.7 / 17.2 / 18.0a;
+// 24: 16.2 / 17.4 / 18.8; 28: 16.0 / - / 18.5 / 19.0a; 32: 16.9 / - / 18.8 / 19.5a;
+// 16 lanes: C = 20: 16.6 / 18.1 / 19.1a; 24: 16.9 / 16.9 / 19.6; 32: 17.5 / 17.5 /
+// 19.6 / 20.4a; 32 lanes: C = 17: - / 18.4 / 18.6a; 24: - / 18.6 / 20.1; 32: - /
+// 19.1 / 20.3 / 20.9a. With every 8-bit word on the FMA pipe C = 26 took 16.3 ms
+// for 2,000,000 sequences, 15.8 with none.
+__host__ __device__ constexpr int hyb_words(int C, int G) {
+  if (G == 32) return C < 17 ? 0 : 8;
+  if (C < (G == 16 ? 13 : 10)) return 0;
+  return C < 18 ? 4 : C < 28 ? 8 : 12;
+}
+__host__ __device__ constexpr int hyb_biased(int C, int CI) { return CI == 4 ? (C < 12 ? 4 : 0) : CI == 8 && C >= 24 ? 0 : 4; }
+
 template <int C, int CI, int G>
 struct HybLayout {
   static_assert(CI % 4 == 0 && CI >= 4 && CI <= C, "8-bit words come in fours");
-  static constexpr int CF = C - CI;
+  static constexpr int CF = C - CI, CB = CF + hyb_biased(C, CI);   // words below CB run on the FMA pipe
   static constexpr int Q4 = CF / 4, R = CF % 4, NO = CI / 8, HALF = (CI % 8) / 4;
-  static constexpr int A_WORDS = NRES * Q4 * G * 4;
+  static constexpr int A_WORDS = NRES * Q4 * GroupCopies<G>::QUAD * G * 4;
   static constexpr int B_WORDS = (R >= 2) ? NRES * GroupCopies<G>::PAIR * G * 2 : 0;
   static constexpr int C_WORDS = (R & 1) ? NRES * GroupCopies<G>::SINGLE * G : 0;
-  static constexpr int D_WORDS = NRES * NO * G * 4;
+  static constexpr int D_WORDS = NRES * NO * GroupCopies<G>::QUAD * G * 4;
   static constexpr int E_WORDS = NRES * HALF * GroupCopies<G>::PAIR * G * 2;   // [x][copy][g][2]
   static constexpr int WORDS = A_WORDS + B_WORDS + C_WORDS + D_WORDS + E_WORDS;
 };
 
-__device__ __forceinline__ uint32_t add_f16x2(uint32_t a, uint32_t b) {
-  uint32_t d; asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d;
+// The costs of two 8-bit words from a table word's bytes: as f16 (t - 128
+// units), or as sign-extended integers.
+__device__ __forceinline__ void hyb_widen(uint32_t t, bool f16, uint32_t &a, uint32_t &b) {
+  constexpr uint32_t m128 = 0x80808080u;        // f16x2 (-128, -128) units of 2^-24
+  a = f16 ? add_f16x2(prmt(t, 0u, 0x4240u), m128) : prmt(t, 0u, 0xA280u);   // bytes 0, 2
+  b = f16 ? add_f16x2(prmt(t, 0u, 0x4341u), m128) : prmt(t, 0u, 0xB391u);   // bytes 1, 3
 }
 
 template <int C, int CI, int G>
@@ -115,11 +141,10 @@ __device__ __forceinline__ void ssv_row_hyb(uint32_t (&dp)[C], uint32_t &acc0, u
   using Cp = GroupCopies<G>;
   constexpr int CF = Lay::CF;
   constexpr uint32_t one2 = 0x3C003C00u;        // f16x2 (1.0, 1.0)
-  constexpr uint32_t m128 = 0x80808080u;        // f16x2 (-128, -128) units of 2^-24
   uint32_t s[C];
 #pragma unroll
   for (int q = 0; q < Lay::Q4; ++q) {
-    const uint4 v = *reinterpret_cast<const uint4 *>(tab + ((x * Lay::Q4 + q) * G + glane) * 4);
+    const uint4 v = *reinterpret_cast<const uint4 *>(tab + (((x * Lay::Q4 + q) * Cp::QUAD + gidx % Cp::QUAD) * G + glane) * 4);
     s[4 * q] = v.x; s[4 * q + 1] = v.y; s[4 * q + 2] = v.z; s[4 * q + 3] = v.w;
   }
   if constexpr (Lay::R >= 2) {
@@ -131,12 +156,11 @@ __device__ __forceinline__ void ssv_row_hyb(uint32_t (&dp)[C], uint32_t &acc0, u
   const uint32_t *td = tab + Lay::A_WORDS + Lay::B_WORDS + Lay::C_WORDS;
 #pragma unroll
   for (int o = 0; o < Lay::NO; ++o) {
-    const uint4 v = *reinterpret_cast<const uint4 *>(td + ((x * Lay::NO + o) * G + glane) * 4);
+    const uint4 v = *reinterpret_cast<const uint4 *>(td + (((x * Lay::NO + o) * Cp::QUAD + gidx % Cp::QUAD) * G + glane) * 4);
     const uint32_t tw[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      s[CF + 8 * o + 2 * k]     = add_f16x2(prmt(tw[k], 0u, 0x4240u), m128);   // bytes 0, 2
-      s[CF + 8 * o + 2 * k + 1] = add_f16x2(prmt(tw[k], 0u, 0x4341u), m128);   // bytes 1, 3
+      hyb_widen(tw[k], CF + 8 * o + 2 * k < Lay::CB, s[CF + 8 * o + 2 * k], s[CF + 8 * o + 2 * k + 1]);
     }
   }
   if constexpr (Lay::HALF) {
@@ -145,13 +169,14 @@ __device__ __forceinline__ void ssv_row_hyb(uint32_t (&dp)[C], uint32_t &acc0, u
     const uint32_t tw[2] = {v.x, v.y};
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      s[CF + 8 * Lay::NO + 2 * k]     = add_f16x2(prmt(tw[k], 0u, 0x4240u), m128);
-      s[CF + 8 * Lay::NO + 2 * k + 1] = add_f16x2(prmt(tw[k], 0u, 0x4341u), m128);
+      hyb_widen(tw[k], CF + 8 * Lay::NO + 2 * k < Lay::CB, s[CF + 8 * Lay::NO + 2 * k], s[CF + 8 * Lay::NO + 2 * k + 1]);
     }
   }
   const uint32_t pred0 = pred_word0(dp[C - 1], src_lane);
 #pragma unroll
-  for (int w = C - 1; w >= 0; --w) dp[w] = fma_relu_f16x2(w ? dp[w - 1] : pred0, one2, s[w]);
+  for (int w = C - 1; w >= 0; --w)
+    dp[w] = w < Lay::CB ? fma_relu_f16x2(w ? dp[w - 1] : pred0, one2, s[w])
+                   : __viaddmax_s16x2(w ? dp[w - 1] : pred0, s[w], 0u);
   // running maximum on the bits (signed: a -0 from the relu is the smallest):
   // one three-input maximum per two words takes fewer issue slots than two
   // maxima, and issue, not the integer pipe, is what this row runs short of
@@ -204,8 +229,8 @@ __device__ __forceinline__ void ssv_group_loop(const ProfDev &P, const uint32_t 
 
   int64_t s = 0;                                      // SEG: kSegItem | work item while the group scores a segment
   int L = 0, i = 0;                                   // L: where the item's rows (SEG: the block's) end
-  const uint32_t *sq = nullptr;
-  uint32_t nextw = kPadWord;
+  const uint2 *sq = nullptr;
+  uint2 nextw = make_uint2(kPadWord, kPadWord);
   bool need = true, done = false;
   uint32_t dp[C];
   uint32_t acc0 = 0u, acc1 = 0u;
@@ -230,11 +255,11 @@ __device__ __forceinline__ void ssv_group_loop(const ProfDev &P, const uint32_t 
         L = db.len[s];
         const int tjb = P.tjb[L];
         if (SEG && k >= 0) {
-          sq = reinterpret_cast<const uint32_t *>(db.codes + db.start[s]);
+          sq = reinterpret_cast<const uint2 *>(db.codes + db.start[s]);
           i = max(0, k * segs.T - segs.warm);
           L = min(L, k * segs.T + segs.R);
           s = kSegItem | t;
-          nextw = __ldg(sq + (i >> 2));
+          nextw = __ldg(sq + (i >> 3));
           need = false;
 #pragma unroll
           for (int w = 0; w < C; ++w) dp[w] = 0u;
@@ -244,7 +269,7 @@ __device__ __forceinline__ void ssv_group_loop(const ProfDev &P, const uint32_t 
         } else if (tjb + tbm + tec + bias >= 127) {   // SSV disabled for this length: full MSV
           if (glane == 0) undecided(s);
         } else {
-          sq = reinterpret_cast<const uint32_t *>(db.codes + db.start[s]);
+          sq = reinterpret_cast<const uint2 *>(db.codes + db.start[s]);
           nextw = __ldg(sq);
           i = 0;
           need = false;
@@ -256,14 +281,16 @@ __device__ __forceinline__ void ssv_group_loop(const ProfDev &P, const uint32_t 
     }
     if (__all_sync(FULL, done)) break;
     const bool active = !need && !done;
-    const uint32_t w4 = active ? nextw : kPadWord;
-    if (active && (SEG || i + 4 < L)) nextw = __ldg(sq + (i >> 2) + 1);   // SEG: may run into the buffer's padding
+    // eight rows a step (sequences are padded to 16)
+    const uint32_t w8[2] = {active ? nextw.x : kPadWord, active ? nextw.y : kPadWord};
+    if (active && (SEG || i + 8 < L)) nextw = __ldg(sq + (i >> 3) + 1);   // SEG: may run into the buffer's padding
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if constexpr (CI > 0) ssv_row_hyb<C, CI, G>(dp, acc0, acc1, tab, (w4 >> (8 * j)) & 0xFF, glane, gidx, src_lane);
-      else                  ssv_row_group<C, G>(dp, acc0, acc1, tab, (w4 >> (8 * j)) & 0xFF, glane, gidx, src_lane);
+    for (int j = 0; j < 8; ++j) {
+      const int x = (w8[j >> 2] >> (8 * (j & 3))) & 0xFF;
+      if constexpr (CI > 0) ssv_row_hyb<C, CI, G>(dp, acc0, acc1, tab, x, glane, gidx, src_lane);
+      else                  ssv_row_group<C, G>(dp, acc0, acc1, tab, x, glane, gidx, src_lane);
     }
-    i += 4;
+    i += 8;
     const bool fin = active && i >= L;
     if (__any_sync(FULL, fin)) {                      // group maxima (all lanes take part)
       float f;
@@ -319,8 +346,9 @@ __device__ __forceinline__ void ssv_group_loop(const ProfDev &P, const uint32_t 
 // Table words of a lane-group SSV table at run-time (Cg, G, CI): the layouts
 // above (GroupLayout, or HybLayout when CI > 0) with their region copies.
 __host__ __device__ constexpr int group_words(int Cg, int G, int CI) {
-  return NRES * G * ((Cg - CI) / 4 * 4 + ((Cg - CI) % 4 >= 2 ? 2 * (G < 16 ? 16 / G : 1) : 0) +
-                     (((Cg - CI) % 4) & 1 ? 32 / G : 0) + CI / 8 * 4 + ((CI % 8) / 4) * 2 * (G < 16 ? 16 / G : 1));
+  const int quad = G < 8 ? 8 / G : 1, pair = G < 16 ? 16 / G : 1;    // GroupCopies
+  return NRES * G * ((Cg - CI) / 4 * 4 * quad + ((Cg - CI) % 4 >= 2 ? 2 * pair : 0) +
+                     (((Cg - CI) % 4) & 1 ? 32 / G : 0) + CI / 8 * 4 * quad + ((CI % 8) / 4) * 2 * pair);
 }
 
 // Table words of the lane-group SSV pass: f16 (CI = 0) or mixed width.
@@ -368,13 +396,6 @@ __device__ __forceinline__ void ssv_group_chunk(const ProfDev &P, const uint32_t
         return k < (unsigned) nseq ? (long long) (s0 + k) : -1ll;
       },
       [&](int64_t s) { und[atomicAdd(n_und, 1u)] = (uint16_t) (s - s0); });
-}
-
-constexpr int hyb_words(int C, int G) {
-  if (G == 8) return C < 10 ? 0 : C < 18 ? 4 : 8;
-  if (G == 16) return C < 13 ? 0 : C < 24 ? 4 : 8;
-  if (G == 32) return C < 17 ? 0 : 8;     // the split 32-lane passes (M 1024-2047): always mixed width
-  return 0;
 }
 
 template <int C, int G, int CI = 0>
@@ -439,7 +460,7 @@ __device__ __forceinline__ uint32_t msv_row_group(uint32_t (&dp)[C], uint32_t xB
   uint32_t s[C];
 #pragma unroll
   for (int q = 0; q < Lay::Q4; ++q) {
-    const uint4 v = *reinterpret_cast<const uint4 *>(tab + ((x * Lay::Q4 + q) * G + glane) * 4);
+    const uint4 v = *reinterpret_cast<const uint4 *>(tab + (((x * Lay::Q4 + q) * Cp::QUAD + gidx % Cp::QUAD) * G + glane) * 4);
     s[4 * q] = v.x; s[4 * q + 1] = v.y; s[4 * q + 2] = v.z; s[4 * q + 3] = v.w;
   }
   if constexpr (Lay::R >= 2) {

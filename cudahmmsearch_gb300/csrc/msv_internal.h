@@ -79,10 +79,11 @@ struct msvgb_profile {
   uint32_t *d_stab = nullptr, *d_mtab = nullptr;
   int G = 32;                         // lanes per sequence in the SSV pass (32: fused kernel)
   bool lanes_auto = false;            // G chosen by msvgb_profile_create (small searches then use 32)
-  int Cg = 0;                         // DP words per lane of the G-lane table
+  int Gk = 32;                        // lanes of the group tables: G, or 4 (kNarrowMaxM)
+  int Cg = 0;                         // DP words per lane of the group tables
   int CI = 0;                         // of those, words whose costs are bytes (mixed-width table); 0: all f16
-  uint32_t *d_stab_g = nullptr;       // SSV table in the G-lane layout (GroupLayout, or HybLayout when CI > 0)
-  uint32_t *d_mtab_g = nullptr;       // MSV table in the G-lane layout (GroupLayout, unclamped costs)
+  uint32_t *d_stab_g = nullptr;       // SSV table in the Gk-lane layout (GroupLayout, or HybLayout when CI > 0)
+  uint32_t *d_mtab_g = nullptr;       // MSV table in the Gk-lane layout (GroupLayout, unclamped costs)
   std::vector<LenTables *> tables;    // one per F1 value used
   std::mutex tables_mu;
 };
@@ -139,6 +140,11 @@ constexpr int kLongTarget = 2400;
 // +2% at 1984).
 constexpr int kWideSplitMinM = 1024;
 
+// Profiles of fewer nodes whose own lane choice is 8 run their large searches
+// on 4 lanes per sequence: at 8 a lane holds at most 16 words of the row, too
+// few to carry the row's fixed instructions.
+constexpr int kNarrowMaxM = 256;
+
 namespace msvgb_detail {
 // Device-side timeline of one call (MSVGB_GPU_TRACE; unlike MSVGB_TRACE it
 // adds no synchronization): timed events recorded on the streams the work
@@ -186,6 +192,9 @@ cudaError_t dispatch(int C, bool f16, const msvgb::LaunchArgs &a, int sms);
 // is not monotone in xJ.
 // hint: the answer at a nearby length (walked from instead of a binary search), or -1.
 int xjmin_for(const msvgb_profile *p, int L, double F1, int hint = -1);
+// Marks a profile's lanes as its own choice (msvgb_profile_create): its large
+// searches may then run on 4 lanes per sequence.
+int profile_auto_lanes(msvgb_profile *p, const msvgb_om *om);
 // Device tables of a profile; force_C > 0 imposes the DP width.
 int profile_build_width(msvgb_ctx *ctx, const msvgb_om *om, int want_f16, int force_C, msvgb_profile **ret);
 // Host images of the device cost tables of a profile at DP width C.

@@ -74,7 +74,7 @@ __device__ __forceinline__ void run_seq_any(int C, const ProfDev &P, const uint3
 // use at lane-group width Cg (0: f16 table): the single-query default
 // (hyb_default_words) at the group widths these kernels compile (kMultiC).
 __host__ __device__ constexpr int multi_hyb_words(int Cg, int G) {
-  return G == 8 ? (Cg < 10 ? 0 : Cg < 18 ? 4 : 8) : G == 16 ? (Cg < 13 ? 0 : Cg < 24 ? 4 : 8) : 0;
+  return G < 32 ? hyb_words(Cg, G) : 0;
 }
 
 // The lane-group SSV pass of one chunk at (G, Cg), with the f16 or the

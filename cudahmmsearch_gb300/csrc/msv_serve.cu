@@ -356,7 +356,7 @@ static int submit_solo(msvgb_server *s, const msvgb_om *om, const msvgb_detail::
   p.scale = om->scale_b; p.mmu = om->mmu; p.mlambda = om->mlambda;
   p.d_stab = (uint32_t *) (tabs + off[0]); p.d_mtab = (uint32_t *) (tabs + off[1]);
   if (!pt.stg.empty()) {
-    p.G = pt.G; p.Cg = pt.Cg; p.CI = pt.CI;
+    p.G = p.Gk = pt.G; p.Cg = pt.Cg; p.CI = pt.CI;
     p.d_stab_g = (uint32_t *) (tabs + off[2]); p.d_mtab_g = (uint32_t *) (tabs + off[3]);
   }
   p.lanes_auto = true;

@@ -90,8 +90,8 @@ uint64_t    msvgb_kernel_launches(void);
  * The profile is uploaded once per context and cached (up to 64 profiles,
  * least recently used out), found by the caller's rbv pointer and M or by a
  * content hash and confirmed byte for byte before use. Each call then makes
- * one host-to-device copy (from pinned staging), one launch and one 2-byte
- * copy back, and waits for them. Thread-safe (serialised per context). */
+ * one host-to-device copy (from pinned staging) and one launch, which writes
+ * its two result bytes to pinned memory, and waits for them. Thread-safe (serialised per context). */
 int msvgb_MSVFilter(msvgb_ctx *ctx, const uint8_t *dsq, int L, const msvgb_om *om,
                     msvgb_omx *ox, float *ret_sc);
 
@@ -112,17 +112,20 @@ int msvgb_profile_create_ex(msvgb_ctx *ctx, const msvgb_om *om, int ssv_variant,
 int msvgb_profile_variant(const msvgb_profile *prof);
 /* Lanes per sequence of the SSV pass: 32 (one warp per sequence, SSV
  * and full MSV in one kernel; for models of 1024 to 2047 nodes, searches of
- * at least ~40e9 cells -- or any search, when lanes are set here -- run the
+ * at least 36M residues -- or any search, when lanes are set here -- run the
  * SSV pass and the full MSV as two launches on 32-lane groups instead, with
  * the mixed-width table), or 16 / 8 (2 / 4 sequences per warp in
  * lockstep, for small models: each lane then holds more DP words per row);
  * with 16 or 8 the sequences SSV leaves undecided are finished by the full
- * MSV in a second launch on the same lane groups, and targets of 2400 residues or more run at 32
- * lanes in a concurrent launch (one long target must not set the length of
- * the search). om must be the profile's own MSV fields. Needs M < 64 * G and,
- * for G < 32, M >= 2 * G. Lanes chosen by msvgb_profile_create apply to
- * searches of at least ~40e9 cells (M x residues); smaller ones run at 32
- * lanes, where the shorter per-sequence latency wins; lanes set here always
+ * MSV in a second launch on the same lane groups. One long target must not
+ * set the length of the search: where lanes or 8-bit words are set by the
+ * caller, targets of 2400 residues or more run at 32 lanes in a concurrent
+ * launch; otherwise long targets are cut into segments that are scored
+ * independently. om must be the profile's own MSV fields. Needs M < 64 * G
+ * and, for G < 32, M >= 2 * G. Lanes chosen by msvgb_profile_create apply to
+ * searches of at least 24M residues (36M from 512 nodes up); smaller ones run
+ * at 32 lanes, where the shorter per-sequence latency wins; where the choice
+ * is 8 and M < 256 those searches run at 4 lanes. Lanes set here always
  * apply. */
 int msvgb_profile_set_lanes(msvgb_profile *prof, const msvgb_om *om, int lanes);
 int msvgb_profile_lanes(const msvgb_profile *prof);
@@ -134,7 +137,7 @@ int msvgb_profile_lanes(const msvgb_profile *prof);
  * where the 32-lane split passes apply) or no kernel is compiled for
  * (DP width, lanes, words). msvgb_profile_set_lanes (and so
  * msvgb_profile_create) sets the default for the model length and lane
- * count: 4 or 8 words from 10 DP words per lane up, measured 4-10% faster
+ * count: 4, 8 or 12 words from 10 DP words per lane up, measured 6-17% faster
  * than all-16-bit costs. */
 int msvgb_profile_set_ssv_int8_words(msvgb_profile *prof, const msvgb_om *om, int words);
 int msvgb_profile_ssv_int8_words(const msvgb_profile *prof);
