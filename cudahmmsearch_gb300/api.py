@@ -37,7 +37,7 @@ EXPORTS = [
     "msvgb_h3f_open", "msvgb_h3f_read", "msvgb_h3f_close", "msvgb_h3f_write", "msvgb_fasta_read",
     "msvgb_seqs_n", "msvgb_seqs_codes", "msvgb_seqs_offsets", "msvgb_seqs_name", "msvgb_seqs_free",
     "msvgb_db_save", "msvgb_db_load", "msvgb_db_lengths", "msvgb_search_host",
-    "msvgb_vprofile_create", "msvgb_vprofile_destroy", "msvgb_vitfilter", "msvgb_vit_score", "msvgb_vit_move_cost",
+    "msvgb_vprofile_create", "msvgb_vprofile_destroy", "msvgb_vitfilter", "msvgb_vit_score", "msvgb_vit_scores", "msvgb_vit_move_cost",
     "msvgb_biasfilter", "msvgb_bias_length_term", "msvgb_null_score", "msvgb_stage_pass", "msvgb_pipeline_filters",
     "msvgb_filter_collect", "msvgb_h3f_filter_params", "msvgb_h3p_open", "msvgb_h3p_read", "msvgb_h3p_close",
 ]
@@ -140,6 +140,7 @@ def lib():
         "msvgb_vprofile_destroy": (i32, [vp]),
         "msvgb_vitfilter": (i32, [vp, vp, vp, vp, ctypes.c_int64, vp, vp]),
         "msvgb_vit_score": (ctypes.c_float, [i32, i32, i32, ctypes.POINTER(_VOm)]),
+        "msvgb_vit_scores": (i32, [vp, vp, vp, i64, ctypes.POINTER(_VOm), vp]),
         "msvgb_vit_move_cost": (ctypes.c_int16, [ctypes.c_float, ctypes.c_float, i32]),
         "msvgb_profile_lanes": (i32, [vp]),
         "msvgb_profile_destroy": (i32, [vp]),
@@ -492,17 +493,11 @@ def vitfilter(ctx: Context, vprof: DeviceVProfile, db: DeviceDB, ids=None):
     st = np.zeros(ids.size, np.uint8)
     _check(lib().msvgb_vitfilter(ctx.h, vprof.h, db.h, ids.ctypes.data if ids.size else None, ids.size,
                                  xc.ctypes.data, st.ctypes.data))
-    # msvgb_vit_score's float expression (vitfilter.c:240-247), vectorized: the
-    # integer sums are exact in float32, the division is IEEE, and subtracting
-    # 3.0 in double then rounding equals the float32 subtraction here
-    vp = vprof.vp
-    L = db.lengths[ids].astype(np.int64)
-    uniq, inv = np.unique(L, return_inverse=True)
-    move = np.array([lib().msvgb_vit_move_cost(vp.scale_w, vp.nj, int(x)) for x in uniq], np.float32)[inv]
-    with np.errstate(over="ignore", invalid="ignore"):
-        sc = (xc.astype(np.float32) + move - np.float32(vp.base_w)) / np.float32(vp.scale_w) - np.float32(3.0)
-    sc = np.where(xc <= -32768, np.float32(-np.inf), sc).astype(np.float32)
-    sc = np.where(st == 1, np.float32(np.inf), sc).astype(np.float32)
+    o, keep = _vom_struct(vprof.vp)
+    lens = np.ascontiguousarray(db.lengths[ids], dtype=np.int32)
+    sc = np.empty(ids.size, np.float32)
+    _check(lib().msvgb_vit_scores(xc.ctypes.data, st.ctypes.data, lens.ctypes.data, ids.size, ctypes.byref(o),
+                                  sc.ctypes.data))
     return st, sc
 
 

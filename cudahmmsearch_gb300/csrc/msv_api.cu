@@ -66,25 +66,65 @@ static float score_from_xj(int xj, int tjb, int base, float scale) {
   return sc;
 }
 
-extern "C" float msvgb_score(uint8_t xj, uint8_t flags, int L, uint8_t base_b, float scale_b) {
+float msvgb_detail::score_at(uint8_t xj, uint8_t flags, int tjb, uint8_t base_b, float scale_b) {
   if (flags & MSVGB_FLAG_ERANGE) return INFINITY;
-  return score_from_xj(xj, msvgb_tjb_b(scale_b, L), base_b, scale_b);
+  return score_from_xj(xj, tjb, base_b, scale_b);
+}
+
+extern "C" float msvgb_score(uint8_t xj, uint8_t flags, int L, uint8_t base_b, float scale_b) {
+  return msvgb_detail::score_at(xj, flags, msvgb_tjb_b(scale_b, L), base_b, scale_b);
 }
 
 // p7_bg_SetLength/p7_bg_NullOne (src/p7_bg.c:191-199, 359-363), seq_score and
 // the F1 test of p7_Pipeline (src/p7_pipeline.c:673-676), esl_gumbel_surv
 // (easel/esl_gumbel.c:129-137).
+static int f1_pass_seq(float seq_score, float mmu, float mlambda, double F1, double *ret_P) {
+  double y = (double) mlambda * ((double) seq_score - (double) mmu);
+  double ey = -exp(-y);
+  double P = (fabs(ey) < 5e-9) ? -ey : 1 - exp(ey);
+  if (ret_P) *ret_P = P;
+  return (P > F1) ? 0 : 1;
+}
+
 extern "C" int msvgb_f1_pass(float usc, int L, float mmu, float mlambda, double F1, double *ret_P) {
   // C semantics: log() of a float argument is computed in double (C++'s
   // float overload of log would round differently).
   float p1 = (float) L / (float) (L + 1);
   float nullsc = (float) ((double) (float) L * ::log((double) p1) + ::log(1. - (double) p1));
   float seq_score = (usc - nullsc) / 0.69314718055994529;
-  double y = (double) mlambda * ((double) seq_score - (double) mmu);
-  double ey = -exp(-y);
-  double P = (fabs(ey) < 5e-9) ? -ey : 1 - exp(ey);
-  if (ret_P) *ret_P = P;
-  return (P > F1) ? 0 : 1;
+  return f1_pass_seq(seq_score, mmu, mlambda, F1, ret_P);
+}
+
+// The gate as an interval of the sequence score: above hi it passes, below lo
+// it does not, between them the P-value decides. P falls with the score; hi
+// and lo lie a relative 1e-5 beside the score where the computed P crosses F1,
+// where P differs from F1 by parts in 1e6, far more than its rounding. One
+// search of about 60 P-values per profile instead of about three per length.
+msvgb_detail::F1Gate msvgb_detail::f1_gate(float mmu, float mlambda, double F1) {
+  F1Gate g;
+  if (!(mlambda > 0.01f && mlambda < 100.0f && fabsf(mmu) < 1e4f && F1 > 1e-12 && F1 < 0.9)) return g;   // P-value for all
+  float a = mmu - 1000.0f / mlambda, b = mmu + 1000.0f / mlambda;     // P near 1, P near 0
+  if (f1_pass_seq(a, mmu, mlambda, F1, nullptr) || !f1_pass_seq(b, mmu, mlambda, F1, nullptr)) return g;
+  for (int i = 0; i < 60; ++i) {
+    const float m = 0.5f * (a + b);
+    (f1_pass_seq(m, mmu, mlambda, F1, nullptr) ? b : a) = m;
+  }
+  const float w = 1e-5f * (1.0f + fabsf(b) + fabsf(mmu));
+  g.lo = a - w;
+  g.hi = b + w;
+  return g;
+}
+
+// p7_bg_NullOne by length: constants, computed where first asked for.
+static float null_score_of(int L) {
+  static std::atomic<float> known[1 << 15];
+  if (L >= (1 << 15)) return msvgb_null_score(L);
+  float v = known[L].load(std::memory_order_relaxed);
+  if (v == 0.0f) {                                          // a null score is negative
+    v = msvgb_null_score(L);
+    known[L].store(v, std::memory_order_relaxed);
+  }
+  return v;
 }
 
 // ------------------------------------------------------------------------------
@@ -261,6 +301,7 @@ extern "C" int msvgb_ctx_destroy(msvgb_ctx *c) {
   cudaSetDevice(c->device);
   for (auto &e : c->dropin) msvgb_profile_destroy(e.p);
   c->dropin.clear();
+  msvgb_ctx_destroy(c->filter);
   if (c->own) cudaStreamSynchronize(c->own);
   cudaFree(c->d_ticket);
   cudaFree(c->d_one); cudaFree(c->d_bad); cudaFree(c->d_list); cudaFree(c->d_seg);
@@ -668,10 +709,14 @@ extern "C" int msvgb_profile_ssv_int8_words(const msvgb_profile *p) {
 // ------------------------------------------------------------------------------
 // per-length tables: tjb_b(L) and the smallest xJ that passes F1 at length L
 
-int msvgb_detail::xjmin_for(const msvgb_profile *p, int L, double F1, int hint) {
+int msvgb_detail::xjmin_for(const msvgb_profile *p, int L, double F1, int hint, const F1Gate &gate) {
   const int tjb = msvgb_tjb_b(p->scale, L);
+  const float nullsc = null_score_of(L);
   auto pass = [&](int xj) {
-    return msvgb_f1_pass(score_from_xj(xj, tjb, p->base, p->scale), L, p->mmu, p->mlambda, F1, nullptr) != 0;
+    const float seq_score = (score_from_xj(xj, tjb, p->base, p->scale) - nullsc) / 0.69314718055994529;
+    if (seq_score > gate.hi) return true;
+    if (seq_score < gate.lo) return false;
+    return f1_pass_seq(seq_score, p->mmu, p->mlambda, F1, nullptr) != 0;
   };
   if (hint >= 0 && hint <= 255) {
     // Walk from a nearby length's answer (the boundary moves by a unit or two
@@ -712,8 +757,7 @@ int msvgb_detail::ensure_tables(msvgb_profile *p, const msvgb_db *db, double F1,
   bool dirty = false;
   if (need > t->cap) {                                  // grow: host images and device buffers
     const int cap = std::max({need, 2 * t->cap, 1024});
-    t->tjb.resize(cap);
-    for (int L = t->cap; L < cap; ++L) t->tjb[L] = msvgb_tjb_b(p->scale, L);
+    t->tjb.resize(cap, 0);                              // entries of lengths that occur, below
     t->xjm.resize(cap, -1);
     uint8_t *nt = nullptr, *nx = nullptr;
     cudaError_t e = cudaMalloc(&nt, cap);
@@ -728,11 +772,15 @@ int msvgb_detail::ensure_tables(msvgb_profile *p, const msvgb_db *db, double F1,
     dirty = true;
   }
   int hint = -1;                                        // the last length's answer (lengths ascend)
+  F1Gate gate;
+  bool gated = false;
   for (int L : db->distinct_len) {
     if (L == 0) continue;
     if (t->xjm[L] >= 0) { hint = t->xjm[L]; continue; }
-    const int v = xjmin_for(p, L, F1, hint);
+    if (!gated) { gate = f1_gate(p->mmu, p->mlambda, F1); gated = true; }
+    const int v = xjmin_for(p, L, F1, hint, gate);
     if (v < 0) return fail(MSVGB_eslESYS, "F1 pass set is not monotone in xJ");
+    t->tjb[L] = msvgb_tjb_b(p->scale, L);
     t->xjm[L] = (int16_t) v;
     hint = v;
     dirty = true;
@@ -786,6 +834,18 @@ static cudaError_t grow_pinned(msvgb_ctx *ctx, size_t need) {
   cudaError_t e = cudaMallocHost(&ctx->h_pin, need);
   if (e == cudaSuccess) ctx->h_pin_cap = need;
   return e;
+}
+
+uint8_t *msvgb_detail::pinned_scratch(msvgb_ctx *ctx, size_t bytes) {
+  if (ctx->h_pin_cap < bytes && grow_pinned(ctx, bytes + bytes / 2) != cudaSuccess) return nullptr;
+  return (uint8_t *) ctx->h_pin;
+}
+
+bool msvgb_detail::is_pinned(const void *p) {
+  cudaPointerAttributes a{};
+  const cudaError_t e = cudaPointerGetAttributes(&a, p);
+  (void) cudaGetLastError();
+  return e == cudaSuccess && a.type == cudaMemoryTypeHost;
 }
 
 cudaMemPool_t msvgb_detail::scratch_pool(int device) {
@@ -1455,11 +1515,23 @@ int msvgb_detail::host_search(msvgb_ctx *c, const msvgb_profile *pc, const uint8
   if (st == MSVGB_eslOK) st = ensure_tables(p, db, F1, &t);
   if (st == MSVGB_eslOK) st = search_chunked(c, p, db, t, d, d + n, ctr, d_list, gt);
   pt.mark("search_host: enqueued");
-  int bad = 0;
+  // results: straight into pinned buffers, else through the context's pinned
+  // scratch (a copy into pageable memory may run as a kernel and then waits
+  // for other streams' kernels to leave the SMs)
+  const bool direct = is_pinned(out_xj) && is_pinned(out_flags);
+  uint8_t *back = nullptr;                                   // [xj n | flags n | bad], or [bad]
   if (st == MSVGB_eslOK) {
-    e = cudaMemcpyAsync(out_xj, d, n, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(out_flags, d + n, n, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+    back = pinned_scratch(c, direct ? 16 : o_bad + 16);
+    if (!back) st = fail(MSVGB_eslEMEM, "search: pinned scratch");
+  }
+  if (st == MSVGB_eslOK) {
+    if (direct) {
+      e = cudaMemcpyAsync(out_xj, d, n, cudaMemcpyDeviceToHost, c->stream);
+      if (e == cudaSuccess) e = cudaMemcpyAsync(out_flags, d + n, n, cudaMemcpyDeviceToHost, c->stream);
+      if (e == cudaSuccess) e = cudaMemcpyAsync(back, d_bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+    } else {
+      e = cudaMemcpyAsync(back, d, o_bad + sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+    }
     if (e != cudaSuccess) st = fail(MSVGB_eslESYS, std::string("search: ") + cudaGetErrorString(e));
   }
   cudaStreamSynchronize(c->upload);
@@ -1470,6 +1542,14 @@ int msvgb_detail::host_search(msvgb_ctx *c, const msvgb_profile *pc, const uint8
   pt.mark("search_host: done");
   gt.mark("results back", c->stream);
   if (st == MSVGB_eslOK && e != cudaSuccess) st = fail(MSVGB_eslESYS, std::string("search: ") + cudaGetErrorString(e));
+  int bad = 0;
+  if (st == MSVGB_eslOK) {
+    memcpy(&bad, direct ? back : back + o_bad, sizeof bad);
+    if (!direct) {
+      memcpy(out_xj, back, (size_t) n);
+      memcpy(out_flags, back + n, (size_t) n);
+    }
+  }
   if (st == MSVGB_eslOK && bad) st = fail(MSVGB_eslEINVAL, "residue code >= 29 (Kp)");
   if (keep_db && st == MSVGB_eslOK) {                       // packed and complete: the stream was synchronized
     db->d_bad_chunks = nullptr;                               // pointed into this call's scratch

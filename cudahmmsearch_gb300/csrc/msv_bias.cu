@@ -428,7 +428,11 @@ extern "C" int msvgb_biasfilter(msvgb_ctx *c, const float *compo, int M, const m
   int32_t *d_cnt = (int32_t *) (d_scr + 2 * a8);
   float *d_out = (float *) (d_scr + 2 * a8 + 4096);
   int32_t *d_len = (int32_t *) (d_scr + 2 * a8 + 4096 + a4);
-  cudaError_t e = cudaMemcpyAsync(d_ids, ids, nids * 8, cudaMemcpyHostToDevice, c->stream);
+  // ids up and results back through pinned scratch (pageable copies may run as kernels)
+  uint8_t *pin = msvgb_detail::pinned_scratch(c, a8 + 2 * a4);
+  if (!pin) { cudaFreeAsync(d_scr, c->stream); return fail(MSVGB_eslEMEM, "biasfilter: pinned scratch"); }
+  memcpy(pin, ids, (size_t) nids * 8);
+  cudaError_t e = cudaMemcpyAsync(d_ids, pin, nids * 8, cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) e = msvgb_detail::launch_gather_ids(d_ids, nids, db->d_inv, c->num_sms, c->stream);
   if (e == cudaSuccess)
     e = msvgb_detail::launch_order_by_length(d_ids, nids, db->d_len, db->Lmax, d_cnt, d_order, c->num_sms, c->stream);
@@ -437,21 +441,22 @@ extern "C" int msvgb_biasfilter(msvgb_ctx *c, const float *compo, int M, const m
     e = launch_bias(B, dbv, d_ids, d_order, nids, d_out, d_len, c->stream);
   }
   if (e == cudaSuccess) msvgb_detail::count_launch();
-  std::vector<char> back(2 * a4);                                // scores, then lengths, in one copy
-  const float *sc = (const float *) back.data();
-  const int32_t *lens = (const int32_t *) (back.data() + a4);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(back.data(), d_out, a4 + (size_t) nids * 4, cudaMemcpyDeviceToHost, c->stream);
+  const float *sc = (const float *) (pin + a8);                  // scores, then lengths, in one copy
+  const int32_t *lens = (const int32_t *) (pin + a8 + a4);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(pin + a8, d_out, a4 + (size_t) nids * 4, cudaMemcpyDeviceToHost, c->stream);
   cudaFreeAsync(d_scr, c->stream);
   const cudaError_t e2 = cudaStreamSynchronize(c->stream);
   if (e == cudaSuccess) e = e2;
   if (e != cudaSuccess) return fail(MSVGB_eslESYS, std::string("biasfilter: ") + cudaGetErrorString(e));
   // the length terms, one pair of logarithms per length (L logf(p1), then logf(1 - p1), as
-  // msvgb_bias_length_term adds them)
-  std::vector<float2> term((size_t) db->Lmax + 1, make_float2(NAN, 0.0f));
+  // msvgb_bias_length_term adds them); the few lengths past kTerms each time
+  constexpr int kTerms = 1 << 16;
+  std::vector<float2> term((size_t) std::min(db->Lmax, kTerms) + 1, make_float2(NAN, 0.0f));
   for (int64_t j = 0; j < nids; ++j) {
     const int L = lens[j];
     if (L <= 0) { out_sc[j] = 0.0f; continue; }
-    float2 &t = term[L];
+    float2 past = make_float2(NAN, 0.0f);
+    float2 &t = L <= kTerms ? term[L] : past;
     if (std::isnan(t.x)) t = length_terms(L);
     out_sc[j] = sc[j] + t.x + t.y;
   }

@@ -2,6 +2,7 @@
 // (not part of the public interface).
 #pragma once
 #include <chrono>
+#include <cmath>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
@@ -52,6 +53,7 @@ struct msvgb_ctx {
   cudaStream_t dma = nullptr;                           // raw residue copies of database creation
   void *h_pin = nullptr; size_t h_pin_cap = 0;          // small pinned scratch (length counts, flags)
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  msvgb_ctx *filter = nullptr;                          // second context of msvgb_pipeline_filters, made at its first call
   TuneTable *tune = nullptr;                            // lane counts measured by msvgb_autotune
   std::mutex tune_mu;
 };
@@ -186,12 +188,17 @@ cudaError_t ensure_inverse(msvgb_ctx *c, const msvgb_db *db);
 extern const float kAminoBg[20];
 // Records msg as the calling thread's last error and returns code.
 int fail(int code, const std::string &msg);
+// msvgb_score with the length's tjb_b.
+float score_at(uint8_t xj, uint8_t flags, int tjb, uint8_t base_b, float scale_b);
 // Launches the search kernel instantiated for C words per lane.
 cudaError_t dispatch(int C, bool f16, const msvgb::LaunchArgs &a, int sms);
 // Smallest xJ passing the F1 gate at length L (255: none); -1 if the pass set
 // is not monotone in xJ.
 // hint: the answer at a nearby length (walked from instead of a binary search), or -1.
-int xjmin_for(const msvgb_profile *p, int L, double F1, int hint = -1);
+// gate: f1_gate of the profile and F1 (default: every P-value computed).
+struct F1Gate { float lo = -INFINITY, hi = INFINITY; };
+F1Gate f1_gate(float mmu, float mlambda, double F1);
+int xjmin_for(const msvgb_profile *p, int L, double F1, int hint = -1, const F1Gate &gate = F1Gate());
 // Marks a profile's lanes as its own choice (msvgb_profile_create): its large
 // searches may then run on 4 lanes per sequence.
 int profile_auto_lanes(msvgb_profile *p, const msvgb_om *om);
@@ -329,6 +336,10 @@ cudaError_t launch_bins(const unsigned long long *hist, int Lmax, int K, int64_t
 // pool, which keeps up to 4 GiB mapped between calls (the default pool would
 // unmap and map again every time).
 cudaMemPool_t scratch_pool(int device);
+// The context's pinned scratch, grown to bytes (null: out of memory). No copy
+// from or into it may be pending.
+uint8_t *pinned_scratch(msvgb_ctx *ctx, size_t bytes);
+bool is_pinned(const void *p);
 // cursor: each key's first slot (used by the long sequences); blk as
 // launch_histogram left it.
 cudaError_t launch_place(const int64_t *off, const int32_t *len_in, int64_t n, unsigned long long *cursor,

@@ -118,17 +118,44 @@ struct HitBlock {
   std::vector<msvgb_filter_hit> hits;
 };
 
+// The logarithms the host takes per survivor depend on its length only: one
+// null score and one tjb_b per length below kLens (a block's survivors share a
+// few thousand lengths).
+struct LenMemo {
+  static constexpr int kLens = 1 << 16;
+  std::vector<float> null;                    // NaN: not computed yet
+  std::vector<int16_t> tjb;                   // -1: not computed yet
+  void reach(int L) {
+    if ((size_t) L < null.size()) return;
+    null.resize((size_t) std::min(kLens, L + L / 2 + 1024), NAN);
+    tjb.resize(null.size(), -1);
+  }
+  float null_score(int L) {
+    if (L >= kLens) return msvgb_null_score(L);
+    reach(L);
+    if (std::isnan(null[L])) null[L] = msvgb_null_score(L);
+    return null[L];
+  }
+  int tjb_b(float scale, int L) {
+    if (L >= kLens) return msvgb_tjb_b(scale, L);
+    reach(L);
+    if (tjb[L] < 0) tjb[L] = msvgb_tjb_b(scale, L);
+    return tjb[L];
+  }
+};
+
 // The bias and Viterbi stages of one block (sequences b0 .. b0 + nb of the
 // caller's arrays, resident as db). keep: local indices and MSV scores of the
 // F1 survivors. Appends the sequences past the last stage to out.
 int filter_block(msvgb_ctx *ctx, const msvgb_filters *f, msvgb_vprofile *vp, const msvgb_db *db, int64_t b0,
                  const int64_t *off, const std::vector<int64_t> &keep, const std::vector<float> &usc,
-                 msvgb_filter_stats &stats, std::vector<msvgb_filter_hit> &out, msvgb_detail::GpuTrace &gt) {
+                 LenMemo &memo, msvgb_filter_stats &stats, std::vector<msvgb_filter_hit> &out,
+                 msvgb_detail::GpuTrace &gt) {
   const std::string tag = "b" + std::to_string(b0) + " ";
   const size_t ns = keep.size();
   std::vector<float> fsc(ns), nsc(ns);
   std::vector<double> P(ns);
-  for (size_t j = 0; j < ns; ++j) nsc[j] = msvgb_null_score((int) (off[b0 + keep[j] + 1] - off[b0 + keep[j]]));
+  for (size_t j = 0; j < ns; ++j) nsc[j] = memo.null_score((int) (off[b0 + keep[j] + 1] - off[b0 + keep[j]]));
   if (f->compo) {
     gt.mark(tag + "bias start", ctx->stream);
     int st = msvgb_biasfilter(ctx, f->compo, f->om->M, db, keep.data(), (int64_t) ns, fsc.data());
@@ -163,10 +190,14 @@ int filter_block(msvgb_ctx *ctx, const msvgb_filters *f, msvgb_vprofile *vp, con
     int st = msvgb_vitfilter(ctx, vp, db, vids.data(), (int64_t) vids.size(), xc.data(), vst.data());
     if (st != MSVGB_eslOK) return st;
     gt.mark(tag + "vit done", ctx->stream);
+    std::vector<int32_t> len(vids.size());
+    std::vector<float> vsc(vids.size());
+    for (size_t t = 0; t < vids.size(); ++t) len[t] = (int32_t) (off[b0 + vids[t] + 1] - off[b0 + vids[t]]);
+    st = msvgb_vit_scores(xc.data(), vst.data(), len.data(), (int64_t) vids.size(), f->vom, vsc.data());
+    if (st != MSVGB_eslOK) return st;
     for (size_t t = 0; t < vids.size(); ++t) {
       const size_t j = vpos[t];
-      const int L = (int) (off[b0 + keep[j] + 1] - off[b0 + keep[j]]);
-      const float vfsc = msvgb_vit_score(xc[t], vst[t], L, f->vom);
+      const float vfsc = vsc[t];
       if (msvgb_stage_pass(vfsc, fsc[j], f->vmu, f->vlambda, f->F2, nullptr)) {
         hit(j, vfsc);
         ++passed;
@@ -214,12 +245,12 @@ extern "C" int msvgb_pipeline_filters(msvgb_ctx *ctx, const msvgb_filters *f, co
   msvgb_ctx *fctx = nullptr;
   msvgb_profile *prof = nullptr;
   msvgb_vprofile *vp = nullptr;
-  int st = msvgb_ctx_create(ctx->device, &fctx);
+  int st = ctx->filter ? MSVGB_eslOK : msvgb_ctx_create(ctx->device, &ctx->filter);
+  fctx = ctx->filter;
   if (st == MSVGB_eslOK) st = msvgb_profile_create(ctx, f->om, &prof);
   if (st == MSVGB_eslOK && f->vom) st = msvgb_vprofile_create(fctx, f->vom, &vp);
   if (st != MSVGB_eslOK) {
     msvgb_profile_destroy(prof);
-    msvgb_ctx_destroy(fctx);
     return st;
   }
 
@@ -236,6 +267,7 @@ extern "C" int msvgb_pipeline_filters(msvgb_ctx *ctx, const msvgb_filters *f, co
   std::string fmsg;
 
   auto filter_thread = [&]() {
+    LenMemo memo;
     for (;;) {
       MsvBlock *b = nullptr;
       {
@@ -259,11 +291,12 @@ extern "C" int msvgb_pipeline_filters(msvgb_ctx *ctx, const msvgb_filters *f, co
           const int L = (int) (off[b->b0 + i + 1] - off[b->b0 + i]);
           if (L == 0) continue;
           keep.push_back(i);
-          usc.push_back(msvgb_score(b->xj[i], fl[i], L, f->om->base_b, f->om->scale_b));
+          usc.push_back(msvgb_detail::score_at(b->xj[i], fl[i], memo.tjb_b(f->om->scale_b, L), f->om->base_b,
+                                               f->om->scale_b));
         }
         stats.n_past_msv += (int64_t) keep.size();
         gt.mark("b" + std::to_string(b->b0) + " survivors listed", nullptr);
-        s2 = filter_block(fctx, f, vp, b->db, b->b0, off, keep, usc, stats, hb->hits, gt);
+        s2 = filter_block(fctx, f, vp, b->db, b->b0, off, keep, usc, memo, stats, hb->hits, gt);
       }
       msvgb_detail::db_release_on(b->db, fctx->stream);   // after its filter stages, without a device-wide wait
       delete b;
@@ -341,7 +374,6 @@ extern "C" int msvgb_pipeline_filters(msvgb_ctx *ctx, const msvgb_filters *f, co
   for (HitBlock *b : hits) delete b;
   msvgb_vprofile_destroy(vp);
   msvgb_profile_destroy(prof);
-  msvgb_ctx_destroy(fctx);
   gt.mark("torn down", nullptr);
   gt.print();
   if (ret_stats) *ret_stats = stats;

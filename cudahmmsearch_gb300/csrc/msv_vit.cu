@@ -737,6 +737,29 @@ extern "C" float msvgb_vit_score(int xc, int status, int L, const msvgb_vom *vom
   return sc;
 }
 
+extern "C" int msvgb_vit_scores(const int *xc, const uint8_t *status, const int32_t *len, int64_t n,
+                                const msvgb_vom *vom, float *out) {
+  if (n < 0 || !vom || (n && (!xc || !status || !len || !out))) return fail(MSVGB_eslEINVAL, "NULL argument");
+  // msvgb_vit_score with one move cost (a logarithm) per length below kMoves
+  constexpr int kMoves = 1 << 16;
+  std::vector<int32_t> move;
+  for (int64_t j = 0; j < n; ++j) {
+    const int L = len[j];
+    if (L < 0) return fail(MSVGB_eslEINVAL, "negative length");
+    if (status[j] == 1) { out[j] = INFINITY; continue; }
+    if (xc[j] <= -32768) { out[j] = -INFINITY; continue; }
+    if (L < kMoves && (size_t) L >= move.size()) move.resize((size_t) std::min(kMoves, L + 1 + L / 2), INT32_MIN);
+    int32_t past = INT32_MIN;
+    int32_t &mv = L < kMoves ? move[L] : past;
+    if (mv == INT32_MIN) mv = msvgb_vit_move_cost(vom->scale_w, vom->nj, L);
+    float sc = (float) xc[j] + (float) mv - (float) vom->base_w;
+    sc /= vom->scale_w;
+    sc -= 3.0;
+    out[j] = sc;
+  }
+  return MSVGB_eslOK;
+}
+
 extern "C" int msvgb_vprofile_create(msvgb_ctx *ctx, const msvgb_vom *v, msvgb_vprofile **ret) {
   if (!ctx || !v || !ret || !v->twv || !v->rwv) return fail(MSVGB_eslEINVAL, "NULL argument");
   *ret = nullptr;
@@ -872,12 +895,18 @@ extern "C" int msvgb_vitfilter(msvgb_ctx *c, msvgb_vprofile *p, const msvgb_db *
   // one scratch block: list slots and order (int64), bucket counts, xC and statuses
   const size_t a8 = ((size_t) nids * 8 + 255) & ~(size_t) 255, a4 = ((size_t) nids * 4 + 255) & ~(size_t) 255;
   char *d_scr = nullptr;
-  CUDA_TRY(cudaMallocAsync((void **) &d_scr, 2 * a8 + 4096 + a4 + (size_t) nids, c->stream));
+  cudaMemPool_t pool = msvgb_detail::scratch_pool(c->device);   // stays mapped between calls
+  if (!pool) return fail(MSVGB_eslESYS, "vitfilter: no memory pool");
+  CUDA_TRY(cudaMallocFromPoolAsync((void **) &d_scr, 2 * a8 + 4096 + a4 + (size_t) nids, pool, c->stream));
   int64_t *d_ids = (int64_t *) d_scr, *d_order = (int64_t *) (d_scr + a8);
   int32_t *d_cnt = (int32_t *) (d_scr + 2 * a8);
   int *d_xc = (int *) (d_scr + 2 * a8 + 4096);
   uint8_t *d_st = (uint8_t *) (d_scr + 2 * a8 + 4096 + a4);
-  cudaError_t e = cudaMemcpyAsync(d_ids, ids, nids * 8, cudaMemcpyHostToDevice, c->stream);
+  // ids up and results back through pinned scratch (pageable copies may run as kernels)
+  uint8_t *pin = msvgb_detail::pinned_scratch(c, a8 + a4 + (size_t) nids);
+  if (!pin) { cudaFreeAsync(d_scr, c->stream); return fail(MSVGB_eslEMEM, "vitfilter: pinned scratch"); }
+  memcpy(pin, ids, (size_t) nids * 8);
+  cudaError_t e = cudaMemcpyAsync(d_ids, pin, nids * 8, cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) e = msvgb_detail::launch_gather_ids(d_ids, nids, db->d_inv, c->num_sms, c->stream);
   if (e == cudaSuccess)
     e = msvgb_detail::launch_order_by_length(d_ids, nids, db->d_len, db->Lmax, d_cnt, d_order, c->num_sms, c->stream);
@@ -896,11 +925,13 @@ extern "C" int msvgb_vitfilter(msvgb_ctx *c, msvgb_vprofile *p, const msvgb_db *
     e = fast ? dispatch_vit_fast(p->fast_form, VF, dbv, d_ids, d_order, nids, d_xc, d_st, c->d_ticket, c->num_sms, c->stream)
              : dispatch_vit(p->CV, V, dbv, d_ids, d_order, nids, d_xc, d_st, c->d_ticket, c->num_sms, c->stream);
   if (e == cudaSuccess) msvgb_detail::count_launch();
-  if (e == cudaSuccess) e = cudaMemcpyAsync(out_xc, d_xc, nids * 4, cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(out_status, d_st, nids, cudaMemcpyDeviceToHost, c->stream);
+  const uint8_t *back = pin + a8;                                // xC, then statuses, in one copy
+  if (e == cudaSuccess) e = cudaMemcpyAsync(pin + a8, d_xc, a4 + (size_t) nids, cudaMemcpyDeviceToHost, c->stream);
   cudaFreeAsync(d_scr, c->stream);
   const cudaError_t e2 = cudaStreamSynchronize(c->stream);
   if (e == cudaSuccess) e = e2;
   if (e != cudaSuccess) return fail(MSVGB_eslESYS, std::string("vitfilter: ") + cudaGetErrorString(e));
+  memcpy(out_xc, back, (size_t) nids * 4);
+  memcpy(out_status, back + a4, (size_t) nids);
   return MSVGB_eslOK;
 }

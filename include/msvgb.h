@@ -194,6 +194,9 @@ int msvgb_vitfilter(msvgb_ctx *ctx, msvgb_vprofile *vp, const msvgb_db *db, cons
 /* The filter score in nats from xC (vitfilter.c:240-247, exact float
  * expressions) and the per-length N/J/C move cost. */
 float   msvgb_vit_score(int xc, int status, int L, const msvgb_vom *vom);
+/* The same for n listed results (targets of length len[j]). */
+int     msvgb_vit_scores(const int *xc, const uint8_t *status, const int32_t *len, int64_t n, const msvgb_vom *vom,
+                         float *out);
 int16_t msvgb_vit_move_cost(float scale_w, float nj, int L);
 
 /* ---- the bias filter: p7_bg_FilterScore (src/p7_bg.c:473-483) -----------------
