@@ -240,58 +240,233 @@ __device__ __forceinline__ void bias_add(const float (&mx)[16 / G], float (&lg)[
   }
 }
 
+// Shared-memory copies of the filter's odds and the log table.
+struct BiasShared {
+  float2 eo[NRES];
+  double2 logtab[kLogTab];
+  __device__ __forceinline__ void load(const BiasDev &B) {
+    for (int i = threadIdx.x; i < NRES; i += blockDim.x) eo[i] = make_float2(B.eo[i][0], B.eo[i][1]);
+    for (int i = threadIdx.x; i < kLogTab; i += blockDim.x) logtab[i] = B.logtab[i];
+    __syncthreads();
+  }
+};
+
+// The Forward score of one sequence, without its length terms.
+template <int G, bool ONE>
+__device__ __forceinline__ float bias_score(const BiasDev &B, const BiasShared &sh, const uint4 *sq, int L, int glane,
+                                            unsigned gmask) {
+  constexpr int K = 16 / G;                      // logs per lane and batch
+  const float t00 = __fdiv_rn((float) L, (float) (L + 1)), t01 = __fadd_rn(1.0f, -t00);
+  float d0 = 0.0f, d1 = 0.0f, logsc = 0.0f;
+  float mx[K], lg[K];                            // this lane's row maxima of the last batch, logs not yet taken
+#pragma unroll
+  for (int k = 0; k < K; ++k) mx[k] = 1.0f;
+  bias_rows<G, ONE, true, false>(B, sh.eo, sq[0], L, glane, t00, t01, d0, d1, mx);
+  int i0 = 16;
+  for (; i0 + 16 <= L; i0 += 16) {               // the previous batch (rows i0-16 .. i0-1) is full
+    float nm[K];
+    const uint32_t fail = bias_logs(mx, lg);
+    bias_rows<G, ONE, false, true>(B, sh.eo, sq[i0 >> 4], 16, glane, t00, t01, d0, d1, nm);
+    bias_add<G>(mx, lg, fail, 16, sh.logtab, gmask, logsc);
+#pragma unroll
+    for (int k = 0; k < K; ++k) mx[k] = nm[k];
+  }
+  if (i0 < L) {
+    float nm[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) nm[k] = 1.0f;
+    const uint32_t fail = bias_logs(mx, lg);
+    bias_rows<G, ONE, false, false>(B, sh.eo, sq[i0 >> 4], L - i0, glane, t00, t01, d0, d1, nm);
+    bias_add<G>(mx, lg, fail, 16, sh.logtab, gmask, logsc);
+#pragma unroll
+    for (int k = 0; k < K; ++k) mx[k] = nm[k];
+  }
+  const uint32_t fail = bias_logs(mx, lg);
+  bias_add<G>(mx, lg, fail, (L - 1) % 16 + 1, sh.logtab, gmask, logsc);
+  return __fadd_rn(logsc, log_rowf(__fadd_rn(d0, d1), sh.logtab));   // dp[L][0] * 1 + dp[L][1] * 1
+}
+
+// ---- long sequences in segments ---------------------------------------------------
+// The chain of a long sequence is cut into segments of kBiasSeg rows that run
+// side by side. A segment does not know the state (d0, d1) it starts from: it
+// starts kBiasWarm rows early from a guess. The filter forgets its state (each
+// row's map contracts, by t11 and the odds of the two compositions), so after
+// the run-in two runs are usually equal in every bit, rounding included; and
+// when the state a segment had at its first row equals, bit for bit, the state
+// the segment before ended in, its rows are the sequence's own. That is
+// checked for every segment, and a sequence that fails is scored from its
+// start, so no result depends on the guess. The row logs go to memory and are
+// summed in row order by one thread: four clocks a row against about 180 for
+// the chain.
+//
+// Run-in of 1024 rows: in a float simulation on background sequences, runs
+// from the guess still differed after 512 rows in 26% of cases with the
+// Pkinase model (composition close to the background: it forgets slowest),
+// after 768 in 0.05%, and in none of 4,000 with four other models after 512.
+constexpr int kBiasSeg = 512, kBiasWarm = 1024, kBiasLong = 3 * kBiasSeg;
+
+struct BiasSegs {                                // of one call; counters zeroed
+  unsigned *n;                                   // [0] long sequences, [1] segments, [2] rows
+  unsigned cap_seq, cap_item, cap_row;           // rows in units of kBiasSeg
+  int32_t *seq;                                  // [cap_seq] list position
+  unsigned *first, *row;                         // [cap_seq] first segment, first block of rows in lg
+  uint2 *item;                                   // [cap_item] long sequence, segment
+  float4 *state;                                 // [cap_item] (d0, d1) before its first row and after its last
+  float *lg;                                     // [cap_row * kBiasSeg] row logs
+  uint8_t *is_long;                              // [nids]
+};
+
+// Picks the long sequences of the list while there is room for them.
+__global__ void __launch_bounds__(256)
+bias_plan_kernel(DbDev db, const int64_t *__restrict__ slots, int64_t nids, BiasSegs S) {
+  const int64_t j = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= nids) return;
+  const int L = db.len[slots[j]];
+  uint8_t is_long = 0;
+  if (L > kBiasLong) {
+    const unsigned nseg = (unsigned) (L + kBiasSeg - 1) / kBiasSeg;
+    const unsigned r = atomicAdd(&S.n[2], nseg);
+    if (r + nseg <= S.cap_row) {                 // cap_seq and cap_item are cap_row or more
+      const unsigned e = atomicAdd(&S.n[0], 1u), f = atomicAdd(&S.n[1], nseg);
+      S.seq[e] = (int32_t) j;
+      S.first[e] = f;
+      S.row[e] = r;
+      for (unsigned k = 0; k < nseg; ++k) S.item[f + k] = make_uint2(e, k);
+      is_long = 1;
+    }
+  }
+  S.is_long[j] = is_long;
+}
+
+template <int G, bool ONE>
+__device__ __forceinline__ void bias_segment(const BiasDev &B, const BiasShared &sh, const DbDev &db,
+                                             const int64_t *slots, const BiasSegs &S, unsigned it, int glane) {
+  constexpr int K = 16 / G;
+  const uint2 item = S.item[it];
+  const int64_t s = slots[S.seq[item.x]];
+  const int L = db.len[s], r0 = (int) item.y * kBiasSeg, r1 = min(L, r0 + kBiasSeg);
+  const uint4 *sq = reinterpret_cast<const uint4 *>(db.codes + db.start[s]);
+  float *lg_out = S.lg + (size_t) (S.row[item.x] + item.y) * kBiasSeg;
+  const float t00 = __fdiv_rn((float) L, (float) (L + 1)), t01 = __fadd_rn(1.0f, -t00);
+  float d0 = 1.0f, d1 = 0.05f;                   // the guess
+  float mx[K], nm[K], lg[K];
+  int i = r0 == 0 ? 0 : r0 - kBiasWarm;
+  if (i <= 0 && r0 > 0) {                        // no guess: from the sequence's start
+    bias_rows<G, ONE, true, false>(B, sh.eo, sq[0], 16, glane, t00, t01, d0, d1, nm);
+    i = 16;
+  }
+  for (; i < r0; i += 16)
+    bias_rows<G, ONE, false, true>(B, sh.eo, sq[i >> 4], 16, glane, t00, t01, d0, d1, nm);
+  const float s0 = d0, s1 = d1;
+  // as bias_score: the logs of one batch beside the next batch's recurrence
+  auto store = [&](int row, uint32_t fail) {
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      lg_out[row + k * G + glane] = (fail >> k & 1u) ? log_row(mx[k], sh.logtab) : lg[k];
+  };
+#pragma unroll
+  for (int k = 0; k < K; ++k) mx[k] = 1.0f;
+  if (r0 == 0) bias_rows<G, ONE, true, false>(B, sh.eo, sq[0], 16, glane, t00, t01, d0, d1, mx);
+  else         bias_rows<G, ONE, false, false>(B, sh.eo, sq[r0 >> 4], r1 - r0, glane, t00, t01, d0, d1, mx);
+  int i0 = r0 + 16;
+  for (; i0 + 16 <= r1; i0 += 16) {
+    const uint32_t fail = bias_logs(mx, lg);
+    bias_rows<G, ONE, false, true>(B, sh.eo, sq[i0 >> 4], 16, glane, t00, t01, d0, d1, nm);
+    store(i0 - 16 - r0, fail);
+#pragma unroll
+    for (int k = 0; k < K; ++k) mx[k] = nm[k];
+  }
+  if (i0 < r1) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) nm[k] = 1.0f;
+    const uint32_t fail = bias_logs(mx, lg);
+    bias_rows<G, ONE, false, false>(B, sh.eo, sq[i0 >> 4], r1 - i0, glane, t00, t01, d0, d1, nm);
+    store(i0 - 16 - r0, fail);
+#pragma unroll
+    for (int k = 0; k < K; ++k) mx[k] = nm[k];
+    i0 += 16;
+  }
+  const uint32_t fail = bias_logs(mx, lg);
+  store(i0 - 16 - r0, fail);                     // the last batch may end in rows no one reads
+  if (glane == 0) S.state[it] = make_float4(s0, s1, d0, d1);
+}
+
+// Groups of G lanes: the first cap_item of them a segment of a long sequence
+// each, the others one listed sequence each.
 template <int G, bool ONE>
 __global__ void __launch_bounds__(128)
 bias_kernel(BiasDev B, DbDev db, const int64_t *__restrict__ slots, const int64_t *__restrict__ order, int64_t nids,
-            float *__restrict__ out, int32_t *__restrict__ out_len) {
-  constexpr int K = 16 / G;                      // logs per lane and batch
-  __shared__ float2 s_eo[NRES];
-  __shared__ double2 s_log[kLogTab];
-  for (int i = threadIdx.x; i < NRES; i += blockDim.x) s_eo[i] = make_float2(B.eo[i][0], B.eo[i][1]);
-  for (int i = threadIdx.x; i < kLogTab; i += blockDim.x) s_log[i] = B.logtab[i];
-  __syncthreads();
+            BiasSegs S, float *__restrict__ out, int32_t *__restrict__ out_len) {
+  __shared__ BiasShared sh;
   const int lane = threadIdx.x & 31, glane = lane % G;
   const unsigned gmask = ((1u << G) - 1u) << (lane - glane);
-  const int64_t t = ((int64_t) blockIdx.x * blockDim.x + threadIdx.x) / G;
+  const int64_t g = ((int64_t) blockIdx.x * blockDim.x + threadIdx.x) / G;
+  if ((int64_t) blockIdx.x * blockDim.x / G >= (int64_t) S.n[1] && ((int64_t) blockIdx.x + 1) * blockDim.x / G <= S.cap_item)
+    return;                                      // a block past the last segment
+  sh.load(B);
+  if (g < S.cap_item) {
+    if (g < S.n[1]) bias_segment<G, ONE>(B, sh, db, slots, S, (unsigned) g, glane);
+    return;
+  }
+  const int64_t t = g - S.cap_item;
   if (t >= nids) return;
   const int64_t j = order[t];
   const int64_t s = slots[j];
   const int L = db.len[s];
   if (glane == 0) out_len[j] = L;
   if (L <= 0) { if (glane == 0) out[j] = 0.0f; return; }
-  const uint4 *sq = reinterpret_cast<const uint4 *>(db.codes + db.start[s]);   // 16-byte aligned, padded to 16
-  const float p1 = __fdiv_rn((float) L, (float) (L + 1));
-  const float t00 = p1, t01 = __fadd_rn(1.0f, -p1);
-  float d0 = 0.0f, d1 = 0.0f, logsc = 0.0f;
-  float mx[K];                                   // this lane's row maxima of the last batch, logs not yet taken
-#pragma unroll
-  for (int k = 0; k < K; ++k) mx[k] = 1.0f;
+  if (S.is_long[j]) return;
+  const float sc = bias_score<G, ONE>(B, sh, reinterpret_cast<const uint4 *>(db.codes + db.start[s]), L, glane, gmask);
+  if (glane == 0) out[j] = sc;
+}
 
-  bias_rows<G, ONE, true, false>(B, s_eo, sq[0], L, glane, t00, t01, d0, d1, mx);
-  int i0 = 16;
-  for (; i0 + 16 <= L; i0 += 16) {               // the previous batch (rows i0-16 .. i0-1) is full
-    float nm[K], lg[K];
-    const uint32_t fail = bias_logs(mx, lg);
-    bias_rows<G, ONE, false, true>(B, s_eo, sq[i0 >> 4], 16, glane, t00, t01, d0, d1, nm);
-    bias_add<G>(mx, lg, fail, 16, s_log, gmask, logsc);
+// One warp per long sequence: are its segments the sequence's own rows? Then
+// the sum of the row logs in row order, by every lane alike; else its score
+// from the start.
+template <bool ONE>
+__global__ void __launch_bounds__(128)
+bias_join_kernel(BiasDev B, DbDev db, const int64_t *__restrict__ slots, BiasSegs S, float *__restrict__ out) {
+  __shared__ BiasShared sh;
+  const int lane = threadIdx.x & 31;
+  if (blockIdx.x * (blockDim.x / 32) >= S.n[0]) return;
+  sh.load(B);
+  const unsigned e = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+  if (e >= S.n[0]) return;
+  const int j = S.seq[e];
+  const int64_t s = slots[j];
+  const int L = db.len[s], nseg = (L + kBiasSeg - 1) / kBiasSeg;
+  const float4 *st = S.state + S.first[e];
+  bool same = true;
+  for (int k = lane + 1; k < nseg; k += 32)
+    same = same && __float_as_uint(st[k].x) == __float_as_uint(st[k - 1].z) &&
+           __float_as_uint(st[k].y) == __float_as_uint(st[k - 1].w);
+  float sc;
+  if (__all_sync(FULL, same)) {
+    const float4 *lg = reinterpret_cast<const float4 *>(S.lg + (size_t) S.row[e] * kBiasSeg);
+    float logsc = 0.0f;
+    int r = 0;
+    constexpr int U = 16;                        // 64 rows' loads ahead of their adds
+    float4 v[U], nx[U];
 #pragma unroll
-    for (int k = 0; k < K; ++k) mx[k] = nm[k];
+    for (int u = 0; u < U; ++u) nx[u] = lg[u];   // a long sequence has more rows than these
+    for (; r + 4 * U <= L; r += 4 * U) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = nx[u];
+      if (r + 8 * U <= L) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) nx[u] = lg[(r >> 2) + U + u];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        logsc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(logsc, v[u].x), v[u].y), v[u].z), v[u].w);
+    }
+    for (; r < L; ++r) logsc = __fadd_rn(logsc, reinterpret_cast<const float *>(lg)[r]);
+    sc = __fadd_rn(logsc, log_rowf(__fadd_rn(st[nseg - 1].z, st[nseg - 1].w), sh.logtab));
+  } else {
+    sc = bias_score<16, ONE>(B, sh, reinterpret_cast<const uint4 *>(db.codes + db.start[s]), L, lane % 16,
+                             lane < 16 ? 0xffffu : 0xffff0000u);
   }
-  float lg[K];
-  if (i0 < L) {
-    float nm[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) nm[k] = 1.0f;
-    const uint32_t fail = bias_logs(mx, lg);
-    bias_rows<G, ONE, false, false>(B, s_eo, sq[i0 >> 4], L - i0, glane, t00, t01, d0, d1, nm);
-    bias_add<G>(mx, lg, fail, 16, s_log, gmask, logsc);
-#pragma unroll
-    for (int k = 0; k < K; ++k) mx[k] = nm[k];
-  }
-  const uint32_t fail = bias_logs(mx, lg);
-  bias_add<G>(mx, lg, fail, (L - 1) % 16 + 1, s_log, gmask, logsc);
-  const float end = __fadd_rn(d0, d1);           // dp[L][0] * 1 + dp[L][1] * 1
-  if (glane == 0) out[j] = __fadd_rn(logsc, log_rowf(end, s_log));
+  if (lane == 0) out[j] = sc;
 }
 
 // degenerate amino codes 21..26 (B J Z O U X) as sets of canonical codes
@@ -350,12 +525,19 @@ bool one_division(const BiasDev &B) {
 constexpr int kBiasLanes = 8;
 
 cudaError_t launch_bias(const BiasDev &B, const DbDev &db, const int64_t *ids, const int64_t *order, int64_t n,
-                        float *out, int32_t *len, cudaStream_t stream) {
+                        const BiasSegs &S, float *out, int32_t *len, cudaStream_t stream) {
   constexpr int G = kBiasLanes;
-  const unsigned grid = (unsigned) ((n * G + 127) / 128);
+  const unsigned grid = (unsigned) (((n + S.cap_item) * G + 127) / 128);
+  const bool one = one_division(B);
   (void) cudaGetLastError();
-  if (one_division(B)) bias_kernel<G, true><<<grid, 128, 0, stream>>>(B, db, ids, order, n, out, len);
-  else bias_kernel<G, false><<<grid, 128, 0, stream>>>(B, db, ids, order, n, out, len);
+  if (S.cap_row) bias_plan_kernel<<<(unsigned) ((n + 255) / 256), 256, 0, stream>>>(db, ids, n, S);
+  if (one) bias_kernel<G, true><<<grid, 128, 0, stream>>>(B, db, ids, order, n, S, out, len);
+  else bias_kernel<G, false><<<grid, 128, 0, stream>>>(B, db, ids, order, n, S, out, len);
+  if (S.cap_row) {
+    const unsigned joins = (S.cap_seq + 3) / 4;
+    if (one) bias_join_kernel<true><<<joins, 128, 0, stream>>>(B, db, ids, S, out);
+    else bias_join_kernel<false><<<joins, 128, 0, stream>>>(B, db, ids, S, out);
+  }
   return cudaGetLastError();
 }
 
@@ -423,7 +605,26 @@ extern "C" int msvgb_biasfilter(msvgb_ctx *c, const float *compo, int M, const m
   char *d_scr = nullptr;
   cudaMemPool_t pool = msvgb_detail::scratch_pool(c->device);   // stays mapped between calls
   if (!pool) return fail(MSVGB_eslESYS, "biasfilter: no memory pool");
-  CUDA_TRY(cudaMallocFromPoolAsync((void **) &d_scr, 2 * a8 + 4096 + 2 * a4, pool, c->stream));
+  // room for the long sequences: at most 4M rows of them at a time, and no more than the list can hold
+  BiasSegs S{};
+  const int64_t most = db->Lmax > kBiasLong ? nids * ((db->Lmax + kBiasSeg - 1) / kBiasSeg) : 0;
+  S.cap_row = (unsigned) std::min<int64_t>(most, (4 << 20) / kBiasSeg);
+  S.cap_item = S.cap_row;
+  S.cap_seq = (unsigned) std::min<int64_t>(nids, S.cap_row / 3);   // a long one has four segments or more
+  size_t end = 2 * a8 + 4096 + 2 * a4;
+  auto take = [&](size_t bytes) { const size_t at = end; end += (bytes + 255) & ~(size_t) 255; return at; };
+  const size_t o_long = take((size_t) nids), o_n = take(12), o_item = take((size_t) S.cap_item * 8),
+               o_state = take((size_t) S.cap_item * 16), o_lg = take((size_t) S.cap_row * kBiasSeg * 4),
+               o_seq = take((size_t) S.cap_seq * 12);
+  CUDA_TRY(cudaMallocFromPoolAsync((void **) &d_scr, end, pool, c->stream));
+  S.is_long = (uint8_t *) d_scr + o_long;
+  S.n = (unsigned *) (d_scr + o_n);
+  S.item = (uint2 *) (d_scr + o_item);
+  S.state = (float4 *) (d_scr + o_state);
+  S.lg = (float *) (d_scr + o_lg);
+  S.seq = (int32_t *) (d_scr + o_seq);
+  S.first = (unsigned *) S.seq + S.cap_seq;
+  S.row = S.first + S.cap_seq;
   int64_t *d_ids = (int64_t *) d_scr, *d_order = (int64_t *) (d_scr + a8);
   int32_t *d_cnt = (int32_t *) (d_scr + 2 * a8);
   float *d_out = (float *) (d_scr + 2 * a8 + 4096);
@@ -437,9 +638,8 @@ extern "C" int msvgb_biasfilter(msvgb_ctx *c, const float *compo, int M, const m
   if (e == cudaSuccess)
     e = msvgb_detail::launch_order_by_length(d_ids, nids, db->d_len, db->Lmax, d_cnt, d_order, c->num_sms, c->stream);
   DbDev dbv{db->d_codes, db->d_start, db->d_len, db->d_orig, db->n};
-  if (e == cudaSuccess) {
-    e = launch_bias(B, dbv, d_ids, d_order, nids, d_out, d_len, c->stream);
-  }
+  if (e == cudaSuccess) e = cudaMemsetAsync(d_scr + o_long, 0, o_n + 12 - o_long, c->stream);   // is_long, n
+  if (e == cudaSuccess) e = launch_bias(B, dbv, d_ids, d_order, nids, S, d_out, d_len, c->stream);
   if (e == cudaSuccess) msvgb_detail::count_launch();
   const float *sc = (const float *) (pin + a8);                  // scores, then lengths, in one copy
   const int32_t *lens = (const int32_t *) (pin + a8 + a4);
