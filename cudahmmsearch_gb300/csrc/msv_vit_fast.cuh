@@ -31,7 +31,8 @@
 // One warp scores a sequence up to 1024 nodes; above, the 4 or 8 warps of a
 // block share it: one warp with its row in registers and the transitions in
 // shared memory took 5.46 ms for a call on 3,000 listed sequences at M = 2400
-// (4.1 without its host work), four warps take 2.27.
+// (4.1 without its host work), four warps take 2.19 (2.27 with the closure's
+// chains only in the rows that ask for them).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -148,19 +149,24 @@ __device__ __forceinline__ void vitf_chains(const uint32_t (&dd)[W], int lane, V
   c.pre = bs - own;
 }
 
-// The closure: both halves of a lane as two chains of W nodes (vitf_chain),
-// then a warp scan over the lanes' ends. A value loses at least -bmax[s] over
-// any 2^s lanes, so the scan stops where even the row's largest D, dm, would
-// end at the floor: usually before its first step. end: the value leaving
-// each lane, from within the warp.
+// The closure: both halves of a lane as two chains of W nodes; end: the value
+// leaving the lane, from within it. Where the warps of a block share a
+// sequence the chains run in every row, beside the maxima's reductions, whose
+// exchange the row waits for anyway (a D closed where the bound does not ask
+// for it changes nothing); a warp on its own runs them only where asked.
 template <int W>
-__device__ __forceinline__ int vitf_chain(uint32_t (&Dv)[W], const uint32_t (&dd)[W], int lane, const VitChains &ch,
-                                          int F, int dm, int &clo) {
+__device__ __forceinline__ int vitf_chain(uint32_t (&Dv)[W], const uint32_t (&dd)[W], const VitChains &ch, int &clo) {
   uint32_t c = Dv[0];
 #pragma unroll
   for (int w = 1; w < W; ++w) { c = __viaddmax_s16x2(c, dd[w], Dv[w]); Dv[w] = c; }
   clo = (int) (int16_t) (c & 0xffffu);
-  int end = max((int) c >> 16, clo + ch.bh);
+  return max((int) c >> 16, clo + ch.bh);
+}
+
+// A warp scan of the lanes' ends, for rows whose largest D, dm, lives through
+// a lane's chains: a value loses at least -bmax[s] over any 2^s lanes, and the
+// scan stops where even dm would end at the floor.
+__device__ __forceinline__ int vitf_scan(int end, int lane, const VitChains &ch, int F, int dm) {
 #pragma unroll
   for (int s = 0; s < 5; ++s) {
     if (dm + ch.bmax[s] <= F) break;
@@ -279,15 +285,22 @@ vit_fast_kernel(VitFastDev V, DbDev db, const int64_t *__restrict__ slots, const
           for (int k = 0; k < NW; ++k) { xe = max(xe, sh.xe[k]); dm = max(dm, sh.dm[k]); }
         }
         Dv[0] = __byte_perm(sdc, dc, 0x5432);
+        int clo = 0, end = 0, vin = F, into = F;
+        if constexpr (NW > 1) {
+          end = vitf_chain<W>(Dv, T[7], ch, clo);
+          vin = __shfl_up_sync(FULL, end, 1);
+        }
         top = max(top, xe);
         xC = (int16_t) max(xC + V.xwC_loop, xe + V.xwE_move);
         xJ = max(xJ, xe + V.xwE_loop);
         xB = max(xJ, xN) + move;
         if (dm + V.ddbound_w > xB || xe >= 32767) {
           if (xe >= 32767) { xC = 32767; st = 1; break; }   // eslERANGE
-          int clo;
-          const int end = vitf_chain<W>(Dv, T[7], lane, ch, F, dm, clo);
-          int vin = __shfl_up_sync(FULL, end, 1), into = F;
+          if constexpr (NW == 1) end = vitf_chain<W>(Dv, T[7], ch, clo);
+          if (NW == 1 || dm + ch.bmax[0] > F) {
+            end = vitf_scan(end, lane, ch, F, dm);
+            vin = __shfl_up_sync(FULL, end, 1);
+          }
           if constexpr (NW > 1) {                     // the earlier warps' ends, carried through the warps between
             if (lane == 31) sh.end[warp] = end;
             __syncthreads();
