@@ -206,7 +206,7 @@ int msvgb_detail::batch_create(msvgb_ctx *ctx, const msvgb_om *const *oms, int n
       const int k = G == 32 ? 0 : G == 16 ? 1 : 2;
       if (vidx[k] < 0) {
         ProfDev V = P;
-        if (G < 32) {
+        if (G < 32 || (!force_lanes && C >= kWideC)) {
           V.G = G; V.Cg = group_C(M, G); V.CI = multi_hyb_words(V.Cg, G);
           const std::vector<uint32_t> gt = V.CI ? msvgb_detail::build_hyb_table(oms[i], V.Cg, G, V.CI)
                                                 : msvgb_detail::build_group_table(oms[i], V.Cg, G);
@@ -259,7 +259,7 @@ int msvgb_detail::batch_create(msvgb_ctx *ctx, const msvgb_om *const *oms, int n
     const int pi = order[oi];
     for (const Range &r : ranges) {
       const int v = var_of[pi][r.bin];
-      const int64_t max_seqs = vars[v].G < 32 ? kChunkMaxSeqs : INT64_MAX;
+      const int64_t max_seqs = vars[v].Cg ? kChunkMaxSeqs : INT64_MAX;
       for (int64_t s = r.a; s < r.b;) {
         int64_t e2 = s;
         double acc = 0;

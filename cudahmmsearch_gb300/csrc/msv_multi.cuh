@@ -2,8 +2,9 @@
 // profiles from one launch (batched search, serving loop). A CTA takes a work
 // item (one profile, a chunk of the sorted database) and scores it either with
 // one warp per sequence (SSV and full MSV fused) or, for the profiles the
-// lane choice puts on 16 or 8 lanes, with the lane-group SSV pass followed by
-// the full MSV on the sequences it left undecided. The DP widths are runtime
+// lane choice puts on 16 or 8 lanes and for a batch's of 1024 nodes or more,
+// with the lane-group SSV pass followed by the full MSV on the sequences it
+// left undecided. The DP widths are runtime
 // values dispatched to compile-time instantiations.
 #pragma once
 #include "msv_device.cuh"
@@ -12,9 +13,16 @@
 namespace msvgb {
 
 // DP widths available to the multi-profile kernels; a profile whose tight
-// width is not listed runs at the next larger one (extra nodes are padding).
-constexpr int kMultiC[] = {1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 14, 16, 20, 24, 28, 32};
+// width is not listed runs at the next larger one (extra nodes are padding:
+// with steps of four words from 16 up the 48 profiles took 18.5 ms, 17.9 with
+// steps of two).
+constexpr int kMultiC[] = {1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 14, 16, 18, 20, 22, 24, 26, 28, 30, 32};
 constexpr int kMultiMaxC = 32;
+
+// From this width (1024 nodes) 32-lane profiles of a batch run the two passes
+// of the lane groups too, a warp being one group, for the mixed-width table
+// (48 profiles of 50 to 1500 nodes vs 20,000 sequences: 17.4 ms, fused 17.9).
+constexpr int kWideC = 18;
 
 inline int multi_C(int M) {
   const int need = M / 64 + 1;
@@ -64,7 +72,8 @@ __device__ __forceinline__ void run_seq_any(int C, const ProfDev &P, const uint3
     MSVGB_MULTI_CASE(1) MSVGB_MULTI_CASE(2) MSVGB_MULTI_CASE(3) MSVGB_MULTI_CASE(4)
     MSVGB_MULTI_CASE(5) MSVGB_MULTI_CASE(6) MSVGB_MULTI_CASE(7) MSVGB_MULTI_CASE(8)
     MSVGB_MULTI_CASE(10) MSVGB_MULTI_CASE(12) MSVGB_MULTI_CASE(14) MSVGB_MULTI_CASE(16)
-    MSVGB_MULTI_CASE(20) MSVGB_MULTI_CASE(24) MSVGB_MULTI_CASE(28) MSVGB_MULTI_CASE(32)
+    MSVGB_MULTI_CASE(18) MSVGB_MULTI_CASE(20) MSVGB_MULTI_CASE(22) MSVGB_MULTI_CASE(24)
+    MSVGB_MULTI_CASE(26) MSVGB_MULTI_CASE(28) MSVGB_MULTI_CASE(30) MSVGB_MULTI_CASE(32)
 #undef MSVGB_MULTI_CASE
     default: break;
   }
@@ -74,34 +83,33 @@ __device__ __forceinline__ void run_seq_any(int C, const ProfDev &P, const uint3
 // use at lane-group width Cg (0: f16 table): the single-query default
 // (hyb_default_words) at the group widths these kernels compile (kMultiC).
 __host__ __device__ constexpr int multi_hyb_words(int Cg, int G) {
-  return G < 32 ? hyb_words(Cg, G) : 0;
+  return G < 32 || Cg >= kWideC ? hyb_words(Cg, G) : 0;
 }
 
-// The lane-group SSV pass of one chunk at (G, Cg), with the f16 or the
-// mixed-width table as P.CI says (0, or multi_hyb_words(Cg, G)).
+// The lane-group SSV pass of one chunk at (G, Cg), with the table of
+// multi_hyb_words(Cg, G).
 __device__ __forceinline__ void ssv_group_chunk_any(int G, int Cg, const ProfDev &P, const uint32_t *tab,
                                                     const DbDev &db, int64_t s0, int nseq, uint8_t *oxj,
                                                     uint8_t *ofl, unsigned *next_seq, uint16_t *und,
                                                     unsigned *n_und) {
-#define MSVGB_GROUP_VARIANT(c, g)                                                                          \
-  if (G == g) {                                                                                            \
-    constexpr int ci = multi_hyb_words(c, g);                                                              \
-    bool done = false;                                                                                     \
-    if constexpr (ci > 0) {                                                                                \
-      if (P.CI == ci) { ssv_group_chunk<c, g, ci>(P, tab, db, s0, nseq, oxj, ofl, next_seq, und, n_und); done = true; } \
-    }                                                                                                      \
-    if (!done) ssv_group_chunk<c, g, 0>(P, tab, db, s0, nseq, oxj, ofl, next_seq, und, n_und);             \
-  }
-#define MSVGB_GROUP_CASE(c) case c: MSVGB_GROUP_VARIANT(c, 8) else MSVGB_GROUP_VARIANT(c, 16) break;
+#define MSVGB_GROUP_RUN(c, g)                                                                              \
+  ssv_group_chunk<c, g, multi_hyb_words(c, g)>(P, tab, db, s0, nseq, oxj, ofl, next_seq, und, n_und)
+#define MSVGB_GROUP_CASE(c)                                                                                \
+  case c:                                                                                                  \
+    if (G == 8) MSVGB_GROUP_RUN(c, 8);                                                                     \
+    else if (G == 16) MSVGB_GROUP_RUN(c, 16);                                                              \
+    else if constexpr (c >= kWideC) MSVGB_GROUP_RUN(c, 32);                                                \
+    break;
   switch (Cg) {
     MSVGB_GROUP_CASE(2) MSVGB_GROUP_CASE(3) MSVGB_GROUP_CASE(4) MSVGB_GROUP_CASE(5)
     MSVGB_GROUP_CASE(6) MSVGB_GROUP_CASE(7) MSVGB_GROUP_CASE(8) MSVGB_GROUP_CASE(10)
-    MSVGB_GROUP_CASE(12) MSVGB_GROUP_CASE(14) MSVGB_GROUP_CASE(16) MSVGB_GROUP_CASE(20)
-    MSVGB_GROUP_CASE(24) MSVGB_GROUP_CASE(28) MSVGB_GROUP_CASE(32)
+    MSVGB_GROUP_CASE(12) MSVGB_GROUP_CASE(14) MSVGB_GROUP_CASE(16) MSVGB_GROUP_CASE(18)
+    MSVGB_GROUP_CASE(20) MSVGB_GROUP_CASE(22) MSVGB_GROUP_CASE(24) MSVGB_GROUP_CASE(26)
+    MSVGB_GROUP_CASE(28) MSVGB_GROUP_CASE(30) MSVGB_GROUP_CASE(32)
     default: break;
   }
 #undef MSVGB_GROUP_CASE
-#undef MSVGB_GROUP_VARIANT
+#undef MSVGB_GROUP_RUN
 }
 
 // Shared state of one CTA's work item.
@@ -113,7 +121,7 @@ struct ChunkShared {
 // Words of a profile's SSV table in shared memory (the MSV table follows it):
 // the lane-group layout with its region copies (group_words), or the 32-lane one.
 __host__ __device__ inline int ssv_words(const ProfDev &P) {
-  return P.G < 32 ? group_words(P.Cg, P.G, P.CI) : NRES * P.C * 32;
+  return P.Cg ? group_words(P.Cg, P.G, P.CI) : NRES * P.C * 32;
 }
 
 // One CTA scores the sorted sequences [s0, s0 + nseq) against P, whose tables
@@ -123,7 +131,7 @@ __device__ __forceinline__ void run_chunk(const ProfDev &P, const uint32_t *stab
                                           const DbDev &db, int64_t s0, int64_t nseq, uint8_t *oxj, uint8_t *ofl,
                                           ChunkShared &cs) {
   const int lane = threadIdx.x & 31;
-  if (P.G == 32) {
+  if (P.Cg == 0) {
     for (;;) {
       unsigned k = 0;
       if (lane == 0) k = atomicAdd(&cs.next_seq, 1u);
