@@ -481,11 +481,11 @@ extern "C" int msvgb_profile_create(msvgb_ctx *ctx, const msvgb_om *om, msvgb_pr
   bool split = false;
   create_choice(ctx, om->M, &G, &split, &want_f16);
   int st = profile_build(ctx, om, want_f16, ret);
-  if (st == MSVGB_eslOK && split && (*ret)->f16) {
-    st = msvgb_profile_set_lanes(*ret, om, G);
+  if (st == MSVGB_eslOK) {
+    if (split && (*ret)->f16) st = msvgb_detail::profile_auto_lanes(*ret, om, G);
+    else (*ret)->lanes_auto = true;
     if (st != MSVGB_eslOK) { msvgb_profile_destroy(*ret); *ret = nullptr; }
   }
-  if (st == MSVGB_eslOK) st = msvgb_detail::profile_auto_lanes(*ret, om);
   return st;
 }
 
@@ -562,6 +562,11 @@ std::vector<uint32_t> msvgb_detail::build_group_msv_table(const msvgb_om *om, in
 
 static int set_group_tables(msvgb_profile *p, const msvgb_om *om, int G);
 
+// Whether a 32-lane profile also has the split passes.
+static bool wide_split(const msvgb_profile *p) {
+  return p->M >= kWideSplitMinM && p->M / 64 + 1 <= 32;
+}
+
 extern "C" int msvgb_profile_set_lanes(msvgb_profile *p, const msvgb_om *om, int G) {
   if (!p || !om) return fail(MSVGB_eslEINVAL, "NULL argument");
   if (om->M != p->M) return fail(MSVGB_eslEINVAL, "om does not match the profile");
@@ -570,8 +575,7 @@ extern "C" int msvgb_profile_set_lanes(msvgb_profile *p, const msvgb_om *om, int
   // 32 lanes: the fused kernel, and for models of 1024 to 2047 nodes also
   // the split passes (32-lane groups, mixed-width SSV table), which large
   // searches use
-  const bool wide = G == 32 && p->M >= kWideSplitMinM && p->M / 64 + 1 <= 32;
-  if (G == 32 && !wide) {
+  if (G == 32 && !wide_split(p)) {
     cudaFree(p->d_stab_g); cudaFree(p->d_mtab_g);
     p->d_stab_g = p->d_mtab_g = nullptr;
     p->G = p->Gk = 32; p->CI = 0;
@@ -582,9 +586,12 @@ extern "C" int msvgb_profile_set_lanes(msvgb_profile *p, const msvgb_om *om, int
   return st;
 }
 
-int msvgb_detail::profile_auto_lanes(msvgb_profile *p, const msvgb_om *om) {
+int msvgb_detail::profile_auto_lanes(msvgb_profile *p, const msvgb_om *om, int G) {
   p->lanes_auto = true;
-  return p->d_stab_g && p->G == 8 && p->M < kNarrowMaxM ? set_group_tables(p, om, 4) : MSVGB_eslOK;
+  if (G == 32 && !wide_split(p)) return MSVGB_eslOK;
+  const int st = set_group_tables(p, om, G == 8 && p->M < kNarrowMaxM ? 4 : G);
+  if (st == MSVGB_eslOK) p->G = G;
+  return st;
 }
 
 // The lane-group tables at G lanes per sequence.

@@ -126,9 +126,9 @@ extern "C" int msvgb_batch_destroy(msvgb_batch *b) {
   return MSVGB_eslOK;
 }
 
-// Profiles whose search alone fills the GPU (M x residues >= 40e9 cells, the
-// size at which a single query switches to lane groups) are scored by their
-// own single-query searches -- lane-group pass, then the full MSV of its
+// Profiles whose search alone fills the GPU (M x residues >= 40e9 cells; 48
+// profiles vs 20,000 sequences took 18.5 ms, and 18.8 with the line at 5e9,
+// 19.4 at 2e9) are scored by their own single-query searches -- lane-group pass, then the full MSV of its
 // undecided sequences -- on four graph branches taken in turn, so that one
 // search's tail overlaps the next one's start; so are profiles above 2047
 // nodes (up to the single-query maximum). The other profiles share the
@@ -180,10 +180,10 @@ int msvgb_detail::batch_create(msvgb_ctx *ctx, const msvgb_om *const *oms, int n
       msvgb_profile *p = nullptr;
       int st = msvgb_detail::profile_build_width(ctx, oms[i], 1, 0, &p);
       const int G = st == MSVGB_eslOK ? msvgb_detail::lanes_for(ctx, M, -1, nullptr) : 32;
-      if (st == MSVGB_eslOK && p->f16) st = msvgb_profile_set_lanes(p, oms[i], G);   // 32: split passes for M 1024-2047
       if (p) b->own.push_back(p);
       if (st != MSVGB_eslOK) { msvgb_batch_destroy(b); return st; }
-      if (st == MSVGB_eslOK) st = msvgb_detail::profile_auto_lanes(p, oms[i]);
+      if (p->f16) st = msvgb_detail::profile_auto_lanes(p, oms[i], G);   // 32: split passes for M 1024-2047
+      else p->lanes_auto = true;
       if (st != MSVGB_eslOK) { msvgb_batch_destroy(b); return st; }
       large.emplace_back(i, p);
       continue;

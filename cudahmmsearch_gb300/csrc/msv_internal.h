@@ -199,9 +199,9 @@ cudaError_t dispatch(int C, bool f16, const msvgb::LaunchArgs &a, int sms);
 struct F1Gate { float lo = -INFINITY, hi = INFINITY; };
 F1Gate f1_gate(float mmu, float mlambda, double F1);
 int xjmin_for(const msvgb_profile *p, int L, double F1, int hint = -1, const F1Gate &gate = F1Gate());
-// Marks a profile's lanes as its own choice (msvgb_profile_create): its large
-// searches may then run on 4 lanes per sequence.
-int profile_auto_lanes(msvgb_profile *p, const msvgb_om *om);
+// G lanes as a profile's own choice (msvgb_profile_create): its large searches
+// may then run on 4 lanes per sequence.
+int profile_auto_lanes(msvgb_profile *p, const msvgb_om *om, int G);
 // Device tables of a profile; force_C > 0 imposes the DP width.
 int profile_build_width(msvgb_ctx *ctx, const msvgb_om *om, int want_f16, int force_C, msvgb_profile **ret);
 // Host images of the device cost tables of a profile at DP width C.

@@ -606,10 +606,11 @@ struct VitFastPlan {
       if (t == 7) return v->twv[(7 * Q8 + (k - 2) % Q8) * 8 + (k - 2) / Q8];
       return v->twv[((k - 1) % Q8 * 7 + t) * 8 + (k - 1) / Q8];
     };
-    auto e_of = [&](int x, int k) -> int { return v->rwv[(x * Q8 + (k - 1) % Q8) * 8 + (k - 1) / Q8]; };
+    auto e_at = [&](int k) { return v->rwv + (k - 1) % Q8 * 8 + (k - 1) / Q8; };   // node k's emissions, one per 8 Q8
     for (int k = M + 1; k <= Np; ++k) {
       for (int t = 0; t < 4; ++t) if (t_of(t, k) != -32768) return;
-      for (int x = 0; x < 29; ++x) if (e_of(x, k) != -32768) return;
+      const int16_t *e = e_at(k);
+      for (int x = 0; x < 29; ++x) if (e[x * Q8 * 8] != -32768) return;
     }
     int bm_min = 0, bm_max = -32768, t_m = 0, t_id = 0, emax = 0, emin = 0;
     for (int k = 1; k <= M; ++k) {
@@ -624,14 +625,16 @@ struct VitFastPlan {
         t_id = std::min(t_id, t_of(6, k));
       }
     }
-    int e_low[NRES];
+    int e_low[NRES] = {};
     uint32_t low_res = 1u << 29;                    // 29, 30: never scored
-    for (int x = 0; x < 29; ++x) {
-      e_low[x] = 0;
-      for (int k = 1; k <= M; ++k) {
-        e_low[x] = std::min(e_low[x], e_of(x, k));
-        emax = std::max(emax, e_of(x, k));
+    for (int k = 1; k <= M; ++k) {
+      const int16_t *e = e_at(k);
+      for (int x = 0; x < 29; ++x) {
+        e_low[x] = std::min<int>(e_low[x], e[x * Q8 * 8]);
+        emax = std::max<int>(emax, e[x * Q8 * 8]);
       }
+    }
+    for (int x = 0; x < 29; ++x) {
       if (e_low[x] < kLowEmission) low_res |= 1u << x;
       else emin = std::min(emin, e_low[x]);
     }
@@ -654,9 +657,8 @@ struct VitFastPlan {
       for (int i = 0; i < w; ++i)
         for (int h = 0; h < 2; ++h) {
           const int k = lane * 2 * w + h * w + i + 1;
-          auto put = [&](int row, int val) {
-            tab[(size_t) row * w * N + vitf_at(w, N, lane, i)] |= (uint32_t) (uint16_t) val << (16 * h);
-          };
+          uint32_t *cell = tab.data() + vitf_at(w, N, lane, i);
+          auto put = [&](int row, int val) { cell[(size_t) row * w * N] |= (uint32_t) (uint16_t) val << (16 * h); };
           for (int t = 0; t < kFT; ++t) {
             const bool in = t < 4 || t == 7;        // into node k, else out of it
             int c;
@@ -666,7 +668,8 @@ struct VitFastPlan {
             else c = t_of(t, k);
             put(t, c);
           }
-          for (int x = 0; x < NRES; ++x) put(kFT + x, k > M || x == 29 ? e_low[x] : e_of(x, k));
+          const int16_t *e = e_at(std::min(k, M));
+          for (int x = 0; x < NRES; ++x) put(kFT + x, k > M || x == 29 ? e_low[x] : e[x * Q8 * 8]);
         }
     form = f;
   }
@@ -710,13 +713,13 @@ struct msvgb_vprofile {
   float scale_w = 0.f, nj = 0.f;
   int16_t base_w = 0, ddbound_w = 0;
   int16_t xw[4][2] = {};
-  void *d_trans = nullptr;
-  uint4 *d_emit = nullptr;
+  void *d_tabs = nullptr;                    // every table, in one block
+  const void *d_trans = nullptr;             // in d_tabs
+  const uint4 *d_emit = nullptr;
   int16_t *d_move = nullptr;
   VitForm fast_form{0, 0};                   // the packed kernel's form (W = 0: not used)
   int fast_move_min = 0;                     // and lowest move cost
   VitFastDev fast{};
-  uint32_t *d_fast = nullptr;
   int move_cap = 0;
   std::vector<int16_t> h_move;
   std::mutex move_mu;                        // the move table grows under concurrent calls
@@ -835,21 +838,28 @@ extern "C" int msvgb_vprofile_create(msvgb_ctx *ctx, const msvgb_vom *v, msvgb_v
   VitFastPlan plan;
   plan.build(v, Q8);
   cudaError_t e = cudaSetDevice(ctx->device);
-  if (e == cudaSuccess && plan.form.W) {
-    e = cudaMalloc(&p->d_fast, plan.tab.size() * 4);
-    if (e == cudaSuccess) e = cudaMemcpy(p->d_fast, plan.tab.data(), plan.tab.size() * 4, cudaMemcpyHostToDevice);
-    p->fast_form = plan.form; p->fast_move_min = plan.move_min;
-    p->fast = plan.V;
-    p->fast.trans = p->d_fast; p->fast.emit = p->d_fast + (size_t) kFT * plan.form.W * 32 * plan.form.NW;
-  }
-  if (e == cudaSuccess) e = cudaMalloc(&p->d_trans, tbytes);
-  if (e == cudaSuccess) e = cudaMalloc(&p->d_emit, ebytes);
-  if (e == cudaSuccess) e = cudaMemcpy(p->d_trans, tsrc, tbytes, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(p->d_emit, esrc, ebytes, cudaMemcpyHostToDevice);
+  // one block and one copy: the packed kernel's tables, then the general kernels'
+  const size_t fbytes = (plan.tab.size() * 4 + 255) / 256 * 256, tpad = (tbytes + 255) / 256 * 256;
+  std::vector<char> up(fbytes + tpad + ebytes);
+  if (plan.form.W) memcpy(up.data(), plan.tab.data(), plan.tab.size() * 4);
+  memcpy(up.data() + fbytes, tsrc, tbytes);
+  memcpy(up.data() + fbytes + tpad, esrc, ebytes);
+  char *d = nullptr;
+  if (e == cudaSuccess) e = cudaMalloc(&d, up.size());
+  p->d_tabs = d;
+  if (e == cudaSuccess) e = cudaMemcpy(d, up.data(), up.size(), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     msvgb_vprofile_destroy(p);
     return fail(MSVGB_eslESYS, std::string("vprofile upload: ") + cudaGetErrorString(e));
   }
+  if (plan.form.W) {
+    const uint32_t *fast = (const uint32_t *) d;
+    p->fast_form = plan.form; p->fast_move_min = plan.move_min;
+    p->fast = plan.V;
+    p->fast.trans = fast; p->fast.emit = fast + (size_t) kFT * plan.form.W * 32 * plan.form.NW;
+  }
+  p->d_trans = d + fbytes;
+  p->d_emit = (const uint4 *) (d + fbytes + tpad);
   *ret = p;
   return MSVGB_eslOK;
 }
@@ -857,7 +867,7 @@ extern "C" int msvgb_vprofile_create(msvgb_ctx *ctx, const msvgb_vom *v, msvgb_v
 extern "C" int msvgb_vprofile_destroy(msvgb_vprofile *p) {
   if (!p) return MSVGB_eslOK;
   cudaSetDevice(p->device);
-  cudaFree(p->d_trans); cudaFree(p->d_emit); cudaFree(p->d_move); cudaFree(p->d_fast);
+  cudaFree(p->d_tabs); cudaFree(p->d_move);
   for (int16_t *t : p->retired) cudaFree(t);
   delete p;
   return MSVGB_eslOK;
