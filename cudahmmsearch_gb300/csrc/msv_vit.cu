@@ -602,10 +602,15 @@ struct VitFastPlan {
     for (VitForm c : kVitForms) if (64 * c.W * c.NW >= M) { f = c; break; }
     const int w = f.W, N = 32 * f.NW;
     if (!w || v->xw[1][1] != 0 || v->xw[2][1] != 0 || v->xw[0][1] > 0) return;
-    auto t_of = [&](int t, int k) -> int {          // t < 7: costs of node k; 7: D(k-1) -> D(k)
-      if (t == 7) return v->twv[(7 * Q8 + (k - 2) % Q8) * 8 + (k - 2) / Q8];
-      return v->twv[((k - 1) % Q8 * 7 + t) * 8 + (k - 1) / Q8];
-    };
+    // node k's costs (8 apart), and D(k-1) -> D(k)
+    std::vector<const int16_t *> tw(Np + 1);
+    std::vector<int16_t> dd(Np + 1);
+    for (int k = 1, z = 0; k <= Np; ++z)
+      for (int q = 0; q < Q8; ++q, ++k) {
+        tw[k] = v->twv + q * 7 * 8 + z;
+        if (k < Np) dd[k + 1] = v->twv[(7 * Q8 + q) * 8 + z];
+      }
+    auto t_of = [&](int t, int k) -> int { return t == 7 ? dd[k] : tw[k][t * 8]; };
     auto e_at = [&](int k) { return v->rwv + (k - 1) % Q8 * 8 + (k - 1) / Q8; };   // node k's emissions, one per 8 Q8
     for (int k = M + 1; k <= Np; ++k) {
       for (int t = 0; t < 4; ++t) if (t_of(t, k) != -32768) return;
