@@ -104,7 +104,9 @@ __device__ __forceinline__ uint32_t add_f16x2(uint32_t a, uint32_t b) {
 // 16 lanes: C = 20: 16.6 / 18.1 / 19.1a; 24: 16.9 / 16.9 / 19.6; 32: 17.5 / 17.5 /
 // 19.6 / 20.4a; 32 lanes: C = 17: - / 18.4 / 18.6a; 24: - / 18.6 / 20.1; 32: - /
 // 19.1 / 20.3 / 20.9a. With every 8-bit word on the FMA pipe C = 26 took 16.3 ms
-// for 2,000,000 sequences, 15.8 with none.
+// for 2,000,000 sequences, 15.8 with none. At C = 26 and 8 words the pass reads
+// shared memory in 97.7% of cycles, but more 8-bit words still lose below 28
+// (12: 18.3a, 16: 18.5 with 8 on the FMA pipe, 8: 19.5): the ALU pipe takes over.
 __host__ __device__ constexpr int hyb_words(int C, int G) {
   if (G == 32) return C < 17 ? 0 : 8;
   if (C < (G == 16 ? 13 : 10)) return 0;

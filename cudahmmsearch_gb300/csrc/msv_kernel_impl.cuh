@@ -50,8 +50,10 @@ template <int C, bool F16>
 __host__ __device__ constexpr int row_words() { return F16 && C <= 8 ? 2 : 1; }
 
 // Persistent kernel: every CTA stages the profile's cost tables into shared
-// memory once, then its warps pull sequences (longest first) from a global
-// ticket until the database is exhausted.
+// memory once, then its warps pull sequences or segments of long ones (longest
+// first) from a global ticket until the database is exhausted. Bound by
+// shared memory where the database fills the SMs (2 bytes of cost per cell),
+// by the longest chain of rows where it does not (SegDev).
 template <int C, bool F16>
 __global__ void __launch_bounds__(cta_threads<C, F16>())
 msv_search_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t *__restrict__ out_flags,
