@@ -25,8 +25,10 @@
 // changes no match cell, because the host checks that the bound covers every
 // D->D->M step.
 //
-// Bound: the fused add-maximum runs at half rate (64 lanes per clock and SM);
-// six per word of two nodes. The transition costs stay in registers across
+// Bound: the ALU pipe (79% busy at M = 260, 40,000 listed sequences), on which
+// the fused add-maximum and the packed add run at half rate (64 lanes per clock
+// and SM): nine such operations per word of two nodes, a third of a row's
+// instructions at 5 words per lane. The transition costs stay in registers across
 // rows (up to 16 words per lane); a row reads only its residue's emissions.
 // One warp scores a sequence up to 1024 nodes; above, the 4 or 8 warps of a
 // block share it: one warp with its row in registers and the transitions in
