@@ -103,6 +103,7 @@ msv_search_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t *__
                                    (int64_t) s, r0);
       if (k >= 0) {                                   // the sequence's last segment to finish decides it
         if (lane == 0) umax = seg_finish(segs, (int64_t) s, L);
+        __syncwarp();                                 // the other lanes read u[] too (msv_full): behind lane 0's fence
         umax = __shfl_sync(FULL, umax, 0);
         if (umax < 0) continue;
       }
