@@ -305,6 +305,7 @@ extern "C" int msvgb_ctx_destroy(msvgb_ctx *c) {
   if (c->own) cudaStreamSynchronize(c->own);
   cudaFree(c->d_ticket);
   cudaFree(c->d_one); cudaFree(c->d_bad); cudaFree(c->d_list); cudaFree(c->d_seg);
+  for (uint8_t *d : c->seg_old) cudaFree(d);
   if (c->own) cudaStreamDestroy(c->own);
   if (c->side) { cudaStreamSynchronize(c->side); cudaStreamDestroy(c->side); }
   if (c->upload) { cudaStreamSynchronize(c->upload); cudaStreamDestroy(c->upload); }
@@ -1187,6 +1188,30 @@ static bool may_cut(const msvgb_profile *p) {
   return !p->d_stab_g || (p->lanes_auto && p->CI == msvgb_detail::hyb_default_words(p->Cg, p->Gk));
 }
 
+// The context's segment scratch, at least bytes of it (null: no room). A
+// search's need depends on its profile and its database, so a program that
+// takes them in turn would meet larger ones again and again: the buffer grows
+// by half as much again and at least twofold, without waiting for the stream,
+// and a smaller one is kept while the context lives, since searches in flight
+// and searches captured into a graph hold its address (twice the largest
+// buffer in all, at most). It does not grow while the stream is captured.
+static uint8_t *seg_scratch(msvgb_ctx *c, size_t bytes) {
+  if (c->seg_cap >= bytes) return c->d_seg;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(c->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return nullptr;
+  size_t cap = std::max({bytes + bytes / 2, 2 * c->seg_cap, (size_t) 1 << 20});
+  uint8_t *d = nullptr;
+  if (cudaMalloc(&d, cap) != cudaSuccess) {
+    cap = bytes;
+    if (cudaMalloc(&d, cap) != cudaSuccess) d = nullptr;
+    (void) cudaGetLastError();
+  }
+  if (!d) return nullptr;
+  if (c->d_seg) c->seg_old.push_back(c->d_seg);
+  c->d_seg = d; c->seg_cap = cap;
+  return d;
+}
+
 extern "C" int msvgb_search_device(msvgb_ctx *c, const msvgb_profile *pc, const msvgb_db *db, double F1,
                                    void *d_xj, void *d_flags) {
   if (!c || !pc || !db || (!d_xj && db->n) || (!d_flags && db->n)) return fail(MSVGB_eslEINVAL, "NULL argument");
@@ -1207,14 +1232,10 @@ extern "C" int msvgb_search_device(msvgb_ctx *c, const msvgb_profile *pc, const 
   SearchScratch sc;
   sc.cut = may_cut(p);
   if (sc.cut) sc.segs = plan_segments(p, db, c->num_sms);
-  const size_t need = seg_bytes(sc.segs);
-  if (c->seg_cap < need) {
-    CUDA_TRY(cudaStreamSynchronize(c->stream));            // as the list
-    cudaFree(c->d_seg); c->d_seg = nullptr; c->seg_cap = 0;
-    CUDA_TRY(cudaMalloc(&c->d_seg, need));
-    c->seg_cap = need;
+  if (const size_t need = seg_bytes(sc.segs)) {
+    sc.seg = seg_scratch(c, need);
+    if (!sc.seg) { sc.cut = false; sc.segs = SegDev(); }   // no room for it: uncut
   }
-  sc.seg = c->d_seg;
   sc.stream = c->stream; sc.side = c->side; sc.ev_fork = c->ev_fork; sc.ev_join = c->ev_join;
   sc.counters = c->d_ticket; sc.list = c->d_list;
   return enqueue_search(sc, p, db, t, (uint8_t *) d_xj, (uint8_t *) d_flags, c->num_sms);
@@ -1393,9 +1414,12 @@ static int search_chunked(msvgb_ctx *c, const msvgb_profile *p, msvgb_db *db, co
     sc.cut = may_cut(p);
     if (sc.cut) sc.segs = plan_segments(p, db, sms);
     const size_t need = seg_bytes(sc.segs);
-    if (need) CUDA_TRY(cudaMallocFromPoolAsync((void **) &sc.seg, need, scratch_pool(c->device), S[0]));
+    if (need && cudaMallocFromPoolAsync((void **) &sc.seg, need, scratch_pool(c->device), S[0]) != cudaSuccess) {
+      (void) cudaGetLastError();                            // no room for it: uncut
+      sc.cut = false; sc.segs = SegDev(); sc.seg = nullptr;
+    }
     st = enqueue_search(sc, p, db, t, d_xj, d_flags, sms);
-    if (need) cudaFreeAsync(sc.seg, S[0]);
+    if (sc.seg) cudaFreeAsync(sc.seg, S[0]);
     gt.mark("passed", S[0]);
     return st;
   }

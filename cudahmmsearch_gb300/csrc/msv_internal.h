@@ -48,6 +48,7 @@ struct msvgb_ctx {
   int *d_bad = nullptr;                                 // database packing: invalid-code flag
   int64_t *d_list = nullptr; size_t list_cap = 0;       // G-lane search: sequences left for the full MSV
   uint8_t *d_seg = nullptr; size_t seg_cap = 0;         // segment maxima and counts of the long targets
+  std::vector<uint8_t *> seg_old;                       // smaller ones (enqueued and captured searches hold them)
   cudaStream_t side = nullptr;                          // long targets of the lane-group search
   cudaStream_t upload = nullptr;                        // chunk uploads of msvgb_search_host
   cudaStream_t dma = nullptr;                           // raw residue copies of database creation
