@@ -1230,8 +1230,7 @@ extern "C" int msvgb_search_device(msvgb_ctx *c, const msvgb_profile *pc, const 
     c->list_cap = db->n;
   }
   SearchScratch sc;
-  sc.cut = may_cut(p);
-  if (sc.cut) sc.segs = plan_segments(p, db, c->num_sms);
+  sc.cut = may_cut(p) && plan_segments(p, db, c->num_sms, false, &sc.segs);
   if (const size_t need = seg_bytes(sc.segs)) {
     sc.seg = seg_scratch(c, need);
     if (!sc.seg) { sc.cut = false; sc.segs = SegDev(); }   // no room for it: uncut
@@ -1262,24 +1261,27 @@ static bool search_fused(const msvgb_profile *p, const msvgb_db *db, bool others
 // that the full MSV may skip: 128 in the fused kernel (M = 200, 20,000
 // targets: 207 us; 256 212 to 238, 512 265, 1024 364), 256 in the lane-group
 // pass, whose list kernel reads them (M = 86, 500,000 targets: 1272 us; 128
-// 1325, 512 1430).
-SegDev msvgb_detail::plan_segments(const msvgb_profile *p, const msvgb_db *db, int num_sms, bool others) {
+// 1325, 512 1430). False: the block maxima of its long targets, targets times
+// blocks of the longest, pass a GiB (131,000 long targets and one of two million
+// rows): the search then runs uncut, the longest at 32 lanes.
+bool msvgb_detail::plan_segments(const msvgb_profile *p, const msvgb_db *db, int num_sms, bool others, SegDev *ret) {
   SegDev g;
+  *ret = g;
   const int M = p->M;
   const bool fused = search_fused(p, db, others);
   const double chains = (double) num_sms * (fused ? (p->C > 32 ? 16.0 : 32.0) : 24.0 * 32.0 / p->Gk);
   const double avg = (double) db->residues / chains;
-  if (db->Lmax < avg / 2) return SegDev();                // no chain sets the search's length
+  if (db->Lmax < avg / 2) return true;                    // no chain sets the search's length
   const double T = std::max({avg, 2.0 * M, 768.0, (double) db->Lmax / kMaxSegs});
-  if (T > 1e8) return SegDev();
+  if (T > 1e8) return false;
   g.R = fused ? 128 : 256;
   g.T = ((int) T + g.R - 1) / g.R * g.R;
   g.warm = (M + 15) / 16 * 16;
   const int cut = 2 * std::max(M, g.R);                   // shorter targets stay whole
-  if (db->Lmax < cut) return SegDev();
+  if (db->Lmax < cut) return true;
   g.S = (db->Lmax + g.T - 1) / g.T;
   g.NB = (db->Lmax + g.R - 1) / g.R;
-  if (g.S > kMaxSegs) return SegDev();
+  if (g.S > kMaxSegs) return false;
   // sequences with more than k * T rows, longest first
   int64_t longer[kMaxSegs] = {}, c = 0;
   size_t i = db->distinct_len.size();
@@ -1294,9 +1296,10 @@ SegDev msvgb_detail::plan_segments(const msvgb_profile *p, const msvgb_db *db, i
     g.base[k] = (uint32_t) total;
     total += longer[k];
   }
-  if (total > (int64_t) 1 << 30 || g.nl * g.NB > (int64_t) 1 << 30) return SegDev();
+  if (total > (int64_t) 1 << 30 || g.nl * g.NB > (int64_t) 1 << 30) return false;
   for (int k = g.S; k <= kMaxSegs; ++k) g.base[k] = (uint32_t) total;
-  return g;
+  *ret = g;
+  return true;
 }
 
 size_t msvgb_detail::seg_bytes(const SegDev &g) { return (size_t) g.nl * (4 + g.NB); }
@@ -1411,8 +1414,7 @@ static int search_chunked(msvgb_ctx *c, const msvgb_profile *p, msvgb_db *db, co
     SearchScratch sc;
     sc.stream = S[0]; sc.side = c->side; sc.ev_fork = c->ev_fork; sc.ev_join = c->ev_join;
     sc.counters = ctr; sc.list = list;
-    sc.cut = may_cut(p);
-    if (sc.cut) sc.segs = plan_segments(p, db, sms);
+    sc.cut = may_cut(p) && plan_segments(p, db, sms, false, &sc.segs);
     const size_t need = seg_bytes(sc.segs);
     if (need && cudaMallocFromPoolAsync((void **) &sc.seg, need, scratch_pool(c->device), S[0]) != cudaSuccess) {
       (void) cudaGetLastError();                            // no room for it: uncut

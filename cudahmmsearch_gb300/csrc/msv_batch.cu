@@ -275,13 +275,20 @@ int msvgb_detail::batch_create(msvgb_ctx *ctx, const msvgb_om *const *oms, int n
   if (e == cudaSuccess) e = cudaMalloc(&b->d_ticket, sizeof(unsigned long long));
   size_t seg_need = 16;
   std::vector<SegDev> large_segs;
+  std::vector<char> large_cut;
   for (auto &lp : large) {
-    large_segs.push_back(msvgb_detail::plan_segments(lp.second, db, ctx->num_sms, true));
+    large_segs.emplace_back();
+    large_cut.push_back(msvgb_detail::plan_segments(lp.second, db, ctx->num_sms, true, &large_segs.back()));
     seg_need = std::max(seg_need, msvgb_detail::seg_bytes(large_segs.back()));
   }
   for (int k = 0; k < kSoloBranches && e == cudaSuccess && !large.empty(); ++k) {
-    e = cudaMalloc(&b->d_solo_seg[k], seg_need);
-    if (e != cudaSuccess) break;
+    if (cudaMalloc(&b->d_solo_seg[k], seg_need) != cudaSuccess) {
+      (void) cudaGetLastError();                             // no room for it: uncut
+      b->d_solo_seg[k] = nullptr;
+      large_cut.assign(large.size(), 0);
+      large_segs.assign(large.size(), SegDev());
+      seg_need = 16;
+    }
     e = cudaMalloc(&b->d_solo_counters[k], 4 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_solo_list[k], sizeof(int64_t) * std::max<int64_t>(1, db->n));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->branch[k], cudaStreamNonBlocking);
@@ -315,7 +322,7 @@ int msvgb_detail::batch_create(msvgb_ctx *ctx, const msvgb_om *const *oms, int n
       msvgb_detail::SearchScratch sc;
       sc.stream = b->branch[k]; sc.side = nullptr;
       sc.counters = b->d_solo_counters[k]; sc.list = b->d_solo_list[k];
-      sc.others = sc.cut = true; sc.segs = large_segs[j]; sc.seg = b->d_solo_seg[k];
+      sc.others = true; sc.cut = large_cut[j]; sc.segs = large_segs[j]; sc.seg = b->d_solo_seg[k];
       const int st = msvgb_detail::enqueue_search(sc, large[j].second, db, large_tables[j],
                                                   (uint8_t *) d_xj + (int64_t) large[j].first * db->n,
                                                   (uint8_t *) d_flags + (int64_t) large[j].first * db->n,

@@ -261,8 +261,9 @@ struct SearchScratch {
   msvgb::SegDev segs{};                               // plan_segments
   uint8_t *seg = nullptr;                             // seg_bytes(segs) bytes
 };
-// How a search of db by p cuts its long targets (pointers unset).
-msvgb::SegDev plan_segments(const msvgb_profile *p, const msvgb_db *db, int num_sms, bool others = false);
+// How a search of db by p cuts its long targets (pointers unset; S = 0: none
+// is worth cutting). False: they cannot be cut (cut = false then).
+bool plan_segments(const msvgb_profile *p, const msvgb_db *db, int num_sms, bool others, msvgb::SegDev *ret);
 size_t seg_bytes(const msvgb::SegDev &g);
 // Enqueues the single-profile search of db (per-length tables t) with the
 // lane-group pass when the profile has one (and the search is not small),
