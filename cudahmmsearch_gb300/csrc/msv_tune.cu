@@ -10,9 +10,10 @@
 //     that applies per-bin choices), on a batch of 8 copies of one sampled
 //     profile against that bin's synthetic sequences, so that work items of
 //     the copies interleave and the timing is throughput, not one long tail;
-//   - each choice (int8 table included) on the single-query path against a
-//     database with the usual protein length law (lognormal, median 300,
-//     sigma 0.7): the choice for a whole length mix.
+//   - each choice (int8 table included) on the single-query path, run as
+//     msvgb_profile_create would run it, against a database with the usual
+//     protein length law (lognormal, median 300, sigma 0.7): the choice for a
+//     whole length mix.
 // It keeps the fastest per (M, bin) and for the mix, and can save / load the
 // table. Without a table the choice is a fixed rule (default_lanes) that
 // measurements on GB300 support.
@@ -245,7 +246,8 @@ extern "C" int msvgb_autotune(msvgb_ctx *ctx, double budget_s) {
       if (!cand_valid(M, kCand[ci])) continue;
       msvgb_profile *p = nullptr;
       st = msvgb_profile_create_ex(ctx, &om, kCand[ci].variant, &p);
-      if (st == MSVGB_eslOK && kCand[ci].lanes < 32) st = msvgb_profile_set_lanes(p, &om, kCand[ci].lanes);
+      // as a profile that chose these lanes itself runs (8 short: 4 lanes, long targets cut)
+      if (st == MSVGB_eslOK && kCand[ci].lanes < 32) st = msvgb_detail::profile_auto_lanes(p, &om, kCand[ci].lanes);
       const bool as_asked = st == MSVGB_eslOK && p->f16 == kCand[ci].variant;
       if (as_asked) {
         const int64_t n = msvgb_db_nseq(mix);
