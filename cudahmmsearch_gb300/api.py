@@ -37,7 +37,7 @@ EXPORTS = [
     "msvgb_h3f_open", "msvgb_h3f_read", "msvgb_h3f_close", "msvgb_h3f_write", "msvgb_fasta_read",
     "msvgb_seqs_n", "msvgb_seqs_codes", "msvgb_seqs_offsets", "msvgb_seqs_name", "msvgb_seqs_free",
     "msvgb_db_save", "msvgb_db_load", "msvgb_db_lengths", "msvgb_search_host",
-    "msvgb_vprofile_create", "msvgb_vprofile_destroy", "msvgb_vitfilter", "msvgb_vit_score", "msvgb_vit_scores", "msvgb_vit_move_cost",
+    "msvgb_vprofile_create", "msvgb_vprofile_destroy", "msvgb_vprofile_packed", "msvgb_vitfilter", "msvgb_vit_score", "msvgb_vit_scores", "msvgb_vit_move_cost",
     "msvgb_biasfilter", "msvgb_bias_length_term", "msvgb_null_score", "msvgb_stage_pass", "msvgb_pipeline_filters",
     "msvgb_filter_collect", "msvgb_h3f_filter_params", "msvgb_h3p_open", "msvgb_h3p_read", "msvgb_h3p_close",
 ]
@@ -138,6 +138,7 @@ def lib():
         "msvgb_search_host": (i32, [vp, vp, vp, vp, ctypes.c_int64, ctypes.c_double, ctypes.c_int64, vp, vp]),
         "msvgb_vprofile_create": (i32, [vp, ctypes.POINTER(_VOm), ctypes.POINTER(vp)]),
         "msvgb_vprofile_destroy": (i32, [vp]),
+        "msvgb_vprofile_packed": (i32, [vp, i32]),
         "msvgb_vitfilter": (i32, [vp, vp, vp, vp, ctypes.c_int64, vp, vp]),
         "msvgb_vit_score": (ctypes.c_float, [i32, i32, i32, ctypes.POINTER(_VOm)]),
         "msvgb_vit_scores": (i32, [vp, vp, vp, i64, ctypes.POINTER(_VOm), vp]),
@@ -471,6 +472,10 @@ class DeviceVProfile:
         h = ctypes.c_void_p()
         _check(lib().msvgb_vprofile_create(ctx.h, ctypes.byref(o), ctypes.byref(h)))
         self.h, self.ctx, self.vp = h, ctx, vp
+
+    def packed(self, longest: int) -> bool:
+        """Whether a database with this longest target is scored by the packed kernel."""
+        return lib().msvgb_vprofile_packed(self.h, int(longest)) == 1
 
     def close(self):
         if self.h:

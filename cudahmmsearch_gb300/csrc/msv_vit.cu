@@ -878,6 +878,18 @@ extern "C" int msvgb_vprofile_destroy(msvgb_vprofile *p) {
   return MSVGB_eslOK;
 }
 
+// The packed kernel scores a whole call wherever its tables hold for the
+// database's longest target, listed or not: xB falls with the length's move
+// cost, and the padding nodes' cost has to stay below it (VitFastPlan: m0; on
+// the models here that term, not a real node's, sets the limit). Longest
+// target, by that rule: M = 400 2,600,000 residues, 1500 148,000, 2400 44,000, 4000
+// 14,800, 6200 6,600, 8000 4,000 (real entry costs; the real nodes' own terms
+// would allow over a million at M = 4000).
+extern "C" int msvgb_vprofile_packed(const msvgb_vprofile *p, int Lmax) {
+  if (!p || Lmax < 0) return -1;
+  return p->fast_form.W && msvgb_vit_move_cost(p->scale_w, p->nj, Lmax) >= p->fast_move_min ? 1 : 0;
+}
+
 // ids: original indices of the sequences to score; out_xc[j], out_status[j]
 // (0 ok, 1 overflow, 2 empty) for ids[j].
 extern "C" int msvgb_vitfilter(msvgb_ctx *c, msvgb_vprofile *p, const msvgb_db *db, const int64_t *ids, int64_t nids,
@@ -932,8 +944,7 @@ extern "C" int msvgb_vitfilter(msvgb_ctx *c, msvgb_vprofile *p, const msvgb_db *
   V.xwN_loop = p->xw[1][1]; V.xwJ_loop = p->xw[2][1]; V.xwC_loop = p->xw[3][1];
   V.trans = p->d_trans; V.emit = p->d_emit; V.move = d_move;
   DbDev dbv{db->d_codes, db->d_start, db->d_len, db->d_orig, db->n};
-  // the packed kernel wherever its tables hold for the database's longest target
-  const bool fast = p->fast_form.W && msvgb_vit_move_cost(p->scale_w, p->nj, db->Lmax) >= p->fast_move_min;
+  const bool fast = msvgb_vprofile_packed(p, db->Lmax) == 1;
   VitFastDev VF = p->fast;
   VF.move = d_move;
   if (e == cudaSuccess)

@@ -182,13 +182,23 @@ typedef struct {
   int16_t        base_w, ddbound_w;
 } msvgb_vom;
 typedef struct msvgb_vprofile msvgb_vprofile;
-/* Models up to 8192 nodes (above 1536 the DP row lives in shared memory). */
+/* Models up to 8192 nodes. */
 int msvgb_vprofile_create(msvgb_ctx *ctx, const msvgb_vom *vom, msvgb_vprofile **ret);
 int msvgb_vprofile_destroy(msvgb_vprofile *vp);
+/* Whether a database whose longest target has Lmax residues is scored by the
+ * packed kernel (1) or by the general ones (0), which give the same scores but
+ * took 2.5 to 15 times as long on lists of thousands: packed up to a length that
+ * falls with the model's (M = 400 about 2,600,000 residues, 1500 148,000, 2400 44,000,
+ * 4000 14,800, 8000 4,000); never for costs outside its conditions. -1: bad
+ * arguments. One long target, listed or not, decides for every call on its
+ * database: for models above about 2400 nodes keep such targets in one of
+ * their own. */
+int msvgb_vprofile_packed(const msvgb_vprofile *vp, int Lmax);
 /* p7_ViterbiFilter on the listed sequences of db (ids: original indices, e.g.
  * the MSV survivors): out_xc[j] the final xC, out_status[j] 0 ok, 1 overflow
- * (eslERANGE: +inf), 2 empty. One warp per sequence; bit-exact with the
- * reference's int16 saturating filter, lazy F included. */
+ * (eslERANGE: +inf), 2 empty. One warp per sequence, or the 4 or 8 warps of a
+ * block above 1024 nodes; bit-exact with the reference's int16 saturating
+ * filter, lazy F included. */
 int msvgb_vitfilter(msvgb_ctx *ctx, msvgb_vprofile *vp, const msvgb_db *db, const int64_t *ids, int64_t nids,
                     int *out_xc, uint8_t *out_status);
 /* The filter score in nats from xC (vitfilter.c:240-247, exact float
