@@ -24,8 +24,6 @@
 #include <cuda_runtime.h>
 
 #include "../../include/msvgb.h"
-#include "msv_device.cuh"
-#include "msv_kernel_impl.cuh"
 #include "msv_internal.h"
 
 using namespace msvgb;
@@ -177,9 +175,6 @@ cudaError_t msvgb_detail::dispatch(int C, bool f16, const LaunchArgs &a, int sms
 #undef CASE_F16
 }
 
-namespace msvgb {
-template <int C, int G, int CI> cudaError_t launch_ssv_group(const GroupArgs &a, int num_sms);
-}
 
 // Mixed-width instantiations (inst_hyb*.cu): (C, G, CI) triples.
 #include "msv_hyb_list.h"
@@ -220,12 +215,6 @@ cudaError_t msvgb_detail::dispatch_group(int C, int G, int CI, const GroupArgs &
 #undef G4
 }
 
-namespace msvgb {
-template <int C, int G>
-cudaError_t launch_list_group(const ProfDev &P, const DbDev &db, uint8_t *out_xj, uint8_t *out_flags,
-                              unsigned long long *ticket, const int64_t *list, const unsigned long long *list_count,
-                              const SegDev &segs, int num_sms, cudaStream_t stream);
-}
 
 cudaError_t msvgb_detail::dispatch_list_group(int C, int G, const ProfDev &P, const DbDev &db, uint8_t *out_xj,
                                               uint8_t *out_flags, unsigned long long *ticket, const int64_t *list,

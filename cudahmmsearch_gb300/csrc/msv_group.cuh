@@ -400,6 +400,9 @@ __device__ __forceinline__ void ssv_group_chunk(const ProfDev &P, const uint32_t
       [&](int64_t s) { und[atomicAdd(n_und, 1u)] = (uint16_t) (s - s0); });
 }
 
+#ifdef MSVGB_LAUNCHERS_ELSEWHERE
+template <int C, int G, int CI = 0> cudaError_t launch_ssv_group(const GroupArgs &a, int num_sms);
+#else
 template <int C, int G, int CI = 0>
 cudaError_t launch_ssv_group(const GroupArgs &a, int num_sms) {
   // wide rows without segments keep their own kernel: the segments' state
@@ -430,6 +433,7 @@ cudaError_t launch_ssv_group(const GroupArgs &a, int num_sms) {
                                       a.s_begin, a.segs);
   return cudaGetLastError();
 }
+#endif
 
 }  // namespace msvgb
 
@@ -589,6 +593,12 @@ msv_list_group_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t
   }
 }
 
+#ifdef MSVGB_LAUNCHERS_ELSEWHERE
+template <int C, int G>
+cudaError_t launch_list_group(const ProfDev &P, const DbDev &db, uint8_t *out_xj, uint8_t *out_flags,
+                              unsigned long long *ticket, const int64_t *list, const unsigned long long *list_count,
+                              const SegDev &segs, int num_sms, cudaStream_t stream);
+#else
 template <int C, int G>
 cudaError_t launch_list_group(const ProfDev &P, const DbDev &db, uint8_t *out_xj, uint8_t *out_flags,
                               unsigned long long *ticket, const int64_t *list, const unsigned long long *list_count,
@@ -613,6 +623,7 @@ cudaError_t launch_list_group(const ProfDev &P, const DbDev &db, uint8_t *out_xj
   kern<<<(unsigned) grid, 256, smem, stream>>>(P, db, out_xj, out_flags, ticket, list, list_count, segs);
   return cudaGetLastError();
 }
+#endif
 
 }  // namespace msvgb
 

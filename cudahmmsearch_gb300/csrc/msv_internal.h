@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/msvgb.h"
+#define MSVGB_LAUNCHERS_ELSEWHERE   // the kernels' launchers are compiled in inst_*.cu only
 #include "msv_kernel_impl.cuh"
 #include "msv_group.cuh"
 

@@ -123,6 +123,9 @@ msv_search_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t *__
   }
 }
 
+#ifdef MSVGB_LAUNCHERS_ELSEWHERE
+template <int C, bool F16> cudaError_t launch_search(const LaunchArgs &a, int num_sms);
+#else
 template <int C, bool F16>
 cudaError_t launch_search(const LaunchArgs &a, int num_sms) {
   auto kern = msv_search_kernel<C, F16>;
@@ -156,6 +159,7 @@ cudaError_t launch_search(const LaunchArgs &a, int num_sms) {
                                                a.range_end, a.segs);
   return cudaGetLastError();
 }
+#endif
 
 }  // namespace msvgb
 
