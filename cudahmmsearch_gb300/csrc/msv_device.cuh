@@ -401,7 +401,7 @@ __device__ __forceinline__ int msv_full(const ProfDev &P, const uint32_t *__rest
   return ST_OK;
 }
 
-template <int C, bool F16>
+template <int C, bool F16, int RW = 1>
 __device__ __forceinline__ int msv_one(const ProfDev &P, const uint32_t *__restrict__ stab,
                                        const uint32_t *__restrict__ mtab,
                                        const uint32_t *__restrict__ sq, int L, int lane,
@@ -409,7 +409,7 @@ __device__ __forceinline__ int msv_one(const ProfDev &P, const uint32_t *__restr
   const int tjb = P.tjb[L];
   full_out = 0;
   if (!skip_ssv && tjb + P.tbm + P.tec + P.bias < 127) {
-    const int umax = ssv_range<C, F16>(stab, sq, 0, L, lane);
+    const int umax = ssv_range<C, F16, RW>(stab, sq, 0, L, lane);
     const int st = ssv_decide(umax, tjb, P.tbm, P.tec, P.base, P.bias, xj_out);
     if (st >= 0) return st;
   }

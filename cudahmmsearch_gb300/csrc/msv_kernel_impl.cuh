@@ -49,6 +49,24 @@ constexpr int cta_threads() { return 2 * smem_bytes<C, F16>() > 227 * 1024 ? MAX
 template <int C, bool F16>
 __host__ __device__ constexpr int row_words() { return F16 && C <= 8 ? 2 : 1; }
 
+// Both tables into shared memory, unless they stay in global memory.
+template <int C, bool F16>
+__device__ __forceinline__ void stage_tables(uint32_t *smem, const uint32_t *&stab, const uint32_t *&mtab) {
+  constexpr int SW = F16 ? NRES * C * 32 : NRES * (C / 2) * 32;   // words of the SSV table
+  constexpr int MW = NRES * ((C + 1) / 2) * 32;                    // words of the MSV table
+  if constexpr (!tables_in_global<C, F16>()) {
+    const uint4 *gs = reinterpret_cast<const uint4 *>(stab);
+    const uint4 *gm = reinterpret_cast<const uint4 *>(mtab);
+    uint4 *ss = reinterpret_cast<uint4 *>(smem);
+    uint4 *sm = reinterpret_cast<uint4 *>(smem + SW);
+    for (int i = threadIdx.x; i < SW / 4; i += blockDim.x) ss[i] = __ldg(gs + i);
+    for (int i = threadIdx.x; i < MW / 4; i += blockDim.x) sm[i] = __ldg(gm + i);
+    stab = smem;
+    mtab = smem + SW;
+    __syncthreads();
+  }
+}
+
 // Persistent kernel: every CTA stages the profile's cost tables into shared
 // memory once, then its warps pull sequences or segments of long ones (longest
 // first) from a global ticket until the database is exhausted. Bound by
@@ -60,21 +78,8 @@ msv_search_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t *__
                   unsigned long long *__restrict__ ticket, int skip_empty,
                   int64_t range_end, const __grid_constant__ SegDev segs) {
   extern __shared__ __align__(16) uint32_t smem[];
-  constexpr int SW = F16 ? NRES * C * 32 : NRES * (C / 2) * 32;   // words of the SSV table
-  constexpr int MW = NRES * ((C + 1) / 2) * 32;                    // words of the MSV table
   const uint32_t *stab = P.stab, *mtab = P.mtab;
-  if constexpr (!tables_in_global<C, F16>()) {
-    const uint4 *gs = reinterpret_cast<const uint4 *>(P.stab);
-    const uint4 *gm = reinterpret_cast<const uint4 *>(P.mtab);
-    uint4 *ss = reinterpret_cast<uint4 *>(smem);
-    uint4 *sm = reinterpret_cast<uint4 *>(smem + SW);
-    for (int i = threadIdx.x; i < SW / 4; i += blockDim.x) ss[i] = __ldg(gs + i);
-    for (int i = threadIdx.x; i < MW / 4; i += blockDim.x) sm[i] = __ldg(gm + i);
-    stab = smem;
-    mtab = smem + SW;
-    __syncthreads();
-  }
-
+  stage_tables<C, F16>(smem, stab, mtab);
   const int lane = threadIdx.x & 31;
   const unsigned long long nseg = segs.S ? segs.base[segs.S] : 0ull;
   const unsigned long long nitems = (unsigned long long) (range_end > 0 ? range_end : db.n - segs.nl) + nseg;
@@ -123,16 +128,68 @@ msv_search_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t *__
   }
 }
 
+// Blocks per SM that the whole-sequence kernel is compiled for (0: the
+// compiler's own choice), and words of four residues per step of its SSV loop.
+template <int C, bool F16>
+__host__ __device__ constexpr int whole_blocks() { return !F16 || C <= 32 ? 1 : 0; }
+template <int C, bool F16>
+__host__ __device__ constexpr int whole_words() { return F16 && C > 8 && C <= 32 ? 1 : 2; }
+
+// The same search with no sequence cut: long targets beside a lane-group pass,
+// chunks of a host search, calls that may not allocate. A warp's time is then
+// the chain of the longest rows it scores, and how far ahead of it the
+// compiler loads the costs sets that chain: a bound of one block per SM frees
+// the registers for it, eight rows a step give it room. ns per row of one warp,
+// SSV / full MSV, in the kernel for both and here (f16 tables): C = 1 22.7 / 137
+// and 21.5 / 129, 3 33.3 / 144 and 17.7 / 135, 6 43.3 / 155 and 18.3 / 144, 11 45.0 / 168
+// and 27.2 / 160, 16 45.0 / 190 and 31.0 / 174, 21 52.4 / 193 and 44.9 / 179, 32 71.0 / 261
+// and 67.3 / 233 (with eight rows a step 60.7 / 249), 52 129 / 395 and 103 / 395 (with
+// the bound 101 / 404), 96 291 / 950 and 268 / 890 (with it 368 / 888, and 34% longer
+// where the SMs are full).
+template <int C, bool F16>
+__global__ void __launch_bounds__(cta_threads<C, F16>(), whole_blocks<C, F16>())
+msv_whole_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t *__restrict__ out_flags,
+                 unsigned long long *__restrict__ ticket, int skip_empty, int64_t range_end) {
+  extern __shared__ __align__(16) uint32_t smem[];
+  const uint32_t *stab = P.stab, *mtab = P.mtab;
+  stage_tables<C, F16>(smem, stab, mtab);
+  const int lane = threadIdx.x & 31;
+  const unsigned long long nitems = (unsigned long long) (range_end > 0 ? range_end : db.n);
+  for (;;) {
+    unsigned long long s = 0;
+    if (lane == 0) s = atomicAdd(ticket, 1ull);
+    s = __shfl_sync(FULL, s, 0);
+    if (s >= nitems) break;
+    const int L = db.len[s];
+    const int64_t oi = db.orig[s];
+    if (L == 0 && skip_empty) {
+      if (lane == 0) { out_xj[oi] = 0; out_flags[oi] = 0x08; }   // MSVGB_FLAG_EMPTY
+      continue;
+    }
+    const uint32_t *sq = reinterpret_cast<const uint32_t *>(db.codes + db.start[s]);
+    int xj, full;
+    const int st = msv_one<C, F16, whole_words<C, F16>()>(P, stab, mtab, sq, L, lane, xj, full);
+    if (lane == 0) {
+      int flags = full ? 0x04 : 0;
+      if (st == ST_ERANGE) flags |= 0x01 | 0x02;                 // +inf always passes F1
+      else if (xj >= P.xjmin[L]) flags |= 0x02;
+      out_xj[oi] = (uint8_t) xj;
+      out_flags[oi] = (uint8_t) flags;
+    }
+  }
+}
+
 #ifdef MSVGB_LAUNCHERS_ELSEWHERE
 template <int C, bool F16> cudaError_t launch_search(const LaunchArgs &a, int num_sms);
 #else
 template <int C, bool F16>
 cudaError_t launch_search(const LaunchArgs &a, int num_sms) {
-  auto kern = msv_search_kernel<C, F16>;
+  const bool cut = a.segs.S != 0;
+  const void *kern = cut ? (const void *) msv_search_kernel<C, F16> : (const void *) msv_whole_kernel<C, F16>;
   constexpr size_t smem = smem_bytes<C, F16>();
-  static std::atomic<unsigned long long> configured{0};
+  static std::atomic<unsigned long long> configured[2];
   {
-    cudaError_t e = ensure_smem_attr((const void *) kern, smem, configured);
+    cudaError_t e = ensure_smem_attr(kern, smem, configured[cut]);
     if (e != cudaSuccess) return e;
   }
   constexpr int threads = cta_threads<C, F16>();
@@ -144,10 +201,10 @@ cudaError_t launch_search(const LaunchArgs &a, int num_sms) {
     if (per_sm < 1) per_sm = 1;
     // Where long targets are cut the chains set the time, and they run faster
     // with fewer warps beside them (8 / 4 / 3 / 2 blocks per SM, us: M = 130, 40,000
-    // targets 369 / 370 / 381 / 431; M = 200, 20,000 247 / 239 / 241 / 243; M = 400, 5,000 261 /
-    // 260 / 248 / 232, 40,000 552 / 553 / 484 / 483; M = 550, 10,000 334 / 329 / 310 / 286,
-    // 60,000 872 / 876 / 834 / 844; M = 800, 10,000 393 / 392 / 398 / 344).
-    if (F16 && a.segs.S) per_sm = std::min(per_sm, C <= 3 ? 4 : C == 4 ? 3 : 2);
+    // targets 369 / 370 / 381 / 431; M = 400, 5,000 261 / 260 / 248 / 232, 40,000 552 / 553 / 484 /
+    // 483; M = 550, 10,000 334 / 329 / 310 / 286, 60,000 872 / 876 / 834 / 844; M = 800, 10,000 393 /
+    // 392 / 398 / 344; 4 / 3 blocks at M = 225: 5,000 189 / 173, 20,000 241 / 233, 40,000 348 / 335).
+    if (F16 && cut) per_sm = std::min(per_sm, C <= 3 ? 4 : C == 4 ? 3 : 2);
     grid = per_sm * num_sms;
     const int warps = threads / 32;
     const long long items = a.range_end > 0 ? a.range_end : a.db.n - a.segs.nl + (a.segs.S ? a.segs.base[a.segs.S] : 0);
@@ -155,8 +212,12 @@ cudaError_t launch_search(const LaunchArgs &a, int num_sms) {
     if (need < grid) grid = (int) (need > 0 ? need : 1);
   }
   (void) cudaGetLastError();   // clear a stale error left by an unrelated call
-  kern<<<grid, threads, smem, a.stream>>>(a.P, a.db, a.out_xj, a.out_flags, a.ticket, a.skip_empty,
-                                               a.range_end, a.segs);
+  if (cut)
+    msv_search_kernel<C, F16><<<grid, threads, smem, a.stream>>>(a.P, a.db, a.out_xj, a.out_flags, a.ticket, a.skip_empty,
+                                                                 a.range_end, a.segs);
+  else
+    msv_whole_kernel<C, F16><<<grid, threads, smem, a.stream>>>(a.P, a.db, a.out_xj, a.out_flags, a.ticket, a.skip_empty,
+                                                                a.range_end);
   return cudaGetLastError();
 }
 #endif
