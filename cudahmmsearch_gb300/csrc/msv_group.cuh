@@ -360,8 +360,19 @@ __host__ __device__ constexpr int group_table_words() {
   else return GroupLayout<C, G>::WORDS;
 }
 
+// Blocks per SM the pass is compiled for (0: the compiler's own choice). Without
+// segments a bound of one, which frees the registers to load costs further
+// ahead, is the faster below 24 words and at 28: us at 100,000 / 400,000 targets of
+// up to 2399 rows without / with it: 8 lanes, C = 9 336 / 1303 and 334 / 1305, 11 514 / 1560 and 441 / 1522,
+// 13 484 / 1711 and 455 / 1682, 18 634 / 2119 and 547 / 2152, 22 648 / 2531 and 637 / 2491, 26 751 /
+// 2944 and 746 / 2958, 28 836 / 3148 and 788 / 3116, 32 891 / 3518 and 893 / 3548; 16 lanes, C = 9 690 /
+// 2599 and 655 / 2595, 19 1239 / 4709 and 1196 / 4758, 28 1710 / 6299 and 1545 / 6143, 32 1759 / 7001 and
+// 1792 / 7147; 32 lanes, C = 28 3378 / 13490 and 3190 / 12742.
+template <int C, bool SEG>
+__host__ __device__ constexpr int group_blocks() { return !SEG && (C < 24 || C == 28) ? 1 : 0; }
+
 template <int C, int G, int CI, bool SEG>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, group_blocks<C, SEG>())
 msv_ssv_group_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t *__restrict__ out_flags,
                      unsigned long long *__restrict__ ticket, int64_t *__restrict__ undecided,
                      unsigned long long *__restrict__ n_undecided, int64_t s_begin,
@@ -405,13 +416,14 @@ template <int C, int G, int CI = 0> cudaError_t launch_ssv_group(const GroupArgs
 #else
 template <int C, int G, int CI = 0>
 cudaError_t launch_ssv_group(const GroupArgs &a, int num_sms) {
-  // wide rows without segments keep their own kernel: the segments' state
-  // takes registers (64 -> 78 at 26 words per lane: 3 blocks per SM for 4);
-  // tables set by hand run without segments
-  constexpr bool cuts = CI == hyb_words(C, G), whole = !cuts || C >= 20;
+  // without segments the pass has a kernel of its own: their state takes
+  // registers (64 -> 78 at 26 words per lane: 3 blocks per SM for 4; 400,000
+  // targets in one kernel for both: 3 to 5% longer at most widths below 20
+  // words); tables set by hand run without segments
+  constexpr bool cuts = CI == hyb_words(C, G);
   if (!cuts && a.segs.S) return cudaErrorInvalidValue;
-  auto kern = msv_ssv_group_kernel<C, G, CI, !whole>;
-  if constexpr (cuts && whole) {
+  auto kern = msv_ssv_group_kernel<C, G, CI, false>;
+  if constexpr (cuts) {
     if (a.segs.S) kern = msv_ssv_group_kernel<C, G, CI, true>;
   }
   static_assert(group_words(C, G, CI) == group_table_words<C, G, CI>(), "host and device table sizes agree");
@@ -490,8 +502,14 @@ __device__ __forceinline__ uint32_t msv_row_group(uint32_t (&dp)[C], uint32_t xB
 
 // Full MSV of the listed sequences list[*ticket .. *list_count) (taken one
 // per group from the ticket), written as msv_search_kernel's list mode does.
-template <int C, int G>
-__global__ void __launch_bounds__(256)
+// SEG: the longest sequences have been cut, and rows no score depends on are
+// skipped. A kernel of its own: the skipping costs every row's chain up to a
+// third, and without it a bound of one block per SM makes the chain shorter (us
+// for 40 / 2,500 listed targets in the kernel for both and without: 8 lanes, C = 9 491 /
+// 496 and 395 / 435, 19 606 / 613 and 440 / 513, 26 573 / 654 and 471 / 566; 16 lanes, C = 10 554 /
+// 631 and 444 / 515, 25 671 / 738 and 614 / 719; 32 lanes, C = 24 696 / 831 and 651 / 761).
+template <int C, int G, bool SEG>
+__global__ void __launch_bounds__(256, SEG ? 0 : 1)
 msv_list_group_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t *__restrict__ out_flags,
                       unsigned long long *__restrict__ ticket, const int64_t *__restrict__ list,
                       const unsigned long long *__restrict__ list_count, const __grid_constant__ SegDev segs) {
@@ -535,7 +553,7 @@ msv_list_group_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t
         xJ = 0;
         xB = max(base - tjbm, 0);
         er = false;
-        next_blk = s < segs.nl ? 0 : -1;
+        if constexpr (SEG) next_blk = s < segs.nl ? 0 : -1;
         sq = reinterpret_cast<const uint32_t *>(db.codes + db.start[s]);
         nextw = __ldg(sq);
         i = 0;
@@ -546,7 +564,7 @@ msv_list_group_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t
     }
     if (__all_sync(FULL, done)) break;
     const bool active = !need && !done;
-    if (active && next_blk >= 0 && i == next_blk * segs.R) {   // rows no score depends on are skipped
+    if (SEG && active && next_blk >= 0 && i == next_blk * segs.R) {   // rows no score depends on are skipped
       const int nb = (L + segs.R - 1) / segs.R;
       const int k = seg_next_hot(segs, s, nb, next_blk, min(xB, 255 - bias), tec, base, bias, xJ);
       const int r = k * segs.R - segs.warm;
@@ -603,11 +621,11 @@ template <int C, int G>
 cudaError_t launch_list_group(const ProfDev &P, const DbDev &db, uint8_t *out_xj, uint8_t *out_flags,
                               unsigned long long *ticket, const int64_t *list, const unsigned long long *list_count,
                               const SegDev &segs, int num_sms, cudaStream_t stream) {
-  auto kern = msv_list_group_kernel<C, G>;
+  auto kern = segs.S ? msv_list_group_kernel<C, G, true> : msv_list_group_kernel<C, G, false>;
   constexpr size_t smem = (size_t) GroupLayout<C, G>::WORDS * 4;
-  static std::atomic<unsigned long long> configured{0};
+  static std::atomic<unsigned long long> configured[2];
   {
-    cudaError_t e = ensure_smem_attr((const void *) kern, smem, configured);
+    cudaError_t e = ensure_smem_attr((const void *) kern, smem, configured[segs.S != 0]);
     if (e != cudaSuccess) return e;
   }
   int per_sm = 0;
