@@ -1389,6 +1389,25 @@ extern "C" int msvgb_search(msvgb_ctx *c, const msvgb_profile *p, const msvgb_db
 // scored by one full-MSV pass at the end, on S[0].
 // ctr: 6 zeroed counters (per-stream tickets for the long and main passes,
 // the list count, the list ticket); list: room for db->n entries.
+// Whether a profile that chose its lanes itself scores a database's chunks on
+// lane groups. A chunk is a search of its own, so the groups fill later than
+// in a resident search (search_fused): from 190M residues or 40e9 cells, at once
+// below 32 nodes (a warp's row is then half padding), and where targets of
+// kLongTarget or more hold a quarter of the residues (they run beside the
+// groups' pass). Groups / fused, ms: M = 22, 72M residues 1.58 / 1.53, 120M 1.77 / 2.01, 240M
+// 2.95 / 3.20; 48, 72M 1.98 / 1.64, 160M 2.63 / 2.42, 240M 3.29 / 3.30, 400M 5.13 / 5.48; 130, 120M
+// 2.92 / 2.75, 160M 3.34 / 3.31, 200M 3.73 / 4.10; 200, 120M 3.63 / 2.94, 160M 4.01 / 3.52; 420, 72M 3.58 /
+// 2.74; half of the residues in long targets: 200, 72M 12.5 / 13.6; 420, 72M 14.3 / 16.4; 86,
+// 72M 14.9 / 14.7; 250, 120M 14.8 / 14.8.
+static bool chunks_on_groups(const msvgb_profile *p, const msvgb_db *db) {
+  if (!p->d_stab_g) return false;
+  if (!p->lanes_auto || p->M < 32 || db->residues >= 190000000 || (double) p->M * (double) db->residues >= 4e10) return true;
+  int64_t in_long = 0;
+  for (size_t i = db->distinct_len.size(); i-- > 0 && db->distinct_len[i] >= kLongTarget;)
+    in_long += db->len_count[i] * db->distinct_len[i];
+  return in_long >= db->residues / 4;
+}
+
 static int search_chunked(msvgb_ctx *c, const msvgb_profile *p, msvgb_db *db, const LenTables *t, uint8_t *d_xj,
                           uint8_t *d_flags, unsigned long long *ctr, int64_t *list, msvgb_detail::GpuTrace &gt) {
   using namespace msvgb_detail;
@@ -1418,7 +1437,7 @@ static int search_chunked(msvgb_ctx *c, const msvgb_profile *p, msvgb_db *db, co
   ProfDev P32;
   P32.M = p->M; P32.C = p->C; P32.tbm = p->tbm; P32.tec = p->tec; P32.base = p->base; P32.bias = p->bias;
   P32.stab = p->d_stab; P32.mtab = p->d_mtab; P32.tjb = t->d_tjb; P32.xjmin = t->d_xjmin; P32.ssv_f16 = p->f16;
-  const bool groups = !search_fused(p, db, false);          // as in enqueue_search, by the whole search
+  const bool groups = chunks_on_groups(p, db);
   ProfDev P = P32;
   int t_long = INT32_MAX;
   if (groups) {
