@@ -1231,14 +1231,22 @@ extern "C" int msvgb_search_device(msvgb_ctx *c, const msvgb_profile *pc, const 
 
 // Whether the search of a profile that chose its lanes itself runs at 32
 // lanes in the fused kernel: where the database is too small to fill the lane
-// groups, by its residues. Lane groups / fused, us: M = 60, 19M residues
-// 295 / 304, 23M 322 / 379; 120, 23M 410 / 395; 160, 23M 460 / 535; 200, 23M
-// 480 / 487; 240, 25M 604 / 550; 400, 23M 749 / 697, 31M 906 / 1111; from 512
-// nodes later: 520, 38M 1457 / 1348; 800, 34M 1734 / 1654; 1200, 23M 1813 /
-// 1575, 34M 2448 / 2337; 2000, 23M 2663 / 2527.
-constexpr int64_t kFusedShort = 24000000, kFusedLong = 36000000;
+// groups, by its residues and the words a lane holds at 32 lanes (the groups
+// pay for a width of 19 words at 5, 9 and 10 of them and of 17 at 17, the fused
+// kernel for one of 6). Lane groups / fused, us: M = 86, 23M residues 405 / 330,
+// 33M 452 / 427, 38M 481 / 491; 200, 23M 473 / 458, 33M 559 / 625; 300, 33M 873 / 773, 38M 999
+// / 899, 48M 1049 / 1113; 350, 23M 666 / 700, 33M 832 / 972; 400, 27M 819 / 797, 33M 925 / 959, 38M 1032 / 1118;
+// 440, 38M 1163 / 1117; 480, 27M 1072 / 869, 48M 1597 / 1500, 58M 1794 / 1788, 73M 2109 / 2255; 576, 38M 1745 /
+// 1474, 58M 2199 / 2168; 688, 38M 1879 / 1642, 58M 2270 / 2371; 800, 38M 1907 / 1849, 48M 2253 / 2289; 1030,
+// 38M 2509 / 2318, 48M 3184 / 2891, 73M 4433 / 4375; 1500, 38M 3075 / 3186, 48M 3837 / 3976.
+static int64_t fused_below(int C) {
+  if (C <= 4 || C == 6) return 24000000;
+  if (C == 5) return 40000000;
+  if (C == 7) return 36000000;
+  return C <= 12 ? 60000000 : 44000000;
+}
 static bool search_fused(const msvgb_profile *p, const msvgb_db *db, bool others) {
-  return !p->d_stab_g || (p->lanes_auto && !others && db->residues < (p->M < 512 ? kFusedShort : kFusedLong));
+  return !p->d_stab_g || (p->lanes_auto && !others && db->residues < fused_below(p->C));
 }
 
 // The segments of a search's long targets. A segment costs its run-in of M
@@ -1260,7 +1268,14 @@ bool msvgb_detail::plan_segments(const msvgb_profile *p, const msvgb_db *db, int
   const bool fused = search_fused(p, db, others);
   const double chains = (double) num_sms * (fused ? (p->C > 32 ? 16.0 : 32.0) : 24.0 * 32.0 / p->Gk);
   const double avg = (double) db->residues / chains;
-  if (db->Lmax < avg / 2) return true;                    // no chain sets the search's length
+  // Chains worth cutting are longer than their share of what the launch holds
+  // scores: half of avg, but in the fused kernel, whose cut form keeps fewer
+  // warps on an SM, all of it from 8 words and 1.7 times it from 17 (us cut /
+  // uncut, longest target 0.9 avg: M = 200 727 / 869, 520 1383 / 1341, 1030 2493 / 2318; 1.4 avg:
+  // 300 646 / 789, 688 1171 / 1355, 1030 1757 / 1634; 2.1 avg: 1030 1149 / 1191), 1.3 times where
+  // the tables are in global memory (1.2 avg: M = 3100 2900 / 2747; 0.7 avg: 5011 / 4754).
+  const double least = !fused || p->C < 8 ? 0.5 : p->C <= 16 ? 1.0 : p->C <= 32 ? 1.7 : p->C <= 40 ? 0.5 : 1.3;
+  if (db->Lmax < least * avg) return true;                // no chain sets the search's length
   const double T = std::max({avg, 2.0 * M, 768.0, (double) db->Lmax / kMaxSegs});
   if (T > 1e8) return false;
   g.R = fused ? 128 : 256;
