@@ -1270,13 +1270,16 @@ bool msvgb_detail::plan_segments(const msvgb_profile *p, const msvgb_db *db, int
   const double avg = (double) db->residues / chains;
   // Chains worth cutting are longer than their share of what the launch holds
   // scores: half of avg, but in the fused kernel, whose cut form keeps fewer
-  // warps on an SM, all of it from 8 words and 1.7 times it from 17 (us cut /
-  // uncut, longest target 0.9 avg: M = 200 727 / 869, 520 1383 / 1341, 1030 2493 / 2318; 1.4 avg:
-  // 300 646 / 789, 688 1171 / 1355, 1030 1757 / 1634; 2.1 avg: 1030 1149 / 1191), 1.3 times where
-  // the tables are in global memory (1.2 avg: M = 3100 2900 / 2747; 0.7 avg: 5011 / 4754).
-  const double least = !fused || p->C < 8 ? 0.5 : p->C <= 16 ? 1.0 : p->C <= 32 ? 1.7 : p->C <= 40 ? 0.5 : 1.3;
-  if (db->Lmax < least * avg) return true;                // no chain sets the search's length
+  // warps on an SM, all of it from 8 words, and from 17, where the run-in weighs,
+  // 1.3 times a segment with its run-in (us cut / uncut, longest
+  // target about 7,300 rows: M = 200, avg 7.9k 727 / 869; 300, 5.5k 646 / 789; 520, 7.9k 1383 / 1341;
+  // 688, 5.5k 1171 / 1355; 1030, 2.8k 910 / 1128, 5.5k 1757 / 1634; 1200, 3.5k 1197 / 1301, 5.5k 1824 / 1803;
+  // 1900, 1.2k 970 / 903, 2.8k 1664 / 1621); 1.3 times avg where the tables are in global
+  // memory (M = 3100, avg 6.3k 2900 / 2747).
   const double T = std::max({avg, 2.0 * M, 768.0, (double) db->Lmax / kMaxSegs});
+  const double least = !fused || p->C < 8 ? 0.5 * avg : p->C <= 16 ? avg : p->C <= 32 ? 1.3 * (T + M)
+                       : p->C <= 40 ? 0.5 * avg : 1.3 * avg;
+  if (db->Lmax < least) return true;                      // no chain sets the search's length
   if (T > 1e8) return false;
   g.R = fused ? 128 : 256;
   g.T = ((int) T + g.R - 1) / g.R * g.R;
