@@ -401,8 +401,8 @@ static int width_for(const msvgb_om *om, int want_f16, int force_C, int *ret_C, 
   return MSVGB_eslOK;
 }
 
-// DP words per lane and 8-bit words per lane of the G-lane tables (G = 16 or
-// 8, or 32 for the split passes of models of 1024-2047 nodes).
+// DP words per lane and 8-bit words per lane of the G-lane tables (G = 16, 8
+// or 4, or 32 for the split passes of models of 1024-2047 nodes).
 static int group_width(int M, int G, int *ret_C, int *ret_CI) {
   const int C = M / (2 * G) + 1;                          // 2*C*G > M: the last node is padding
   if (C > 32) return fail(MSVGB_eslEINVAL, "model too long for this many lanes per sequence");

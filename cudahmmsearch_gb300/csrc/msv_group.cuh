@@ -2,15 +2,16 @@
 //
 // For small models a whole warp per sequence leaves each lane only a few DP
 // words per row, so the per-row overhead (the shuffle, the residue decode,
-// the table address) dominates. Here G lanes (8 or 16) score one sequence and
-// a warp carries 32/G sequences in lockstep: each group owns its sequence
+// the table address) dominates. Here G lanes (4, 8 or 16; 32 for models of 1024
+// nodes and more) score one sequence and a warp carries 32/G sequences in
+// lockstep: each group owns its sequence
 // state (index, row, residue word) and fetches the next sequence when its own
 // ends, while all lanes execute the same row code every step (finished groups
 // run pad rows, whose costs keep every cell at the floor). Lane g of a group
 // owns nodes g*2C+1 .. (g+1)*2C with the same two-way striping as the 32-lane
 // kernel. Only phase A (SSV) runs here; sequences SSV leaves undecided, or
-// whose length disables SSV, are appended to a list that the 32-lane kernel
-// then scores with the full MSV recurrence (list mode).
+// whose length disables SSV, are appended to a list that the same lane groups
+// then score with the full MSV recurrence (msv_list_group_kernel).
 #pragma once
 #include "msv_device.cuh"
 
@@ -106,7 +107,9 @@ __device__ __forceinline__ uint32_t add_f16x2(uint32_t a, uint32_t b) {
 // 19.1 / 20.3 / 20.9a. With every 8-bit word on the FMA pipe C = 26 took 16.3 ms
 // for 2,000,000 sequences, 15.8 with none. At C = 26 and 8 words the pass reads
 // shared memory in 97.7% of cycles, but more 8-bit words still lose below 28
-// (12: 18.3a, 16: 18.5 with 8 on the FMA pipe, 8: 19.5): the ALU pipe takes over.
+// (12 with 4 on the FMA pipe: 18.3, 16 with 8: 18.5, 8: 19.5): the ALU pipe takes
+// over; 12 with none there was not measured. 4 lanes take the 8-lane shares,
+// unswept.
 __host__ __device__ constexpr int hyb_words(int C, int G) {
   if (G == 32) return C < 17 ? 0 : 8;
   if (C < (G == 16 ? 13 : 10)) return 0;
@@ -179,7 +182,9 @@ __device__ __forceinline__ void ssv_row_hyb(uint32_t (&dp)[C], uint32_t &acc0, u
   for (int w = C - 1; w >= 0; --w)
     dp[w] = w < Lay::CB ? fma_relu_f16x2(w ? dp[w - 1] : pred0, one2, s[w])
                    : __viaddmax_s16x2(w ? dp[w - 1] : pred0, s[w], 0u);
-  // running maximum on the bits (signed: a -0 from the relu is the smallest):
+  // running maximum on the bits (non-negative; fma.rn.relu gives +0, never -0,
+  // which the integer words would read as -32768: all 2048 x 511 pairs of a
+  // cell and a cost checked on the GPU):
   // one three-input maximum per two words takes fewer issue slots than two
   // maxima, and issue, not the integer pipe, is what this row runs short of
   // (measured: 16.3 vs 17.0 ms at M = 400 on 2,000,000 sequences)
@@ -501,7 +506,7 @@ __device__ __forceinline__ uint32_t msv_row_group(uint32_t (&dp)[C], uint32_t xB
 }
 
 // Full MSV of the listed sequences list[*ticket .. *list_count) (taken one
-// per group from the ticket), written as msv_search_kernel's list mode does.
+// per group from the ticket), written with the full-MSV flag.
 // SEG: the longest sequences have been cut, and rows no score depends on are
 // skipped. A kernel of its own: the skipping costs every row's chain up to a
 // third, and without it a bound of one block per SM makes the chain shorter (us

@@ -67,9 +67,10 @@ __device__ __forceinline__ void stage_tables(uint32_t *smem, const uint32_t *&st
   }
 }
 
-// Persistent kernel: every CTA stages the profile's cost tables into shared
-// memory once, then its warps pull sequences or segments of long ones (longest
-// first) from a global ticket until the database is exhausted. Bound by
+// Persistent kernel for searches that cut their long targets (segs.S > 0;
+// msv_whole_kernel otherwise): every CTA stages the profile's cost tables into
+// shared memory once, then its warps pull segments and whole sequences
+// (longest first) from a global ticket until the database is exhausted. Bound by
 // shared memory where the database fills the SMs (2 bytes of cost per cell),
 // by the longest chain of rows where it does not (SegDev).
 template <int C, bool F16>

@@ -807,7 +807,7 @@ extern "C" int msvgb_vprofile_create(msvgb_ctx *ctx, const msvgb_vom *v, msvgb_v
   size_t tbytes = trans.size() * (vit_t32(CV) ? 4 : 2);
   const void *esrc = emit.data();
   size_t ebytes = emit.size() * 2;
-  // the packed form (8 .. 96 nodes per lane): two nodes per word
+  // the packed form (40 and 48 nodes per lane): two nodes per word
   const bool packed = vit_packed(CV);
   std::vector<uint32_t> ptr, pem;
   if (packed) {

@@ -112,7 +112,7 @@ int msvgb_profile_create_ex(msvgb_ctx *ctx, const msvgb_om *om, int ssv_variant,
 int msvgb_profile_variant(const msvgb_profile *prof);
 /* Lanes per sequence of the SSV pass: 32 (one warp per sequence, SSV
  * and full MSV in one kernel; for models of 1024 to 2047 nodes, searches of
- * at least 36M residues -- or any search, when lanes are set here -- run the
+ * at least 44M residues -- or any search, when lanes are set here -- run the
  * SSV pass and the full MSV as two launches on 32-lane groups instead, with
  * the mixed-width table), or 16 / 8 (2 / 4 sequences per warp in
  * lockstep, for small models: each lane then holds more DP words per row);
@@ -123,8 +123,8 @@ int msvgb_profile_variant(const msvgb_profile *prof);
  * launch; otherwise long targets are cut into segments that are scored
  * independently. om must be the profile's own MSV fields. Needs M < 64 * G
  * and, for G < 32, M >= 2 * G. Lanes chosen by msvgb_profile_create apply to
- * searches of at least 24M residues (36M from 512 nodes up); smaller ones run
- * at 32 lanes, where the shorter per-sequence latency wins; where the choice
+ * searches of at least 24M to 60M residues, by the model's length; smaller ones
+ * run at 32 lanes, where the shorter per-sequence latency wins; where the choice
  * is 8 and M < 256 those searches run at 4 lanes. Lanes set here always
  * apply. */
 int msvgb_profile_set_lanes(msvgb_profile *prof, const msvgb_om *om, int lanes);
@@ -216,7 +216,8 @@ int16_t msvgb_vit_move_cost(float scale_w, float nj, int L);
  * transition, scored with esl_hmm_Forward (easel/esl_hmm.c:351-409) on the
  * listed sequences of db (ids: original indices): out_sc[j] the filter null
  * score in nats (0 for an empty sequence), bit-exact with the reference's
- * float arithmetic. One thread per sequence. */
+ * float arithmetic. A few lanes per sequence; sequences of more than 1536
+ * residues in segments scored side by side. */
 int   msvgb_biasfilter(msvgb_ctx *ctx, const float *compo, int M, const msvgb_db *db, const int64_t *ids,
                        int64_t nids, float *out_sc);
 /* The length term p7_bg_FilterScore adds to the Forward score of length L. */
