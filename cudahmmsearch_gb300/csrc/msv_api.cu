@@ -1238,15 +1238,18 @@ extern "C" int msvgb_search_device(msvgb_ctx *c, const msvgb_profile *pc, const 
 // / 899, 48M 1049 / 1113; 350, 23M 666 / 700, 33M 832 / 972; 400, 27M 819 / 797, 33M 925 / 959, 38M 1032 / 1118;
 // 440, 38M 1163 / 1117; 480, 27M 1072 / 869, 48M 1597 / 1500, 58M 1794 / 1788, 73M 2109 / 2255; 576, 38M 1745 /
 // 1474, 58M 2199 / 2168; 688, 38M 1879 / 1642, 58M 2270 / 2371; 800, 38M 1907 / 1849, 48M 2253 / 2289; 1030,
-// 38M 2509 / 2318, 48M 3184 / 2891, 73M 4433 / 4375; 1500, 38M 3075 / 3186, 48M 3837 / 3976.
-static int64_t fused_below(int C) {
+// 38M 2509 / 2318, 48M 3184 / 2891, 73M 4433 / 4375; 1500, 38M 3075 / 3186, 48M 3837 / 3976; 1937, 43M 4346 /
+// 4564. The filter cascade's blocks (M = 260, 38M residues), where other kernels share the
+// GPU: 6.90 ms on the groups, 7.48 fused.
+static int64_t fused_below(const msvgb_profile *p) {
+  const int C = p->C;
   if (C <= 4 || C == 6) return 24000000;
-  if (C == 5) return 40000000;
+  if (C == 5) return p->Cg == 19 ? 40000000 : 36000000;
   if (C == 7) return 36000000;
-  return C <= 12 ? 60000000 : 44000000;
+  return C <= 12 || C == 17 ? 60000000 : 42000000;
 }
 static bool search_fused(const msvgb_profile *p, const msvgb_db *db, bool others) {
-  return !p->d_stab_g || (p->lanes_auto && !others && db->residues < fused_below(p->C));
+  return !p->d_stab_g || (p->lanes_auto && !others && db->residues < fused_below(p));
 }
 
 // The segments of a search's long targets. A segment costs its run-in of M

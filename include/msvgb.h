@@ -112,7 +112,7 @@ int msvgb_profile_create_ex(msvgb_ctx *ctx, const msvgb_om *om, int ssv_variant,
 int msvgb_profile_variant(const msvgb_profile *prof);
 /* Lanes per sequence of the SSV pass: 32 (one warp per sequence, SSV
  * and full MSV in one kernel; for models of 1024 to 2047 nodes, searches of
- * at least 44M residues -- or any search, when lanes are set here -- run the
+ * at least 42M residues (60M below 1088 nodes) -- or any search, when lanes are set here -- run the
  * SSV pass and the full MSV as two launches on 32-lane groups instead, with
  * the mixed-width table), or 16 / 8 (2 / 4 sequences per warp in
  * lockstep, for small models: each lane then holds more DP words per row);

@@ -31,9 +31,9 @@ def of_residues(millions):
     return F.SeqSet(s.codes[:s.off[n]], s.off[:n + 1])
 
 
-@pytest.mark.parametrize("M,below,above", [(86, 22, 26), (255, 22, 26), (256, 38, 42), (319, 38, 42), (350, 22, 26), (384, 34, 38),
+@pytest.mark.parametrize("M,below,above", [(86, 22, 26), (255, 22, 26), (256, 34, 38), (300, 38, 42), (319, 34, 38), (350, 22, 26), (384, 34, 38),
                                            (447, 34, 38), (448, 56, 64), (511, 56, 64), (576, 56, 64), (767, 56, 64),
-                                           (768, 42, 46), (1030, 42, 46), (1900, 42, 46)])
+                                           (768, 40, 44), (1023, 40, 44), (1030, 56, 64), (1090, 40, 44), (1900, 40, 44)])
 def test_both_sides_of_the_line(ctx, M, below, above):
     p = api.sample_profile(M, M, ctx)
     dp = api.DeviceProfile(ctx, p)
