@@ -140,13 +140,14 @@ __host__ __device__ constexpr int whole_words() { return F16 && C > 8 && C <= 32
 // chunks of a host search, calls that may not allocate. A warp's time is then
 // the chain of the longest rows it scores, and how far ahead of it the
 // compiler loads the costs sets that chain: a bound of one block per SM frees
-// the registers for it, eight rows a step give it room. ns per row of one warp,
-// SSV / full MSV, in the kernel for both and here (f16 tables): C = 1 22.7 / 137
-// and 21.5 / 129, 3 33.3 / 144 and 17.7 / 135, 6 43.3 / 155 and 18.3 / 144, 11 45.0 / 168
-// and 27.2 / 160, 16 45.0 / 190 and 31.0 / 174, 21 52.4 / 193 and 44.9 / 179, 32 71.0 / 261
-// and 67.3 / 233 (with eight rows a step 60.7 / 249), 52 129 / 395 and 103 / 395 (with
-// the bound 101 / 404), 96 291 / 950 and 268 / 890 (with it 368 / 888, and 34% longer
-// where the SMs are full).
+// the registers for it, eight rows a step give it room (from 9 to 32 words they
+// shorten the SSV row but lengthen the full MSV's: M = 760, 60,000 targets 1659 us
+// with eight, 1566 with four). ns per row of one warp, SSV / full MSV, in the
+// kernel for both and here (f16 tables): C = 1 23.4 / 143 and 21.5 / 129, 3 35.0 / 151
+// and 18.0 / 135, 6 45.4 / 163 and 18.4 / 144, 11 47.0 / 175 and 33.5 / 156, 16 47.1 / 199 and
+// 37.8 / 173, 21 52.5 / 194 and 45.0 / 178, 32 71.0 / 261 and 67.2 / 233, 52 129 / 396 and
+// 103 / 395 (with the bound 101 / 404), 96 292 / 1090 and 270 / 1029 (with it 368 for the SSV
+// row, and 34% longer where the SMs are full).
 template <int C, bool F16>
 __global__ void __launch_bounds__(cta_threads<C, F16>(), whole_blocks<C, F16>())
 msv_whole_kernel(ProfDev P, DbDev db, uint8_t *__restrict__ out_xj, uint8_t *__restrict__ out_flags,
